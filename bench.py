@@ -298,7 +298,7 @@ def surrogate_leg(args, gm, stream):
         run(P, T, Y, out=Wg)
         e = ((Wg - W64).abs().max(dim=0).values / W64.abs().max(dim=0).values).cpu().numpy()
         return ms, e, {"tol": args.surrogate_tol, "margin": margin, "exact_mode": exact_mode,
-                       "exact_path": "counted batch (staged FP64, no host wait)" if run._counted else
+                       "exact_path": "counted batch (FP64 tiles, no host wait)" if run._counted else
                        "batch of cap points, count read at the end of the call",
                        "fallback_rate": run.last_fallback,
                        "mpts_with_fallback": mp(ms),

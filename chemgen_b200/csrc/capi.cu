@@ -21,12 +21,12 @@ cudaError_t launch_getrates_fp64(const DevMech& m, const double* P, const double
 int fp64_smem_block(int ns, size_t smem_per_sm, size_t smem_per_block, long* pts_per_sm);
 size_t fp64_global_slice_bytes(int ns);
 int fp64_global_blocks_per_sm();
-struct StagedPlan;
-cudaError_t staged_prepare(const DevMech& m, const cg_mech_view& v, int device, StagedPlan** out);
-void staged_release(StagedPlan* p);
-cudaError_t launch_getrates_staged(const StagedPlan* p, const DevMech& m, const double* P, const double* T,
-                                   const double* Y, double* wdot, int64_t ng, cudaStream_t s,
-                                   const unsigned long long* count = nullptr);
+struct QuadPlan;
+cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, int mixed, QuadPlan** out);
+void quad_release(QuadPlan* p);
+cudaError_t launch_getrates_quad(const QuadPlan* p, const DevMech& m, const double* P, const double* T,
+                                 const double* Y, double* wdot, int64_t i0, int64_t ng, int64_t n1, cudaStream_t s,
+                                 const unsigned long long* count = nullptr);
 
 struct MixedPlan;
 cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, MixedPlan** out);
@@ -62,8 +62,8 @@ struct chemgen_handle {
     cg::DevMech m{};
     void* dbuf = nullptr;
     int sm_count = 0;
-    int fp64_block = 0;             // 32/64/128: shared-memory state; 0: staged kernel or global scratch
-    cg::StagedPlan* staged = nullptr;   // FP64 staged kernel (state on chip) when fp64_block is 0
+    int fp64_block = 0;             // 32/64/128: shared-memory state; 0: quad kernel or global scratch
+    cg::QuadPlan* quad = nullptr;       // FP64 kernel on eight-point tiles (state on chip)
     cg::JacPlan* jac = nullptr;         // row-owner Jacobian (J written once) when its tile fits
     int64_t fp64_slices = 0;        // persistent blocks of the global variant
     std::mutex mu;
@@ -352,7 +352,7 @@ int ensure_ws_locked(chemgen_handle* h, size_t bytes) {
 }
 
 size_t fp64_ws_bytes(const chemgen_handle* h, int64_t ng) {
-    if (h->fp64_block || h->staged) return 0;
+    if (h->fp64_block || h->quad) return 0;
     int64_t chunks = (ng + 63) / 64;
     int64_t slices = std::min<int64_t>(chunks, h->fp64_slices);
     return (size_t)slices * cg::fp64_global_slice_bytes(h->ns);
@@ -384,8 +384,8 @@ int launch(chemgen_handle* h, int mode, const double* P, const double* T, int64_
         (h->gen_modes & (1u << mode)))
         return h->gen_fn(mode, P, T, ng, Y, w, s);
     if (mode == CHEMGEN_MODE_FP64) {
-        if (!h->fp64_block && h->staged)
-            return status_of(cg::launch_getrates_staged(h->staged, h->m, P, T, Y, w, ng, s));
+        if (!h->fp64_block && h->quad)
+            return status_of(cg::launch_getrates_quad(h->quad, h->m, P, T, Y, w, 0, ng, ng, s));
         int64_t slices = 0;
         if (!h->fp64_block) {
             if (!ws || (reinterpret_cast<uintptr_t>(ws) & 255u)) return CHEMGEN_ERR_INVALID_ARGUMENT;
@@ -486,13 +486,13 @@ int chemgen_create(const void* blob, size_t nbytes, int device, chemgen_handle**
     h->fp64_block = cg::fp64_smem_block(h->ns, prop.sharedMemPerMultiprocessor, prop.sharedMemPerBlockOptin,
                                         &smem_pts);
     h->fp64_slices = (int64_t)h->sm_count * cg::fp64_global_blocks_per_sm();
-    // The staged kernel whenever its tile fits: it is the FP64 kernel when
-    // the one-thread-per-point kernel would hold fewer than 8 warps of points
-    // per SM in shared memory (state too large for one thread per point to
-    // hide its latencies) or none, and it serves the batches whose size is
-    // known only on the device (chemgen_getrates_counted).  Beyond it, the
+    // The quad kernel whenever its tile fits: it is the FP64 kernel when the
+    // one-thread-per-point kernel would hold fewer than 8 warps of points per
+    // SM in shared memory (state too large for one thread per point to hide
+    // its latencies) or none, and it serves the batches whose size is known
+    // only on the device (chemgen_getrates_counted).  Beyond it, the
     // global-scratch kernel.
-    e = cg::staged_prepare(h->m, v, device, &h->staged);
+    e = cg::quad_prepare(h->m, v, device, 0, &h->quad);
     if (e == cudaSuccess) {
         if (smem_pts < 256) h->fp64_block = 0;
     } else if (e != cudaErrorNotSupported) {
@@ -502,7 +502,7 @@ int chemgen_create(const void* blob, size_t nbytes, int device, chemgen_handle**
     }
     e = cg::jac_prepare(h->m, v, device, &h->jac);
     if (e != cudaSuccess && e != cudaErrorNotSupported) {
-        if (h->staged) cg::staged_release(h->staged);
+        if (h->quad) cg::quad_release(h->quad);
         cudaFree(h->dbuf);
         delete h;
         return status_of(e);
@@ -518,7 +518,7 @@ int chemgen_destroy(chemgen_handle* h) {
     DeviceGuard g(h->device);
     cudaDeviceSynchronize();
     if (h->mixed) cg::mixed_release(h->mixed);
-    if (h->staged) cg::staged_release(h->staged);
+    if (h->quad) cg::quad_release(h->quad);
     if (h->jac) cg::jac_release(h->jac);
     if (h->ws) cudaFree(h->ws);
     if (h->dbuf) cudaFree(h->dbuf);
@@ -610,10 +610,10 @@ int chemgen_getrates_counted(chemgen_handle* h, const double* P, const double* T
     if (st || ng == 0) return st;
     if (!count) return CHEMGEN_ERR_INVALID_ARGUMENT;
     if (reinterpret_cast<uintptr_t>(count) & 7u) return CHEMGEN_ERR_MISALIGNED;
-    if (!h->staged) return CHEMGEN_ERR_UNSUPPORTED;
+    if (!h->quad) return CHEMGEN_ERR_UNSUPPORTED;
     DeviceGuard g(h->device);
-    return status_of(cg::launch_getrates_staged(h->staged, h->m, P, T, Y, wdot, ng, (cudaStream_t)stream,
-                                                reinterpret_cast<const unsigned long long*>(count)));
+    return status_of(cg::launch_getrates_quad(h->quad, h->m, P, T, Y, wdot, 0, ng, ng, (cudaStream_t)stream,
+                                              reinterpret_cast<const unsigned long long*>(count)));
 }
 
 int chemgen_workspace_bytes(const chemgen_handle* h, int mode, int64_t ng, size_t* bytes) {
@@ -775,7 +775,7 @@ void wrapper_body(double* P, double* Temp, int ng, double* Ysp, double* wdot, do
     // Large mechanisms keep per-point state in scratch: the caller's log_c
     // (ng*ns doubles) when it holds at least one block's slice, otherwise
     // library-owned scratch.
-    if (!h->fp64_block && !h->staged && log_c) {
+    if (!h->fp64_block && !h->quad && log_c) {
         uintptr_t a = reinterpret_cast<uintptr_t>(log_c);
         uintptr_t al = (a + 255) & ~(uintptr_t)255;
         size_t bytes = (size_t)ng * h->ns * sizeof(double);

@@ -1,0 +1,501 @@
+// getrates on eight-point tiles, four reactions to a warp (quad.cuh), FP64
+// and mixed precision.
+//
+// Computes the same quantities as the reference's generated getrates
+// (chemgen/templates/python_header.j2:25-56, ytoc.j2, exp_g.j2,
+// reactions/{standard,third_body,troe,plog}.j2), with Lindemann and SRI
+// falloff added.  A CTA owns a tile of eight points and keeps its state
+// {C, EGp} (FP64) or {log2 Gibbs, C * 2^32} (mixed) in shared memory:
+//   1  species quads: C and EGp of the tile;
+//   2  reaction quads: the net rates of progress q, into shared memory, all
+//      reactions at once when they fit, else chunk by chunk;
+//   3  species quads: wdot = sum nu q from per-species row lists
+//      (reactions/standard.j2:21-27), each species with one owner, so no
+//      atomics and one order of summation.
+// What bounds it: the load/store unit's 128 bytes per clock (70 % busy at
+// 348 species: the four 16-byte state loads of a reaction, its record, the
+// list rows) and the issue rate (53 %).  Measured on B200, FP64: 348/2163,
+// 2^17 points, 5.63 -> 3.65 ms and JetSurf 2.0 7.2 -> 4.0 ms against the
+// kernel it replaced (32-point tiles, one reaction a warp, 13 chunks with two
+// barriers each); 53/325 on the table-driven path 191 -> 219 Mpts/s.
+// The mixed form repeats the generated mixed kernel's arithmetic reaction by
+// reaction (FP64 exponents and sums, FP32 2^f, products and falloff blend).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <mutex>
+#include <utility>
+#include <vector>
+
+#include "quad.cuh"
+#include "rates_generic.cuh"
+
+namespace cg {
+
+struct QuadPlan {
+    int nquad = 0, nchunk = 0, nsq = 0, rows = 0, warps = 0;
+    int mixed = 0;
+    size_t smem = 0;
+    int grid = 0;
+    const QRec* rec = nullptr;
+    const int4* seg = nullptr;         // runs of quads of one class: {class, first, end, 0}
+    const int2* efl = nullptr;         // [nquad] efficiency lists
+    const QEff* eff = nullptr;
+    const QFall* fall = nullptr;
+    const int* sbeg = nullptr;         // [nchunk + 1] first segment of each chunk
+    const double* th = nullptr;        // quad_thermo's rows
+    const int* sid = nullptr;          // [4 nsq] species of each owner slot (-1: none)
+    QLists lists{};                    // [nchunk][nsq]
+    void* dbuf = nullptr;
+};
+
+struct QuadView {
+    int nchunk, nsq, rows;
+    const QRec* __restrict__ rec;
+    const int4* __restrict__ seg;
+    const int2* __restrict__ efl;
+    const QEff* __restrict__ eff;
+    const QFall* __restrict__ fall;
+    const int* __restrict__ sbeg;
+    const double* __restrict__ th;
+    const int* __restrict__ sid;
+    QLists lists;
+};
+
+// qf - qb of this lane's reaction with forward rate constant kf
+// (reactions/standard.j2:3-19).
+template <bool WIDE, bool REV>
+__device__ __forceinline__ double quad_net(const QRec& R, double kf, const double2* ce) {
+    const double2 a0 = quad_row(ce, R.s[0]), a1 = quad_row(ce, R.s[1]);
+    double cf = a0.x * a1.x, num = a0.y * a1.y;
+    if (WIDE) {
+        const double2 a2 = quad_row(ce, R.s2);
+        cf *= a2.x;
+        num *= a2.y;
+    }
+    if (!REV) return kf * cf;
+    const double2 b0 = quad_row(ce, R.p[0]), b1 = quad_row(ce, R.p[1]);
+    double cb = b0.x * b1.x, den = b0.y * b1.y;
+    if (WIDE) {
+        const double2 b2 = quad_row(ce, R.p2);
+        cb *= b2.x;
+        den *= b2.y;
+    }
+    return kf * cf - kf * num * q_rcp(den) * cb;
+}
+
+__device__ __forceinline__ double quad_net(int cls, const QRec& R, double kf, const double2* ce) {
+    switch (cls & (kQWide | kQRev)) {
+        case 0: return quad_net<false, false>(R, kf, ce);
+        case kQRev: return quad_net<false, true>(R, kf, ce);
+        case kQWide: return quad_net<true, false>(R, kf, ce);
+        default: return quad_net<true, true>(R, kf, ce);
+    }
+}
+
+struct QuadCtx {
+    PointT pt;
+    double P, lnP, ctot;
+    const double2* ce;
+    const double* tab;
+    double* out;                       // this lane's slot of the chunk's first quad
+    int g;
+};
+
+// Elementary reactions: quads q, q + W, ... of a segment.  The record of the
+// warp's next quad is loaded while this one is evaluated.
+template <int W, bool WIDE, bool REV>
+__device__ __forceinline__ void quad_standard(const QuadView& v, const QuadCtx& c, int q, int end, int base) {
+    if (q >= end) return;
+    const QRec* rec = v.rec + kQG * q + c.g;
+    double* out = c.out + (q - base) * 32;
+    QRec N = load_qrec<WIDE>(rec);
+    for (; q < end; q += W, out += 32 * W) {
+        const QRec R = N;
+        rec += kQG * W;
+        if (q + W < end) N = load_qrec<WIDE>(rec);
+        *out = quad_net<WIDE, REV>(R, q_exp(fma(R.b, c.pt.lnT, R.lnA) - R.th * c.pt.invT, c.tab), c.ce);
+    }
+}
+
+template <int W>
+__device__ __forceinline__ void quad_segment(const DevMech& m, const QuadView& v, const QuadCtx& c, int cls, int q,
+                                             int end, int base) {
+    const int kind = cls & 15;
+    if (kind == CG_STANDARD) {
+        switch (cls) {
+            case 0: quad_standard<W, false, false>(v, c, q, end, base); break;
+            case kQRev: quad_standard<W, false, true>(v, c, q, end, base); break;
+            case kQWide: quad_standard<W, true, false>(v, c, q, end, base); break;
+            default: quad_standard<W, true, true>(v, c, q, end, base); break;
+        }
+        return;
+    }
+    if (kind == kQKindGeneric) {
+        for (; q < end; q += W) {
+            const unsigned r = __ldg(&v.rec[kQG * q + c.g].r);
+            const double* s = reinterpret_cast<const double*>(c.ce);
+            c.out[(q - base) * 32] = generic_rate<2 * kQP>(m, r, c.pt, c.P, c.lnP, c.ctot, s, s + 1);
+        }
+        return;
+    }
+    for (; q < end; q += W) {
+        const QRec R = load_qrec<true>(v.rec + kQG * q + c.g);
+        const double M = quad_m(v.eff, __ldg(v.efl + q), c.g, c.ctot, c.ce);
+        double x;
+        if (kind == CG_THIRD_BODY)
+            x = M * quad_net(cls, R, q_exp(fma(R.b, c.pt.lnT, R.lnA) - R.th * c.pt.invT, c.tab), c.ce);
+        else
+            x = quad_net(cls, R, quad_falloff(kind, R, v.fall, M, c.pt, c.tab), c.ce);
+        c.out[(q - base) * 32] = x;
+    }
+}
+
+struct MixPt {
+    double lnT2, invT;
+    float ctot32, Tf, invTf, lnT2f;
+};
+
+// The state of the mixed form in its 16-byte pair: G in x, C * 2^32 in the
+// low word of y.
+__device__ __forceinline__ float mix_c(const double2& s) { return __int_as_float(__double2loint(s.y)); }
+
+// Net rate of progress, mixed precision: the generated mixed kernel's
+// expressions (emit_cuda.py reaction32, falloff32) with molecules as slots.
+__device__ __forceinline__ double quad_rate_mixed(const QuadView& v, int cls, int2 list, const QRec& R, int g,
+                                                  const MixPt& pt, const double2* ce) {
+    const int kind = cls & 15;
+    float Ms = pt.ctot32;
+    if (kind != CG_STANDARD) {
+        const double2* e = reinterpret_cast<const double2*>(v.eff + list.x + g);
+        for (int k = 0; k < list.y; k += 4) {
+            double2 x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = __ldg(e + kQG * (k + u));
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                Ms = fmaf(__int_as_float(__double2hiint(x[u].y)), mix_c(quad_row(ce, __double2loint(x[u].y))), Ms);
+        }
+    }
+    double akf = fma(-R.th, pt.invT, fma(R.b, pt.lnT2, R.lnA));
+    if (kind > CG_THIRD_BODY) {
+        const double2* q = reinterpret_cast<const double2*>(v.fall + R.aux);
+        const double2 f0 = __ldg(q), f1 = __ldg(q + 1), f2 = __ldg(q + 2);
+        const float c0 = __int_as_float(__double2loint(f1.y)), c1 = __int_as_float(__double2hiint(f1.y));
+        const float c2 = __int_as_float(__double2loint(f2.x)), c3 = __int_as_float(__double2hiint(f2.x));
+        const float c4 = __int_as_float(__double2loint(f2.y));
+        const double ainf = akf;
+        const double a0 = fma(-f1.x, pt.invT, fma(f0.y, pt.lnT2, f0.x));
+        int npr;
+        float fpr;
+        cgg::split2(a0 - ainf, npr, fpr);
+        float mpr = cgg::ex2f(fpr) * Ms;
+        const int ex = ((__float_as_int(mpr) >> 23) & 0xff) - 126;
+        npr += ex - 32;
+        mpr = __int_as_float((__float_as_int(mpr) & 0x807fffff) | (126 << 23));   // [0.5, 1)
+        float l2r;
+        int nfix;
+        const float l2m = cgg::lg2f(mpr), l2pr = (float)npr + l2m;
+        cgg::falloff_blend(mpr, npr, l2m, l2r, nfix);
+        constexpr float kL = 0.30102999566398119521f, kIL = (float)(1.0 / 0.30102999566398119521);
+        float l2F = 0.0f;
+        if (kind == CG_TROE) {
+            float Fc = fmaf(c0, cgg::ex2f(c1 * pt.Tf), c2 * cgg::ex2f(c3 * pt.Tf));
+            if (c4 != 0.0f) Fc = Fc + cgg::ex2f(c4 * pt.invTf);
+            const float lFc = kL * cgg::lg2f(Fc);
+            const float lp = kL * l2pr + fmaf(-0.67f, lFc, -0.4f);
+            const float f = __fdividef(lp, fmaf(-0.14f, lp, fmaf(-1.27f, lFc, 0.75f)));
+            l2F = kIL * __fdividef(lFc, fmaf(f, f, 1.0f));
+        } else if (kind == CG_SRI) {
+            const float lp = kL * l2pr;
+            const float X = __fdividef(1.0f, fmaf(lp, lp, 1.0f));
+            const float base = fmaf(c0, cgg::ex2f(c1 * pt.invTf), cgg::ex2f(c2 * pt.Tf));
+            l2F = c3 + X * cgg::lg2f(base) + c4 * pt.lnT2f;
+        }
+        akf = ainf + ((double)nfix + (double)(l2r + l2F));
+    }
+    const float mf = kind == CG_THIRD_BODY ? Ms : 1.0f;
+    const double2 a0 = quad_row(ce, R.s[0]), a1 = quad_row(ce, R.s[1]);
+    float cf = mix_c(a0) * mix_c(a1);
+    double gs = a0.x + a1.x;
+    if (cls & kQWide) {
+        const double2 a2 = quad_row(ce, R.s2);
+        cf *= mix_c(a2);
+        gs += a2.x;
+    }
+    double q = cgg::rate2(akf, cf * mf, -32 * (int)(R.ord & 0xffu));
+    if (cls & kQRev) {
+        const double2 b0 = quad_row(ce, R.p[0]), b1 = quad_row(ce, R.p[1]);
+        float cb = mix_c(b0) * mix_c(b1);
+        gs = (gs - b0.x) - b1.x;
+        if (cls & kQWide) {
+            const double2 b2 = quad_row(ce, R.p2);
+            cb *= mix_c(b2);
+            gs -= b2.x;
+        }
+        q -= cgg::rate2(akf + gs, cb * mf, -32 * (int)((R.ord >> 8) & 0xffu));
+    }
+    return q;
+}
+
+template <int W, int MINB, bool MIXED>
+__global__ void __launch_bounds__(32 * W, MINB)
+    getrates_quad(const __grid_constant__ DevMech m, const __grid_constant__ QuadView v, const double* __restrict__ P, const double* __restrict__ Tg,
+                  const double* __restrict__ Y, double* __restrict__ wdot, int64_t i0, int64_t ng, int64_t n1,
+                  const unsigned long long* __restrict__ count) {
+    extern __shared__ __align__(16) double smem[];
+    const int ns = m.ns;
+    const int lane = threadIdx.x & 31, p = lane & (kQP - 1), g = lane >> 3;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform
+    double* sTab = smem;                                   // [16] 2^(j/16)
+    double* sRed = sTab + 16;                              // [W][8]
+    double2* sCE = reinterpret_cast<double2*>(sRed + W * kQP);   // [ns + 1][8]
+    double* sQ = reinterpret_cast<double*>(sCE + (ns + 1) * kQP);   // [rows + 1][8]
+    double* sW = sQ + (v.rows + 1) * kQP;                  // [ns][8], several chunks only
+    // points [i0, n1) of arrays with stride ng; with a device-side count only
+    // those below min(*count, n1)
+    const int64_t npts = count ? min(n1, (int64_t)*count) : n1;
+    if (threadIdx.x < 16) sTab[threadIdx.x] = kQExpTab[threadIdx.x];
+    if (threadIdx.x < kQP) {
+        sQ[v.rows * kQP + p] = 0.0;                        // the zero row of the lists
+        if (MIXED) sCE[ns * kQP + p] = make_double2(0.0, __hiloint2double(0, __float_as_int(1.0f)));
+        else sCE[ns * kQP + p] = make_double2(1.0, 1.0);
+    }
+    __syncthreads();
+    const double2* ce = sCE + p;
+    for (int64_t t0 = i0 + (int64_t)blockIdx.x * kQP; t0 < npts; t0 += (int64_t)gridDim.x * kQP) {
+        const int64_t i = t0 + p;
+        const bool act = i < npts;
+        const double T = act ? __ldcs(Tg + i) : 1000.0;
+        const double Pp = act ? __ldcs(P + i) : kPatm;
+        PointT pt;
+        pt.T = T;
+        pt.lnT = cgm::cg_log(T);
+        pt.invT = fmin(cgm::cg_rcp(T), kQMaxInvT);
+        MixPt mp;
+        mp.lnT2 = pt.lnT * cgg::kLog2e;
+        mp.invT = pt.invT;
+        // exp_g.j2:2-27 with pfac = Patm/(R0 T) folded in; the sum of Y/W
+        const double pfac = kPatm / kR0 * pt.invT;
+        const double lpfac2 = -6.35856916300311 - mp.lnT2;   // log2(Patm/R0) - log2 T
+        double part = 0.0;
+        for (int k = 4 * warp + g; k < ns; k += 4 * W) {
+            const double c = (act ? __ldcs(Y + (int64_t)k * ng + i) : 1.0) * __ldg(m.inv_mw + k);
+            double cf[8];
+            quad_thermo(v.th, k, T, cf);
+            const double smh = smh_poly(cf, T, pt.lnT, pt.invT);
+            part += c;
+            if (MIXED) sCE[k * kQP + p] = make_double2(fma(smh, cgg::kLog2e, lpfac2), c);
+            else sCE[k * kQP + p] = make_double2(c, q_exp(smh, sTab) * pfac);
+        }
+        part += __shfl_xor_sync(0xffffffffu, part, 8);
+        part += __shfl_xor_sync(0xffffffffu, part, 16);
+        if (g == 0) sRed[warp * kQP + p] = part;
+        __syncthreads();
+        double csum = 0.0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) csum += sRed[w * kQP + p];
+        const double fac = Pp * cgm::cg_rcp(kR0 * csum * T);   // ytoc.j2:3-18
+        const double ctot = csum * fac;
+        for (int k = 4 * warp + g; k < ns; k += 4 * W) {
+            if (MIXED) {
+                const float c = (float)(sCE[k * kQP + p].y * (fac * 4294967296.0));
+                sCE[k * kQP + p].y = __hiloint2double(0, __float_as_int(c));
+            } else {
+                sCE[k * kQP + p].x *= fac;
+            }
+        }
+        mp.ctot32 = (float)(ctot * 4294967296.0);
+        mp.Tf = (float)T;
+        mp.invTf = (float)pt.invT;
+        mp.lnT2f = (float)mp.lnT2;
+        const double lnP = (!MIXED && m.seg[CG_PLOG] < m.seg[CG_PLOG + 1]) ? cgm::cg_log(Pp) : 0.0;
+        __syncthreads();
+        for (int c = 0; c < v.nchunk; ++c) {
+            // the chunk's segments; quad q runs on warp q mod W
+            const int s0 = __ldg(v.sbeg + c), s1 = __ldg(v.sbeg + c + 1);
+            const int base = __ldg(&v.seg[s0].y);
+            for (int s = s0; s < s1; ++s) {
+                const int4 sg = __ldg(v.seg + s);
+                const int cls = __shfl_sync(0xffffffffu, sg.x, 0), end = __shfl_sync(0xffffffffu, sg.z, 0);
+                int q = __shfl_sync(0xffffffffu, sg.y, 0);
+                q += (warp - (q - base) % W + W) % W;
+                if (MIXED) {
+                    for (; q < end; q += W)
+                        sQ[(q - base) * 32 + lane] = quad_rate_mixed(v, cls, __ldg(v.efl + q),
+                                                                     load_qrec<true>(v.rec + kQG * q + g), g, mp, ce);
+                } else {
+                    const QuadCtx qc{pt, Pp, lnP, ctot, ce, sTab, sQ + lane, g};
+                    quad_segment<W>(m, v, qc, cls, q, end, base);
+                }
+            }
+            __syncthreads();
+            const bool last = c == v.nchunk - 1;
+            for (int s = warp; s < v.nsq; s += W) {
+                const int k = __ldg(v.sid + kQG * s + g);
+                double acc = list_sum(v.lists, __ldg(v.lists.info + c * v.nsq + s), g, sQ + p);
+                if (k >= 0) {
+                    if (c > 0) acc += sW[k * kQP + p];
+                    if (!last) sW[k * kQP + p] = acc;
+                    else if (act) __stcs(wdot + (int64_t)k * ng + i, acc);
+                }
+            }
+            if (!last) __syncthreads();
+        }
+    }
+}
+
+using QuadKernel = void (*)(const DevMech, const QuadView, const double*, const double*, const double*, double*, int64_t, int64_t,
+                            int64_t, const unsigned long long*);
+
+static QuadKernel quad_kernel(int warps, int mixed) {
+    switch (warps) {
+        case 8: return mixed ? getrates_quad<8, 3, true> : getrates_quad<8, 3, false>;
+        case 12: return mixed ? getrates_quad<12, 2, true> : getrates_quad<12, 2, false>;
+        default: return mixed ? getrates_quad<24, 1, true> : getrates_quad<24, 1, false>;
+    }
+}
+
+// Species beyond which the FP64 call keeps its caller-visible workspace and
+// runs the global-scratch kernel.
+constexpr int kQuadMaxSpecies = 434;
+
+cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, int mixed, QuadPlan** out) {
+    *out = nullptr;
+    const int ns = m.ns, nr = m.nr;
+    if (nr == 0 || ns > kQuadMaxSpecies) return cudaErrorNotSupported;
+    HostQuads h;
+    build_quads(v, h);
+    if (mixed && !h.mixed_ok) return cudaErrorNotSupported;
+    cudaDeviceProp prop;
+    cudaError_t e = cudaGetDeviceProperties(&prop, device);
+    if (e != cudaSuccess) return e;
+    const size_t limit = prop.sharedMemPerBlockOptin, per_sm = prop.sharedMemPerMultiprocessor;
+    QuadPlan pl;
+    pl.mixed = mixed;
+    pl.nquad = h.nquad;
+    // chunks: every reaction at once when the rates fit beside the state
+    auto bytes = [&](int rows, int chunks, int warps) {
+        return (16 + ((size_t)2 * (ns + 1) + rows + 1 + warps + (chunks > 1 ? ns : 0)) * kQP) * sizeof(double);
+    };
+    int qpc = h.nquad;
+    if (bytes(4 * qpc, 1, 24) > limit) {
+        qpc = (int)((limit - bytes(0, 2, 24)) / (4 * kQP * sizeof(double)));
+        qpc = std::min(qpc, 16000);                        // rows are 16-bit indices
+    }
+    pl.nchunk = (h.nquad + qpc - 1) / qpc;
+    qpc = (h.nquad + pl.nchunk - 1) / pl.nchunk;
+    pl.rows = 4 * qpc;
+    // warps per CTA and CTAs per SM: 24 resident warps of 80 registers, in as
+    // many CTAs as shared memory allows
+    const int fit = (int)(per_sm / (bytes(pl.rows, pl.nchunk, 24) + 1024));
+    pl.warps = fit >= 3 ? 8 : fit == 2 ? 12 : 24;
+    pl.smem = bytes(pl.rows, pl.nchunk, pl.warps);
+    const int resident = std::max(1, std::min((int)(per_sm / (pl.smem + 1024)), 24 / pl.warps));
+    pl.grid = prop.multiProcessorCount * resident;
+    // per-species lists of (row, net coefficient), in sorted-reaction order
+    std::vector<int> qbeg(pl.nchunk + 1), sbeg(1, 0);
+    std::vector<int4> seg;
+    for (int c = 0; c <= pl.nchunk; ++c) qbeg[c] = std::min(h.nquad, c * qpc);
+    for (int c = 0; c < pl.nchunk; ++c) {
+        for (int q = qbeg[c]; q < qbeg[c + 1]; ++q) {
+            if (q == qbeg[c] || h.key[q] != h.key[q - 1]) seg.push_back(make_int4(h.key[q], q, q, 0));
+            seg.back().z = q + 1;
+        }
+        sbeg.push_back((int)seg.size());
+    }
+    const int32_t* rp = (const int32_t*)v.a[CG_RPTR];
+    const int32_t* pp = (const int32_t*)v.a[CG_PPTR];
+    const int32_t* rsp = (const int32_t*)v.a[CG_RSP];
+    const int32_t* psp = (const int32_t*)v.a[CG_PSP];
+    const double* rnu = (const double*)v.a[CG_RNU];
+    const double* pnu = (const double*)v.a[CG_PNU];
+    std::vector<int> order(nr);
+    for (int r = 0; r < nr; ++r) order[r] = r;
+    std::sort(order.begin(), order.end(), [&](int a, int b) { return h.at[a] < h.at[b]; });
+    std::vector<std::vector<ListBuilder::List>> lists(pl.nchunk, std::vector<ListBuilder::List>(ns));
+    std::vector<double> net(ns, 0.0);
+    for (int r : order) {
+        const int c = (h.at[r] / 4) / qpc, row = h.at[r] - 4 * qbeg[c];
+        for (int j = rp[r]; j < rp[r + 1]; ++j) net[rsp[j]] -= rnu[j];
+        for (int j = pp[r]; j < pp[r + 1]; ++j) net[psp[j]] += pnu[j];
+        for (int side = 0; side < 2; ++side)
+            for (int j = side ? pp[r] : rp[r]; j < (side ? pp[r + 1] : rp[r + 1]); ++j) {
+                const int k = side ? psp[j] : rsp[j];
+                if (net[k] != 0.0) lists[c][k].push_back({row, net[k]});
+                net[k] = 0.0;
+            }
+    }
+    std::vector<size_t> len(ns, 0);
+    for (int k = 0; k < ns; ++k)
+        for (int c = 0; c < pl.nchunk; ++c) len[k] += ListBuilder::length(lists[c][k]);
+    const std::vector<std::vector<int>> quads = ListBuilder::group(len, pl.warps);
+    pl.nsq = (int)quads.size();
+    std::vector<int> sid(4 * pl.nsq, -1);
+    ListBuilder lb;
+    for (int s = 0; s < pl.nsq; ++s)
+        for (size_t g = 0; g < quads[s].size(); ++g) sid[4 * s + g] = quads[s][g];
+    for (int c = 0; c < pl.nchunk; ++c)
+        for (const std::vector<int>& q : quads) {
+            std::vector<const ListBuilder::List*> own;
+            for (int k : q) own.push_back(&lists[c][k]);
+            lb.add_quad(own, pl.rows);
+        }
+    Image im;
+    const size_t o_rec = im.put(mixed ? h.rec2 : h.rec), o_seg = im.put(seg), o_efl = im.put(h.efl), o_eff = im.put(h.eff);
+    const size_t o_fall = im.put(mixed ? h.fall2 : h.fall), o_sb = im.put(sbeg), o_th = im.put(quad_thermo_rows(v)), o_sid = im.put(sid);
+    const size_t o_li = im.put(lb.info), o_le = im.put(lb.ent), o_lg = im.put(lb.gen);
+    QuadPlan* q = new QuadPlan(pl);
+    e = im.upload(&q->dbuf);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(quad_kernel(q->warps, mixed), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)q->smem);
+    if (e != cudaSuccess) {
+        if (q->dbuf) cudaFree(q->dbuf);
+        delete q;
+        return e;
+    }
+    char* d = (char*)q->dbuf;
+    q->rec = (const QRec*)(d + o_rec);
+    q->seg = (const int4*)(d + o_seg);
+    q->efl = (const int2*)(d + o_efl);
+    q->eff = (const QEff*)(d + o_eff);
+    q->fall = (const QFall*)(d + o_fall);
+    q->sbeg = (const int*)(d + o_sb);
+    q->th = (const double*)(d + o_th);
+    q->sid = (const int*)(d + o_sid);
+    q->lists.info = (const int4*)(d + o_li);
+    q->lists.ent = (const uint4*)(d + o_le);
+    q->lists.gen = (const QGen*)(d + o_lg);
+    *out = q;
+    return cudaSuccess;
+}
+
+void quad_release(QuadPlan* p) {
+    if (!p) return;
+    if (p->dbuf) cudaFree(p->dbuf);
+    delete p;
+}
+
+// Points [i0, n1) of arrays laid out for ng points (all: i0 = 0, n1 = ng).
+cudaError_t launch_getrates_quad(const QuadPlan* p, const DevMech& m, const double* P, const double* T,
+                                 const double* Y, double* wdot, int64_t i0, int64_t ng, int64_t n1, cudaStream_t s,
+                                 const unsigned long long* count) {
+    if (n1 <= i0) return cudaSuccess;
+    const int64_t tiles = (n1 - i0 + kQP - 1) / kQP;
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles, p->grid);
+    const QuadView v{p->nchunk, p->nsq, p->rows, p->rec, p->seg, p->efl, p->eff, p->fall, p->sbeg, p->th, p->sid, p->lists};
+    // Every plan of the same kernel instance (one per handle) has its own
+    // shared-memory size: the limit is set and the kernel launched under one
+    // lock, so that a handle made later for a smaller mechanism cannot leave
+    // the limit below this plan's.
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    const QuadKernel fn = quad_kernel(p->warps, p->mixed);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
+    if (e != cudaSuccess) return e;
+    fn<<<grid, 32u * (unsigned)p->warps, p->smem, s>>>(m, v, P, T, Y, wdot, i0, ng, n1, count);
+    return cudaGetLastError();
+}
+
+}  // namespace cg

@@ -738,15 +738,15 @@ class SurrogateGetrates:
     exact kernel runs on that batch and chemgen_gate_scatter writes its
     results over the surrogate's.  Two ways to run the batch:
 
-    * exact_mode="fp64" (when the mechanism's handle has the staged FP64
+    * exact_mode="fp64" (when the mechanism's handle has the tiled FP64
       kernel): the batch holds every point and chemgen_getrates_counted
       computes only the points counted on the device, so nothing waits for
       the host; the fallback rate is read when `last_fallback` is asked for.
-      The staged kernel costs ~5x the generated mixed kernel per point, so
+      The tiled kernel costs ~4x the generated mixed kernel per point, so
       this suits the few-tenths-of-a-percent fallback of a gate at its
       tolerance.  The batch buffers hold 2 ns + 3 values per point (a copy
       of the states and rates of every point, on the device).
-    * otherwise (exact_mode="mixed", or no staged kernel): a batch of `cap`
+    * otherwise (exact_mode="mixed", or no tiled kernel): a batch of `cap`
       points on the exact kernel of that mode, and one read of the count at
       the end of the call; if more points failed than the batch holds, all
       failing points go through the host path (`_host_gate`) and the batch
@@ -766,7 +766,7 @@ class SurrogateGetrates:
         self._pending = None          # (buffers, ng) of a call whose count is still on the device
         self._cap = cap
         self._bufs = None
-        self._counted = exact_mode == "fp64"   # cleared when the handle has no staged kernel
+        self._counted = exact_mode == "fp64"   # cleared when the handle has no tiled kernel
 
     @property
     def threshold(self) -> float:
@@ -857,7 +857,7 @@ class SurrogateGetrates:
         if self._counted:
             st = L.chemgen_getrates_counted(self.sur.gm._h, b["p_P"], b["p_T"], cap, b["p_Y"], b["p_W"],
                                             b["p_count"], s)
-            if st == 6:                             # no staged kernel for this mechanism: batch path
+            if st == 6:                             # no tiled kernel for this mechanism: batch path
                 self._counted = False
                 self._bufs = None
                 return self(P, T, Y, out=W)

@@ -75,7 +75,7 @@ int chemgen_getrates_ex(chemgen_handle* h, int mode, const double* P, const doub
  * only on the device, such as the points an error gate sends back
  * (chemgen_gate_select): a launch covers only the points counted, so the
  * batch can be sized for every point and nothing waits for the host.  Points
- * past the count are left as they are.  Runs on the staged FP64 kernel;
+ * past the count are left as they are.  Runs on the FP64 tile kernel;
  * CHEMGEN_ERR_UNSUPPORTED for a mechanism too large for it.  Asynchronous. */
 int chemgen_getrates_counted(chemgen_handle* h, const double* P, const double* T, int64_t ng, const double* Y,
                              double* wdot, const uint64_t* count, void* stream);

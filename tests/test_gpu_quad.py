@@ -1,0 +1,51 @@
+"""The eight-point-tile kernels (four reactions to a warp) at the sizes where
+they can go wrong: part tiles, one point, several chunks of reactions, owners
+with long lists, reactions without a pre-decoded form."""
+import numpy as np
+import pytest
+
+from chemgen_b200 import pack, synthetic
+from chemgen_b200.runtime import GpuMechanism
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+TOL_FP64 = 1e-10          # the FP64 kernels' bar (rounding of ~300-term sums is 1e-13)
+
+
+def _cuda(*arrays):
+    import torch
+    return [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in arrays]
+
+
+def _check(mech, ng, seed=0):
+    blob = pack.pack(mech).to_blob()
+    P, T, Y = synthetic.states(mech.ns, ng, seed=seed)
+    w = GpuMechanism(blob).getrates(*_cuda(P, T, Y)).cpu().numpy()
+    r = oracle.rates(blob, P, T, Y, mech.nr)
+    e = oracle.errors(w, r["wdot"], r["S"])
+    assert e["norm_max"] <= TOL_FP64 and e["gross_max"] <= TOL_FP64, e
+
+
+@pytest.mark.parametrize("ng", [1, 7, 8, 9, 8 * 148 * 3 + 5])
+def test_part_tiles(ng):
+    _check(synthetic.gri_shape(), ng, seed=ng)
+
+
+def test_several_chunks_of_reactions():
+    # the rates of 4200 reactions (268 KB for eight points) take two chunks
+    _check(synthetic.synthetic_mechanism(120, 4200, 40, 60, seed=9), 41)
+
+
+def test_every_kind_and_general_stoichiometry():
+    # PLOG, SRI, Lindemann; a negative and a zero pre-exponential factor,
+    # fractional coefficients and four molecules on a side take the generic path
+    mech = synthetic.synthetic_mechanism(60, 200, 12, 12, seed=6, n_lindemann=6, n_sri=6, n_plog=6)
+    rx = [r for r in mech.reactions if r.kind == "standard"]
+    rx[0].arh = (-rx[0].arh[0],) + rx[0].arh[1:]
+    rx[1].arh = (0.0,) + rx[1].arh[1:]
+    s = mech.species_names
+    rx[2].reactants, rx[2].products = {s[0]: 1.0, s[1]: 1.0}, {s[2]: 0.5, s[3]: 1.5}
+    rx[2].reversible = False
+    rx[3].reactants, rx[3].products = {s[4]: 1.0}, {s[5]: 2.0, s[6]: 1.0, s[7]: 1.0}
+    rx[3].reversible = False
+    _check(mech, 83)
