@@ -36,6 +36,13 @@ cudaError_t launch_getrates_mixed(const MixedPlan* p, const DevMech& m, const do
                                   cudaStream_t s);
 size_t mixed_workspace_bytes(const MixedPlan* p, int64_t ng);
 size_t deriv_workspace_bytes(int ns, int64_t ng);
+struct GradPlan;
+cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, int adjoint, GradPlan** out);
+void grad_release(GradPlan* p);
+cudaError_t launch_jacobian_quad(const GradPlan* p, const DevMech& m, int precision, const double* P, const double* T,
+                                 const double* Y, void* J, int64_t ng, cudaStream_t s);
+cudaError_t launch_vjp_quad(const GradPlan* p, const DevMech& m, const double* P, const double* T, const double* Y,
+                            const double* G, double* gT, double* gY, double* gP, int64_t ng, cudaStream_t s);
 struct JacPlan;
 cudaError_t jac_prepare(const DevMech& m, const cg_mech_view& v, int device, JacPlan** out);
 void jac_release(JacPlan* p);
@@ -64,7 +71,9 @@ struct chemgen_handle {
     int sm_count = 0;
     int fp64_block = 0;             // 32/64/128: shared-memory state; 0: quad kernel or global scratch
     cg::QuadPlan* quad = nullptr;       // FP64 kernel on eight-point tiles (state on chip)
-    cg::JacPlan* jac = nullptr;         // row-owner Jacobian (J written once) when its tile fits
+    cg::GradPlan* jacq = nullptr;       // Jacobian on eight-point tiles when every reaction's rows fit
+    cg::GradPlan* vjpq = nullptr;       // adjoint on eight-point tiles
+    cg::JacPlan* jac = nullptr;         // row-owner Jacobian (J written once) otherwise, when its tile fits
     int64_t fp64_slices = 0;        // persistent blocks of the global variant
     std::mutex mu;
     void* ws = nullptr;             // library-owned scratch
@@ -500,8 +509,11 @@ int chemgen_create(const void* blob, size_t nbytes, int device, chemgen_handle**
         delete h;
         return status_of(e);
     }
-    e = cg::jac_prepare(h->m, v, device, &h->jac);
+    e = cg::grad_prepare(h->m, v, device, 1, &h->vjpq);
+    if (e == cudaSuccess || e == cudaErrorNotSupported) e = cg::grad_prepare(h->m, v, device, 0, &h->jacq);
+    if (e == cudaErrorNotSupported) e = cg::jac_prepare(h->m, v, device, &h->jac);
     if (e != cudaSuccess && e != cudaErrorNotSupported) {
+        cg::grad_release(h->vjpq);
         if (h->quad) cg::quad_release(h->quad);
         cudaFree(h->dbuf);
         delete h;
@@ -520,6 +532,8 @@ int chemgen_destroy(chemgen_handle* h) {
     if (h->mixed) cg::mixed_release(h->mixed);
     if (h->quad) cg::quad_release(h->quad);
     if (h->jac) cg::jac_release(h->jac);
+    cg::grad_release(h->jacq);
+    cg::grad_release(h->vjpq);
     if (h->ws) cudaFree(h->ws);
     if (h->dbuf) cudaFree(h->dbuf);
     if (h->iobuf) cudaFree(h->iobuf);
@@ -548,6 +562,8 @@ int chemgen_jacobian(chemgen_handle* h, int precision, const double* P, const do
     if (precision != 0 && precision != 1) return CHEMGEN_ERR_INVALID_ARGUMENT;
     DeviceGuard g(h->device);
     if (h->max_side > 16) return CHEMGEN_ERR_UNSUPPORTED;
+    if (h->jacq)
+        return status_of(cg::launch_jacobian_quad(h->jacq, h->m, precision, P, T, Y, J, ng, (cudaStream_t)stream));
     std::lock_guard<std::mutex> lk(h->mu);
     if (h->jac) {
         st = ensure_ws_locked(h, cg::jac_rows_workspace_bytes(h->jac, h->m, ng));
@@ -569,6 +585,8 @@ int chemgen_getrates_vjp(chemgen_handle* h, const double* P, const double* T, in
         return G && gT ? CHEMGEN_ERR_MISALIGNED : CHEMGEN_ERR_INVALID_ARGUMENT;
     DeviceGuard g(h->device);
     if (h->max_side > 16) return CHEMGEN_ERR_UNSUPPORTED;
+    if (h->vjpq)
+        return status_of(cg::launch_vjp_quad(h->vjpq, h->m, P, T, Y, G, gT, gY, gP, ng, (cudaStream_t)stream));
     std::lock_guard<std::mutex> lk(h->mu);
     st = ensure_ws_locked(h, cg::deriv_workspace_bytes(h->ns, ng));
     if (st) return st;

@@ -15,9 +15,10 @@
 // What bounds it: the load/store unit's 128 bytes per clock (70 % busy at
 // 348 species: the four 16-byte state loads of a reaction, its record, the
 // list rows) and the issue rate (53 %).  Measured on B200, FP64: 348/2163,
-// 2^17 points, 5.63 -> 3.65 ms and JetSurf 2.0 7.2 -> 4.0 ms against the
-// kernel it replaced (32-point tiles, one reaction a warp, 13 chunks with two
-// barriers each); 53/325 on the table-driven path 191 -> 219 Mpts/s.
+// 2^17 points, 5.63 -> 3.29 ms against the kernel it replaced (32-point tiles,
+// one reaction a warp, 13 chunks with two barriers each); JetSurf 2.0 3.6 ms;
+// 53/325 on the table-driven path 191 -> 272 Mpts/s.  A loop per class (build_runs)
+// is 18 % faster than a dispatch per quad (3.31 against 4.04 ms at 348/2163).
 // The mixed form repeats the generated mixed kernel's arithmetic reaction by
 // reaction (FP64 exponents and sums, FP32 2^f, products and falloff blend).
 #include <cuda_runtime.h>
@@ -38,27 +39,25 @@ struct QuadPlan {
     size_t smem = 0;
     int grid = 0;
     const QRec* rec = nullptr;
-    const int4* seg = nullptr;         // runs of quads of one class: {class, first, end, 0}
+    const int4* run = nullptr;         // {class, first quad, how many, first slot}
     const int2* efl = nullptr;         // [nquad] efficiency lists
     const QEff* eff = nullptr;
     const QFall* fall = nullptr;
-    const int* sbeg = nullptr;         // [nchunk + 1] first segment of each chunk
+    const int* rbeg = nullptr;         // [nchunk W + 1] first run of each warp in each chunk
     const double* th = nullptr;        // quad_thermo's rows
-    const int* sid = nullptr;          // [4 nsq] species of each owner slot (-1: none)
-    QLists lists{};                    // [nchunk][nsq]
+    QLists lists{};                    // owners: species, [nchunk][nsq] quads
     void* dbuf = nullptr;
 };
 
 struct QuadView {
     int nchunk, nsq, rows;
     const QRec* __restrict__ rec;
-    const int4* __restrict__ seg;
+    const int4* __restrict__ run;
     const int2* __restrict__ efl;
     const QEff* __restrict__ eff;
     const QFall* __restrict__ fall;
-    const int* __restrict__ sbeg;
+    const int* __restrict__ rbeg;
     const double* __restrict__ th;
-    const int* __restrict__ sid;
     QLists lists;
 };
 
@@ -98,56 +97,51 @@ struct QuadCtx {
     double P, lnP, ctot;
     const double2* ce;
     const double* tab;
-    double* out;                       // this lane's slot of the chunk's first quad
     int g;
 };
 
-// Elementary reactions: quads q, q + W, ... of a segment.  The record of the
-// warp's next quad is loaded while this one is evaluated.
+// Elementary reactions: the n quads of a run.  The record of the next quad is
+// loaded while this one is evaluated.
 template <int W, bool WIDE, bool REV>
-__device__ __forceinline__ void quad_standard(const QuadView& v, const QuadCtx& c, int q, int end, int base) {
-    if (q >= end) return;
-    const QRec* rec = v.rec + kQG * q + c.g;
-    double* out = c.out + (q - base) * 32;
+__device__ __forceinline__ void quad_standard(const QuadCtx& c, const QRec* rec, int n, double* out) {
     QRec N = load_qrec<WIDE>(rec);
-    for (; q < end; q += W, out += 32 * W) {
+    for (; n > 0; --n, out += 32 * W) {
         const QRec R = N;
         rec += kQG * W;
-        if (q + W < end) N = load_qrec<WIDE>(rec);
+        if (n > 1) N = load_qrec<WIDE>(rec);
         *out = quad_net<WIDE, REV>(R, q_exp(fma(R.b, c.pt.lnT, R.lnA) - R.th * c.pt.invT, c.tab), c.ce);
     }
 }
 
 template <int W>
-__device__ __forceinline__ void quad_segment(const DevMech& m, const QuadView& v, const QuadCtx& c, int cls, int q,
-                                             int end, int base) {
+__device__ __forceinline__ void quad_run(const DevMech& m, const QuadView& v, const QuadCtx& c, int cls, int q, int n,
+                                         double* out) {
     const int kind = cls & 15;
+    const QRec* rec = v.rec + kQG * q + c.g;
     if (kind == CG_STANDARD) {
         switch (cls) {
-            case 0: quad_standard<W, false, false>(v, c, q, end, base); break;
-            case kQRev: quad_standard<W, false, true>(v, c, q, end, base); break;
-            case kQWide: quad_standard<W, true, false>(v, c, q, end, base); break;
-            default: quad_standard<W, true, true>(v, c, q, end, base); break;
+            case 0: quad_standard<W, false, false>(c, rec, n, out); break;
+            case kQRev: quad_standard<W, false, true>(c, rec, n, out); break;
+            case kQWide: quad_standard<W, true, false>(c, rec, n, out); break;
+            default: quad_standard<W, true, true>(c, rec, n, out); break;
         }
         return;
     }
     if (kind == kQKindGeneric) {
-        for (; q < end; q += W) {
-            const unsigned r = __ldg(&v.rec[kQG * q + c.g].r);
+        for (; n > 0; --n, rec += kQG * W, out += 32 * W) {
+            const unsigned r = __ldg(&rec->r);
             const double* s = reinterpret_cast<const double*>(c.ce);
-            c.out[(q - base) * 32] = generic_rate<2 * kQP>(m, r, c.pt, c.P, c.lnP, c.ctot, s, s + 1);
+            *out = r == kQNone ? 0.0 : generic_rate<2 * kQP>(m, r, c.pt, c.P, c.lnP, c.ctot, s, s + 1);
         }
         return;
     }
-    for (; q < end; q += W) {
-        const QRec R = load_qrec<true>(v.rec + kQG * q + c.g);
+    for (; n > 0; --n, q += W, rec += kQG * W, out += 32 * W) {
+        const QRec R = load_qrec(rec);
         const double M = quad_m(v.eff, __ldg(v.efl + q), c.g, c.ctot, c.ce);
-        double x;
         if (kind == CG_THIRD_BODY)
-            x = M * quad_net(cls, R, q_exp(fma(R.b, c.pt.lnT, R.lnA) - R.th * c.pt.invT, c.tab), c.ce);
+            *out = M * quad_net(cls, R, q_exp(fma(R.b, c.pt.lnT, R.lnA) - R.th * c.pt.invT, c.tab), c.ce);
         else
-            x = quad_net(cls, R, quad_falloff(kind, R, v.fall, M, c.pt, c.tab), c.ce);
-        c.out[(q - base) * 32] = x;
+            *out = quad_net(cls, R, quad_falloff(kind, R, v.fall, M, c.pt, c.tab), c.ce);
     }
 }
 
@@ -162,11 +156,12 @@ __device__ __forceinline__ float mix_c(const double2& s) { return __int_as_float
 
 // Net rate of progress, mixed precision: the generated mixed kernel's
 // expressions (emit_cuda.py reaction32, falloff32) with molecules as slots.
-__device__ __forceinline__ double quad_rate_mixed(const QuadView& v, int cls, int2 list, const QRec& R, int g,
+__device__ __forceinline__ double quad_rate_mixed(const QuadView& v, int cls, int q, const QRec& R, int g,
                                                   const MixPt& pt, const double2* ce) {
     const int kind = cls & 15;
     float Ms = pt.ctot32;
     if (kind != CG_STANDARD) {
+        const int2 list = __ldg(v.efl + q);
         const double2* e = reinterpret_cast<const double2*>(v.eff + list.x + g);
         for (int k = 0; k < list.y; k += 4) {
             double2 x[4];
@@ -179,8 +174,8 @@ __device__ __forceinline__ double quad_rate_mixed(const QuadView& v, int cls, in
     }
     double akf = fma(-R.th, pt.invT, fma(R.b, pt.lnT2, R.lnA));
     if (kind > CG_THIRD_BODY) {
-        const double2* q = reinterpret_cast<const double2*>(v.fall + R.aux);
-        const double2 f0 = __ldg(q), f1 = __ldg(q + 1), f2 = __ldg(q + 2);
+        const double2* fp = reinterpret_cast<const double2*>(v.fall + R.aux);
+        const double2 f0 = __ldg(fp), f1 = __ldg(fp + 1), f2 = __ldg(fp + 2);
         const float c0 = __int_as_float(__double2loint(f1.y)), c1 = __int_as_float(__double2hiint(f1.y));
         const float c2 = __int_as_float(__double2loint(f2.x)), c3 = __int_as_float(__double2hiint(f2.x));
         const float c4 = __int_as_float(__double2loint(f2.y));
@@ -223,7 +218,7 @@ __device__ __forceinline__ double quad_rate_mixed(const QuadView& v, int cls, in
         cf *= mix_c(a2);
         gs += a2.x;
     }
-    double q = cgg::rate2(akf, cf * mf, -32 * (int)(R.ord & 0xffu));
+    double rr = cgg::rate2(akf, cf * mf, -32 * (int)(R.ord & 0xffu));
     if (cls & kQRev) {
         const double2 b0 = quad_row(ce, R.p[0]), b1 = quad_row(ce, R.p[1]);
         float cb = mix_c(b0) * mix_c(b1);
@@ -233,9 +228,9 @@ __device__ __forceinline__ double quad_rate_mixed(const QuadView& v, int cls, in
             cb *= mix_c(b2);
             gs -= b2.x;
         }
-        q -= cgg::rate2(akf + gs, cb * mf, -32 * (int)((R.ord >> 8) & 0xffu));
+        rr -= cgg::rate2(akf + gs, cb * mf, -32 * (int)((R.ord >> 8) & 0xffu));
     }
-    return q;
+    return rr;
 }
 
 template <int W, int MINB, bool MIXED>
@@ -248,7 +243,8 @@ __global__ void __launch_bounds__(32 * W, MINB)
     const int lane = threadIdx.x & 31, p = lane & (kQP - 1), g = lane >> 3;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // warp-uniform
     double* sTab = smem;                                   // [16] 2^(j/16)
-    double* sRed = sTab + 16;                              // [W][8]
+    double* sH = sTab + 16;                                // [2][4][8] this tile's and the next one's T, ln T, 1/T, P
+    double* sRed = sH + 8 * kQP;                           // [W][8]
     double2* sCE = reinterpret_cast<double2*>(sRed + W * kQP);   // [ns + 1][8]
     double* sQ = reinterpret_cast<double*>(sCE + (ns + 1) * kQP);   // [rows + 1][8]
     double* sW = sQ + (v.rows + 1) * kQP;                  // [ns][8], several chunks only
@@ -256,6 +252,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
     // those below min(*count, n1)
     const int64_t npts = count ? min(n1, (int64_t)*count) : n1;
     if (threadIdx.x < 16) sTab[threadIdx.x] = kQExpTab[threadIdx.x];
+    if (warp == W - 1 && g == 0) quad_head(sH, i0 + (int64_t)blockIdx.x * kQP + p, npts, P, Tg);
     if (threadIdx.x < kQP) {
         sQ[v.rows * kQP + p] = 0.0;                        // the zero row of the lists
         if (MIXED) sCE[ns * kQP + p] = make_double2(0.0, __hiloint2double(0, __float_as_int(1.0f)));
@@ -263,15 +260,17 @@ __global__ void __launch_bounds__(32 * W, MINB)
     }
     __syncthreads();
     const double2* ce = sCE + p;
-    for (int64_t t0 = i0 + (int64_t)blockIdx.x * kQP; t0 < npts; t0 += (int64_t)gridDim.x * kQP) {
+    const int64_t step = (int64_t)gridDim.x * kQP;
+    int buf = 0;
+    for (int64_t t0 = i0 + (int64_t)blockIdx.x * kQP; t0 < npts; t0 += step, buf ^= 1) {
         const int64_t i = t0 + p;
         const bool act = i < npts;
-        const double T = act ? __ldcs(Tg + i) : 1000.0;
-        const double Pp = act ? __ldcs(P + i) : kPatm;
+        const double* h = sH + buf * 4 * kQP + p;
         PointT pt;
-        pt.T = T;
-        pt.lnT = cgm::cg_log(T);
-        pt.invT = fmin(cgm::cg_rcp(T), kQMaxInvT);
+        pt.T = h[0];
+        pt.lnT = h[kQP];
+        pt.invT = h[2 * kQP];
+        const double T = pt.T, Pp = h[3 * kQP];
         MixPt mp;
         mp.lnT2 = pt.lnT * cgg::kLog2e;
         mp.invT = pt.invT;
@@ -292,9 +291,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
         part += __shfl_xor_sync(0xffffffffu, part, 16);
         if (g == 0) sRed[warp * kQP + p] = part;
         __syncthreads();
-        double csum = 0.0;
-#pragma unroll
-        for (int w = 0; w < W; ++w) csum += sRed[w * kQP + p];
+        const double csum = quad_total<W>(sRed, g);
         const double fac = Pp * cgm::cg_rcp(kR0 * csum * T);   // ytoc.j2:3-18
         const double ctot = csum * fac;
         for (int k = 4 * warp + g; k < ns; k += 4 * W) {
@@ -312,32 +309,38 @@ __global__ void __launch_bounds__(32 * W, MINB)
         const double lnP = (!MIXED && m.seg[CG_PLOG] < m.seg[CG_PLOG + 1]) ? cgm::cg_log(Pp) : 0.0;
         __syncthreads();
         for (int c = 0; c < v.nchunk; ++c) {
-            // the chunk's segments; quad q runs on warp q mod W
-            const int s0 = __ldg(v.sbeg + c), s1 = __ldg(v.sbeg + c + 1);
-            const int base = __ldg(&v.seg[s0].y);
-            for (int s = s0; s < s1; ++s) {
-                const int4 sg = __ldg(v.seg + s);
-                const int cls = __shfl_sync(0xffffffffu, sg.x, 0), end = __shfl_sync(0xffffffffu, sg.z, 0);
-                int q = __shfl_sync(0xffffffffu, sg.y, 0);
-                q += (warp - (q - base) % W + W) % W;
+            const int* rb = v.rbeg + c * W + warp;
+            const int r1 = __ldg(rb + 1);
+            for (int r = __ldg(rb); r < r1; ++r) {
+                const int4 rn = __ldg(v.run + r);
+                const int cls = __shfl_sync(0xffffffffu, rn.x, 0), n = __shfl_sync(0xffffffffu, rn.z, 0);
+                double* out = sQ + rn.w + lane;
                 if (MIXED) {
-                    for (; q < end; q += W)
-                        sQ[(q - base) * 32 + lane] = quad_rate_mixed(v, cls, __ldg(v.efl + q),
-                                                                     load_qrec<true>(v.rec + kQG * q + g), g, mp, ce);
+                    for (int j = 0, q = rn.y; j < n; ++j, q += W)
+                        out[j * 32 * W] = quad_rate_mixed(v, cls, q, load_qrec(v.rec + kQG * q + g), g, mp, ce);
                 } else {
-                    const QuadCtx qc{pt, Pp, lnP, ctot, ce, sTab, sQ + lane, g};
-                    quad_segment<W>(m, v, qc, cls, q, end, base);
+                    const QuadCtx qc{pt, Pp, lnP, ctot, ce, sTab, g};
+                    quad_run<W>(m, v, qc, cls, rn.y, n, out);
                 }
             }
+            if (c == 0 && warp == W - 1 && g == 0 && t0 + step < npts)
+                quad_head(sH + (buf ^ 1) * 4 * kQP, t0 + step + p, npts, P, Tg);
             __syncthreads();
             const bool last = c == v.nchunk - 1;
-            for (int s = warp; s < v.nsq; s += W) {
-                const int k = __ldg(v.sid + kQG * s + g);
-                double acc = list_sum(v.lists, __ldg(v.lists.info + c * v.nsq + s), g, sQ + p);
-                if (k >= 0) {
-                    if (c > 0) acc += sW[k * kQP + p];
-                    if (!last) sW[k * kQP + p] = acc;
-                    else if (act) __stcs(wdot + (int64_t)k * ng + i, acc);
+            if (warp < v.nsq) {
+                const QOwn* op = v.lists.own + kQG * (c * v.nsq + warp) + g;
+                QOwn N = load_qown(op);
+                for (int s = warp; s < v.nsq; s += W) {
+                    const QOwn o = N;
+                    op += kQG * W;
+                    if (s + W < v.nsq) N = load_qown(op);
+                    double acc = list_sum(v.lists, o, g, sQ + p);
+                    const int k = o.own;
+                    if (k >= 0) {
+                        if (c > 0) acc += sW[k * kQP + p];
+                        if (!last) sW[k * kQP + p] = acc;
+                        else if (act) __stcs(wdot + (int64_t)k * ng + i, acc);
+                    }
                 }
             }
             if (!last) __syncthreads();
@@ -376,7 +379,7 @@ cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     pl.nquad = h.nquad;
     // chunks: every reaction at once when the rates fit beside the state
     auto bytes = [&](int rows, int chunks, int warps) {
-        return (16 + ((size_t)2 * (ns + 1) + rows + 1 + warps + (chunks > 1 ? ns : 0)) * kQP) * sizeof(double);
+        return (16 + ((size_t)8 + 2 * (ns + 1) + rows + 1 + warps + (chunks > 1 ? ns : 0)) * kQP) * sizeof(double);
     };
     int qpc = h.nquad;
     if (bytes(4 * qpc, 1, 24) > limit) {
@@ -394,16 +397,13 @@ cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     const int resident = std::max(1, std::min((int)(per_sm / (pl.smem + 1024)), 24 / pl.warps));
     pl.grid = prop.multiProcessorCount * resident;
     // per-species lists of (row, net coefficient), in sorted-reaction order
-    std::vector<int> qbeg(pl.nchunk + 1), sbeg(1, 0);
-    std::vector<int4> seg;
+    std::vector<int> qbeg(pl.nchunk + 1);
     for (int c = 0; c <= pl.nchunk; ++c) qbeg[c] = std::min(h.nquad, c * qpc);
-    for (int c = 0; c < pl.nchunk; ++c) {
-        for (int q = qbeg[c]; q < qbeg[c + 1]; ++q) {
-            if (q == qbeg[c] || h.key[q] != h.key[q - 1]) seg.push_back(make_int4(h.key[q], q, q, 0));
-            seg.back().z = q + 1;
-        }
-        sbeg.push_back((int)seg.size());
-    }
+    std::vector<int4> run;
+    std::vector<int> rbeg;
+    build_runs(h, qbeg, pl.warps, run, rbeg);
+    for (int c = 0; c < pl.nchunk; ++c)
+        for (int r = rbeg[c * pl.warps]; r < rbeg[(c + 1) * pl.warps]; ++r) run[r].w = (run[r].y - qbeg[c]) * 32;
     const int32_t* rp = (const int32_t*)v.a[CG_RPTR];
     const int32_t* pp = (const int32_t*)v.a[CG_PPTR];
     const int32_t* rsp = (const int32_t*)v.a[CG_RSP];
@@ -426,25 +426,26 @@ cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
                 net[k] = 0.0;
             }
     }
-    std::vector<size_t> len(ns, 0);
-    for (int k = 0; k < ns; ++k)
-        for (int c = 0; c < pl.nchunk; ++c) len[k] += ListBuilder::length(lists[c][k]);
-    const std::vector<std::vector<int>> quads = ListBuilder::group(len, pl.warps);
+    // (with several chunks, grouped by the lists over all of them)
+    std::vector<ListBuilder::List> all(ns);
+    for (const auto& l : lists)
+        for (int k = 0; k < ns; ++k) all[k].insert(all[k].end(), l[k].begin(), l[k].end());
+    std::vector<const ListBuilder::List*> al;
+    for (const auto& l : all) al.push_back(&l);
+    const std::vector<std::vector<int>> quads = ListBuilder::group(al, pl.warps);
     pl.nsq = (int)quads.size();
-    std::vector<int> sid(4 * pl.nsq, -1);
     ListBuilder lb;
-    for (int s = 0; s < pl.nsq; ++s)
-        for (size_t g = 0; g < quads[s].size(); ++g) sid[4 * s + g] = quads[s][g];
     for (int c = 0; c < pl.nchunk; ++c)
         for (const std::vector<int>& q : quads) {
             std::vector<const ListBuilder::List*> own;
             for (int k : q) own.push_back(&lists[c][k]);
-            lb.add_quad(own, pl.rows);
+            lb.add_quad(own, q, pl.rows);
         }
+    if (!lb.fits) return cudaErrorNotSupported;
     Image im;
-    const size_t o_rec = im.put(mixed ? h.rec2 : h.rec), o_seg = im.put(seg), o_efl = im.put(h.efl), o_eff = im.put(h.eff);
-    const size_t o_fall = im.put(mixed ? h.fall2 : h.fall), o_sb = im.put(sbeg), o_th = im.put(quad_thermo_rows(v)), o_sid = im.put(sid);
-    const size_t o_li = im.put(lb.info), o_le = im.put(lb.ent), o_lg = im.put(lb.gen);
+    const size_t o_rec = im.put(mixed ? h.rec2 : h.rec), o_run = im.put(run), o_efl = im.put(h.efl), o_eff = im.put(h.eff);
+    const size_t o_fall = im.put(mixed ? h.fall2 : h.fall), o_rb = im.put(rbeg), o_th = im.put(quad_thermo_rows(v));
+    const size_t o_li = im.put(lb.own), o_le = im.put(lb.ent), o_lg = im.put(lb.gen);
     QuadPlan* q = new QuadPlan(pl);
     e = im.upload(&q->dbuf);
     if (e == cudaSuccess)
@@ -457,16 +458,13 @@ cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     }
     char* d = (char*)q->dbuf;
     q->rec = (const QRec*)(d + o_rec);
-    q->seg = (const int4*)(d + o_seg);
+    q->run = (const int4*)(d + o_run);
     q->efl = (const int2*)(d + o_efl);
     q->eff = (const QEff*)(d + o_eff);
     q->fall = (const QFall*)(d + o_fall);
-    q->sbeg = (const int*)(d + o_sb);
+    q->rbeg = (const int*)(d + o_rb);
     q->th = (const double*)(d + o_th);
-    q->sid = (const int*)(d + o_sid);
-    q->lists.info = (const int4*)(d + o_li);
-    q->lists.ent = (const uint4*)(d + o_le);
-    q->lists.gen = (const QGen*)(d + o_lg);
+    q->lists = QLists{(const QOwn*)(d + o_li), (const uint4*)(d + o_le), (const QGen*)(d + o_lg)};
     *out = q;
     return cudaSuccess;
 }
@@ -484,7 +482,7 @@ cudaError_t launch_getrates_quad(const QuadPlan* p, const DevMech& m, const doub
     if (n1 <= i0) return cudaSuccess;
     const int64_t tiles = (n1 - i0 + kQP - 1) / kQP;
     const unsigned grid = (unsigned)std::min<int64_t>(tiles, p->grid);
-    const QuadView v{p->nchunk, p->nsq, p->rows, p->rec, p->seg, p->efl, p->eff, p->fall, p->sbeg, p->th, p->sid, p->lists};
+    const QuadView v{p->nchunk, p->nsq, p->rows, p->rec, p->run, p->efl, p->eff, p->fall, p->rbeg, p->th, p->lists};
     // Every plan of the same kernel instance (one per handle) has its own
     // shared-memory size: the limit is set and the kernel launched under one
     // lock, so that a handle made later for a smaller mechanism cannot leave

@@ -87,9 +87,9 @@ __device__ __forceinline__ double q_rcp(double x) {
 
 // One reaction, 48 bytes.  s, p: byte offset (species * kQRow) of each
 // reactant and product molecule's row of the state; unused slots name the
-// dummy species ns (C = EGp = 1, G = 0).  The first 32 bytes are all that an
-// elementary reaction with at most two molecules a side needs.  FP64 tables
-// hold ln|A|, b, Ea/Rc; mixed ones log2|A|, b, (Ea/Rc) log2 e.
+// dummy species ns (C = EGp = 1, G = 0).  FP64 tables hold
+// ln|A|, b, Ea/Rc; mixed ones log2|A|, b, (Ea/Rc) log2 e.  An elementary
+// reaction with at most two molecules a side needs the first 32 bytes only.
 struct __align__(16) QRec {
     double lnA, b, th;
     unsigned short s[2], p[2];         // the first two molecules of each side
@@ -116,9 +116,9 @@ struct __align__(16) QFall {
 static_assert(sizeof(QFall) == 64, "QFall must stay 64 bytes");
 
 // Class of a quad's reactions: kind | kQWide (three molecules on a side that
-// counts) | kQRev.  A segment is a run of quads of one class; eff of a quad
-// is {first efficiency, number of them}.
+// counts) | kQRev.
 constexpr int kQWide = 16, kQRev = 32;
+constexpr unsigned kQNone = 0xffffffffu;   // QRec.r of a repeat that fills a quad
 
 // Weighted entry of a row list (net coefficients other than +-1).
 struct __align__(16) QGen {
@@ -128,19 +128,36 @@ struct __align__(16) QGen {
 
 // Row lists.  A quad is either four owners (species, matrix entries), one to a
 // quarter-warp, or one owner with a long list split four ways, whose parts
-// are added by shuffles.  For each quarter-warp the quad holds n8 steps of
-// eight 16-bit rows from `ptr` (uint4 per step and quarter-warp): n4neg
-// half-steps of rows to subtract, then rows to add, then rows of zeros; and
-// ngen weighted entries from gptr.
-//   info = {ptr, n4neg | n8 << 16, gptr, ngen | kListWide}
-constexpr int kListWide = 1 << 30;
+// are added by shuffles.  An owner's list is n4 half-steps of four 16-bit rows
+// -- n4neg half-steps of rows to subtract, then rows to add -- two to a step,
+// and ngen weighted entries.  The first step is in the owner's record, so
+// that a short list costs one load, which the loop over quads makes a quad
+// ahead; the others follow at ent[ptr], uint4 per step and quarter-warp.
+struct __align__(16) QOwn {
+    int own;                           // what the sum is for; < 0: nothing
+    unsigned cnt;                      // n4neg | n4 << 16 | kOwnWide
+    int ptr;
+    unsigned gen;                      // first weighted entry / kQG | ngen << 20
+    uint4 rows;
+};
+static_assert(sizeof(QOwn) == 32, "QOwn must stay 32 bytes");
+constexpr unsigned kOwnWide = 1u << 31;
 struct QLists {
-    const int4* info;
+    const QOwn* own;                   // [4 quads]
     const uint4* ent;
     const QGen* gen;
 };
 
-template <bool ALL>
+__device__ __forceinline__ QOwn load_qown(const QOwn* p) {
+    const uint4* q = reinterpret_cast<const uint4*>(p);
+    QOwn o;
+    uint4* d = reinterpret_cast<uint4*>(&o);
+    d[0] = __ldg(q);
+    d[1] = __ldg(q + 1);
+    return o;
+}
+
+template <bool ALL = true>
 __device__ __forceinline__ QRec load_qrec(const QRec* p) {
     const int4* q = reinterpret_cast<const int4*>(p);
     QRec r;
@@ -168,40 +185,45 @@ __device__ __forceinline__ double2 quad_row(const double2* ce, unsigned off) {
 }
 
 // Sum of the row list of this quarter-warp's owner.  `rows` points at this
-// lane's point of row 0 (a row is kQP doubles).  Steps are loaded two ahead:
-// a list of a large mechanism comes from L2, and with one step in flight the
-// longest list alone took longer than the reactions.
-__device__ __forceinline__ double list_sum(const QLists& L, int4 in, int g, const double* rows) {
-    const uint4* e = L.ent + in.x + g;
-    const int neg = in.y & 0xffff, n = (int)((unsigned)in.y >> 16);
-    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
-    uint4 w0 = n > 0 ? __ldg(e) : none, w1 = n > 1 ? __ldg(e + kQG) : none;
-    double acc = 0.0;
+// lane's point of row 0 (a row is kQP doubles).  Steps after the first are
+// loaded two ahead: with one in flight, a large mechanism's longest list,
+// coming from L2, took longer than its reactions.
+__device__ __forceinline__ double list_sum(const QLists& L, const QOwn& o, int g, const double* rows) {
+    const int neg = (int)(o.cnt & 0xffffu), n4 = (int)((o.cnt >> 16) & 0x7fffu);
     auto row = [&](unsigned r) { return rows[r * kQP]; };
-    auto step = [&](int k, const uint4& c) {
-        const double x0 = row(c.x & 0xffffu), x1 = row(c.x >> 16), x2 = row(c.y & 0xffffu), x3 = row(c.y >> 16);
-        const double x4 = row(c.z & 0xffffu), x5 = row(c.z >> 16), x6 = row(c.w & 0xffffu), x7 = row(c.w >> 16);
-        if (2 * k == neg) acc = -acc;
-        acc += (x0 + x1) + (x2 + x3);
-        if (2 * k + 1 == neg) acc = -acc;
-        acc += (x4 + x5) + (x6 + x7);
+    auto half = [&](unsigned a, unsigned b, bool minus) {
+        const double x = (row(a & 0xffffu) + row(a >> 16)) + (row(b & 0xffffu) + row(b >> 16));
+        return minus ? -x : x;
     };
-    for (int k = 0; k < n; k += 2) {
-        const uint4 c0 = w0, c1 = w1;
-        e += 2 * kQG;
-        if (k + 2 < n) w0 = __ldg(e);
-        if (k + 3 < n) w1 = __ldg(e + kQG);
-        step(k, c0);
-        if (k + 1 < n) step(k + 1, c1);
+    double acc = half(o.rows.x, o.rows.y, neg > 0);
+    if (n4 > 1) acc += half(o.rows.z, o.rows.w, neg > 1);
+    if (n4 > 2) {
+        const int n = (n4 + 1) >> 1;
+        auto step = [&](double x, int k, const uint4& c) {
+            x += half(c.x, c.y, 2 * k < neg);
+            return x + half(c.z, c.w, 2 * k + 1 < neg);    // rows of zeros past n4
+        };
+        const uint4* e = L.ent + o.ptr + g;
+        uint4 w0 = __ldg(e), w1 = n > 2 ? __ldg(e + kQG) : w0;
+        for (int k = 1; k < n; k += 2) {
+            const uint4 c0 = w0, c1 = w1;
+            e += 2 * kQG;
+            if (k + 2 < n) w0 = __ldg(e);
+            if (k + 3 < n) w1 = __ldg(e + kQG);
+            acc = step(acc, k, c0);
+            if (k + 1 < n) acc = step(acc, k + 1, c1);
+        }
     }
-    if (2 * n == neg) acc = -acc;
-    const QGen* ge = L.gen + in.z + g;
-    const int ngen = in.w & (kListWide - 1);
-    for (int k = 0; k < ngen; ++k) {
-        const double2 v = __ldg(reinterpret_cast<const double2*>(ge + kQG * k));
-        acc = fma(v.x, row((unsigned)__double2loint(v.y)), acc);
+    const int ngen = (int)(o.gen >> 20);
+    if (ngen) {
+        const double2* ge = reinterpret_cast<const double2*>(L.gen + kQG * (o.gen & 0xfffffu) + g);
+        for (int k = 0; k < ngen; k += 2) {                 // padded to pairs
+            const double2 v0 = __ldg(ge + kQG * k), v1 = __ldg(ge + kQG * (k + 1));
+            acc = fma(v0.x, row((unsigned)__double2loint(v0.y)), acc);
+            acc = fma(v1.x, row((unsigned)__double2loint(v1.y)), acc);
+        }
     }
-    if (in.w & kListWide) {
+    if (o.cnt & kOwnWide) {
         acc += __shfl_xor_sync(0xffffffffu, acc, 8);
         acc += __shfl_xor_sync(0xffffffffu, acc, 16);
     }
@@ -248,6 +270,29 @@ __device__ __forceinline__ double quad_falloff(int kind, const QRec& R, const QF
     return cgm::cg_exp_clamped(lkinf + lnF) * (Pr * q_rcp(1.0 + Pr));
 }
 
+// A tile's T, ln T, 1/T and P, [4][8] in shared memory.  One warp forms the
+// next tile's while the others evaluate reactions: ln T in every warp was a
+// tenth of a 53-species tile's instructions.
+__device__ __forceinline__ void quad_head(double* h, int64_t i, int64_t n, const double* P, const double* Tg) {
+    const int p = threadIdx.x & (kQP - 1);
+    const double T = i < n ? __ldcs(Tg + i) : 1000.0;
+    h[p] = T;
+    h[kQP + p] = cgm::cg_log(T);
+    h[2 * kQP + p] = fmin(cgm::cg_rcp(T), kQMaxInvT);
+    h[3 * kQP + p] = i < n ? __ldcs(P + i) : kPatm;
+}
+
+// Sum over the warps' parts sRed[w][8], each quarter-warp a share of them.
+template <int W>
+__device__ __forceinline__ double quad_total(const double* red, int g) {
+    double x = 0.0;
+    const int p = threadIdx.x & (kQP - 1);
+#pragma unroll
+    for (int w = 0; w < W / kQG; ++w) x += red[(kQG * w + g) * kQP + p];
+    x += __shfl_xor_sync(0xffffffffu, x, 8);
+    return x + __shfl_xor_sync(0xffffffffu, x, 16);
+}
+
 // ------------------------------------------------------------------ host
 // The reactions sorted into quads.
 struct HostQuads {
@@ -275,7 +320,9 @@ inline std::vector<double> quad_thermo_rows(const cg_mech_view& v) {
     return th;
 }
 
-inline void build_quads(const cg_mech_view& v, HostQuads& h) {
+// `products`: a side of three products makes a reaction wide even when it is
+// irreversible (the adjoint reads every product).
+inline void build_quads(const cg_mech_view& v, HostQuads& h, bool products = false) {
     const int ns = h.ns = (int)v.s[CG_S_NS], nr = h.nr = (int)v.s[CG_S_NR];
     const int32_t* flags = (const int32_t*)v.a[CG_FLAGS];
     const int32_t* rp = (const int32_t*)v.a[CG_RPTR];
@@ -345,7 +392,7 @@ inline void build_quads(const cg_mech_view& v, HostQuads& h) {
         if (ok) {
             it.b.lnA = std::log2(std::fabs(arh[3 * r]));
             it.b.th = it.a.th * kLog2e;
-            const bool wide = n[0] > 2 || (rev && n[1] > 2);
+            const bool wide = n[0] > 2 || ((rev || products) && n[1] > 2);
             it.key = kind | (wide ? kQWide : 0) | (rev ? kQRev : 0);
         } else {
             it.key = kQKindGeneric;
@@ -380,10 +427,18 @@ inline void build_quads(const cg_mech_view& v, HostQuads& h) {
                 h.eff.push_back(q);
             }
         for (size_t g = 0; g < kQG; ++g) {
-            // a quad short of four repeats its last reaction; no list names the repeats
+            // a quad short of four repeats its last reaction on the dummy
+            // species: no list names the repeats, and their adjoint is zero
             const Item& it = items[std::min(i + g, e - 1)];
-            h.rec.push_back(it.a);
-            h.rec2.push_back(it.b);
+            QRec a = it.a, b = it.b;
+            if (i + g >= e) {
+                for (QRec* x : {&a, &b}) {
+                    x->s[0] = x->s[1] = x->p[0] = x->p[1] = x->s2 = x->p2 = (unsigned short)(ns * kQRow);
+                    x->r = kQNone;
+                }
+            }
+            h.rec.push_back(a);
+            h.rec2.push_back(b);
             if (i + g < e) h.at[it.r] = 4 * h.nquad + (int)g;
         }
         h.key.push_back(items[i].key);
@@ -436,9 +491,10 @@ struct ListBuilder {
     using List = std::vector<std::pair<int, double>>;
     static constexpr size_t kListSplit = 24;
 
-    std::vector<int4> info;
+    std::vector<QOwn> own;
     std::vector<uint4> ent;
     std::vector<QGen> gen;
+    bool fits = true;                  // every count fits its field
 
     // steps of one owner's rows and coefficients: +-1, +-2, +-3 as repeated
     // rows, others weighted
@@ -466,24 +522,39 @@ struct ListBuilder {
         return n;
     }
 
-    // own: one list, split four ways, or up to four lists
-    void add_quad(const std::vector<const List*>& own, int zero) {
+    static size_t weighted(const List& l) {
+        size_t n = 0;
+        for (const auto& x : l) {
+            const double a = std::fabs(x.second);
+            n += a != 0.0 && a != 1.0 && a != 2.0 && a != 3.0;
+        }
+        return n;
+    }
+
+    // One owner's list, split four ways, or those of two to four owners;
+    // `zero` is a row of zeros.
+    void add_quad(const std::vector<const List*>& lists, const std::vector<int>& what, int zero) {
         Split q[kQG];
-        if (own.size() == 1) split(*own[0], q, kQG);
+        const bool wide = lists.size() == 1;
+        if (wide) split(*lists[0], q, kQG);
         else
-            for (size_t g = 0; g < own.size(); ++g) split(*own[g], q + g, 1);
+            for (size_t g = 0; g < lists.size(); ++g) split(*lists[g], q + g, 1);
         size_t np = 0, nn = 0, ng = 0;
         for (int g = 0; g < kQG; ++g) {
             np = std::max(np, (q[g].pos.size() + 3) / 4);
             nn = std::max(nn, (q[g].neg.size() + 3) / 4);
             ng = std::max(ng, q[g].ge.size());
         }
-        const size_t n8 = (np + nn + 1) / 2;
-        int4 in;
-        in.x = (int)ent.size();
-        in.y = (int)((unsigned)nn | (unsigned)n8 << 16);
-        in.z = (int)gen.size();
-        in.w = (int)ng | (own.size() == 1 ? kListWide : 0);
+        ng = (ng + 1) / 2 * 2;
+        const size_t n4 = np + nn, n8 = std::max<size_t>((n4 + 1) / 2, 1);
+        fits = fits && nn < 0xffff && n4 < 0x7fff && ng < 0xfff && gen.size() / kQG < 0xfffff;
+        QOwn o[kQG];
+        for (int g = 0; g < kQG; ++g) {
+            o[g].own = wide ? what[0] : g < (int)what.size() ? what[g] : -1;
+            o[g].cnt = (unsigned)nn | (unsigned)n4 << 16 | (wide ? kOwnWide : 0u);
+            o[g].ptr = (int)ent.size();
+            o[g].gen = (unsigned)(gen.size() / kQG) | (unsigned)ng << 20;
+        }
         for (size_t k = 0; k < n8; ++k)
             for (int g = 0; g < kQG; ++g) {
                 unsigned r[8];
@@ -493,7 +564,9 @@ struct ListBuilder {
                     const size_t j = 4 * (h < nn ? h : h - nn) + u % 4;
                     r[u] = j < l.size() ? (unsigned)l[j] : (unsigned)zero;
                 }
-                ent.push_back(make_uint4(r[0] | r[1] << 16, r[2] | r[3] << 16, r[4] | r[5] << 16, r[6] | r[7] << 16));
+                const uint4 w = make_uint4(r[0] | r[1] << 16, r[2] | r[3] << 16, r[4] | r[5] << 16, r[6] | r[7] << 16);
+                if (k == 0) o[g].rows = w;
+                else ent.push_back(w);
             }
         for (size_t k = 0; k < ng; ++k)
             for (int g = 0; g < kQG; ++g) {
@@ -504,23 +577,37 @@ struct ListBuilder {
                 x.pad = 0;
                 gen.push_back(x);
             }
-        info.push_back(in);
+        own.insert(own.end(), o, o + kQG);
     }
 
-    // Groups owners 0 .. n-1 of lengths len into quads and orders the quads
-    // for `warps` warps; each quad lists its owners.
-    static std::vector<std::vector<int>> group(const std::vector<size_t>& len, int warps) {
-        std::vector<int> own(len.size());
-        for (size_t k = 0; k < len.size(); ++k) own[k] = (int)k;
-        std::stable_sort(own.begin(), own.end(), [&](int a, int b) { return len[a] > len[b]; });
+    // Groups the owners of the lists into quads and orders the quads for
+    // `warps` warps; each quad names its owners.
+    static std::vector<std::vector<int>> group(const std::vector<const List*>& lists, int warps) {
+        const size_t no = lists.size();
+        std::vector<size_t> len(no), wt(no);
+        std::vector<int> own(no);
+        for (size_t k = 0; k < no; ++k) {
+            own[k] = (int)k;
+            len[k] = length(*lists[k]);
+            wt[k] = weighted(*lists[k]);
+        }
+        // long lists first, then lists with weighted entries together
+        std::stable_sort(own.begin(), own.end(), [&](int a, int b) {
+            const bool la = len[a] > kListSplit, lb = len[b] > kListSplit;
+            if (la != lb) return la;
+            if (!la && wt[a] != wt[b]) return wt[a] > wt[b];
+            return len[a] > len[b];
+        });
         std::vector<std::vector<int>> quads;
         std::vector<size_t> cost;
         for (size_t k = 0; k < own.size();) {
             std::vector<int> q{own[k]};
-            const size_t l = len[own[k++]];
+            size_t l = len[own[k++]];
             if (l <= kListSplit)
-                while (q.size() < (size_t)kQG && k < own.size()) q.push_back(own[k++]);
-            // a lone last owner shares its quad with nobody: it is split like a long one
+                while (q.size() < (size_t)kQG && k < own.size()) {
+                    l = std::max(l, len[own[k]]);
+                    q.push_back(own[k++]);
+                }
             cost.push_back(12 + (q.size() == 1 ? l / 4 : l));
             quads.push_back(q);
         }
@@ -543,6 +630,26 @@ struct ListBuilder {
         return out;
     }
 };
+
+// Runs: the quads of one class that one warp takes, quads first, first + W,
+// ....  Quad q of a chunk runs on warp (q - chunk's first) mod W; each warp has
+// the list of its runs, so that a loop over one class holds no dispatch and
+// no warp looks at classes it has no quad of.
+//   run = {class, first quad, how many, 0}; of warp w in chunk c:
+//   run[beg[c W + w]] .. run[beg[c W + w + 1] - 1]
+inline void build_runs(const HostQuads& h, const std::vector<int>& qbeg, int warps, std::vector<int4>& run,
+                       std::vector<int>& beg) {
+    beg.assign(1, 0);
+    for (size_t c = 0; c + 1 < qbeg.size(); ++c)
+        for (int w = 0; w < warps; ++w) {
+            const size_t first = run.size();
+            for (int q = qbeg[c] + w; q < qbeg[c + 1]; q += warps) {
+                if (run.size() == first || run.back().x != h.key[q]) run.push_back(make_int4(h.key[q], q, 0, 0));
+                ++run.back().z;
+            }
+            beg.push_back((int)run.size());
+        }
+}
 
 // Host image of a plan's tables, copied to the device in one piece.
 struct Image {

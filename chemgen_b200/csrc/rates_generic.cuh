@@ -126,7 +126,7 @@ __device__ __forceinline__ double plog_kf(const DevMech& m, int row, double P, d
 
 // Net rate of progress of reaction r; C and EGp are read with stride B.
 template <int B>
-__device__ __noinline__ double generic_rate(const DevMech& m, unsigned r, const PointT& pt, double P, double lnP,
+__device__ __noinline__ double generic_rate(const DevMech& m, unsigned r, PointT pt, double P, double lnP,
                                             double ctot, const double* C, const double* E) {
     const DRxn R = load_rxn(m.rxn + r);
     int kind = CG_STANDARD;

@@ -114,18 +114,18 @@ int chemgen_kernel_kind(chemgen_handle* h, int mode);
  * prototype chemgen/chemistry_nn.py:15-85 never ran).
  * chemgen_jacobian: dense d wdot/d(T, Y) per point, J[(k*(ns+1) + c)*ng + i],
  *   column c = 0 for T, 1 + j for Y_j; precision 0 = double, 1 = float
- *   (FP64 rate evaluation and accumulation, J stored in FP32).  Each row is
- *   accumulated on chip and J is written once when a 32-point tile's state
- *   and two rows fit in shared memory (up to ~180 species); each tile's
- *   reaction derivatives or rate constants go to library-owned scratch of
- *   8*nr*32 doubles per SM (about 100 MB at 325 reactions).  Larger
- *   mechanisms accumulate J in place with library-owned scratch of 4*ns*ng
- *   doubles (FP32 accumulation for precision 1).
+ *   (FP64 rate evaluation and accumulation, J stored in FP32).  J is written
+ *   once, without scratch, when an eight-point tile's derivatives fit in shared
+ *   memory (about 520 reactions).  Otherwise each row is accumulated on chip
+ *   when a 32-point tile's state and two rows fit (up to ~180 species), each
+ *   tile's reaction derivatives going to library-owned scratch of 8*nr*32
+ *   doubles per SM; larger mechanisms accumulate J in place with library-owned
+ *   scratch of 4*ns*ng doubles (FP32 accumulation for precision 1).
  * chemgen_getrates_vjp: given G = dL/dwdot [ns*ng], the adjoint
  *   gT = dL/dT [ng], gY = dL/dY [ns*ng] and (if gP != NULL) gP = dL/dP [ng],
- *   without forming J: up to ~110 species with each 32-point tile's state in
- *   shared memory and a result that does not depend on scheduling, beyond
- *   that with library-owned scratch of 4*ns*ng doubles. */
+ *   without forming J: on eight-point tiles in shared memory, without scratch
+ *   and with a result that does not depend on scheduling (up to ~500
+ *   species), beyond that with library-owned scratch of 4*ns*ng doubles. */
 int chemgen_jacobian(chemgen_handle* h, int precision, const double* P, const double* T, int64_t ng,
                      const double* Y, void* J, void* stream);
 int chemgen_getrates_vjp(chemgen_handle* h, const double* P, const double* T, int64_t ng, const double* Y,

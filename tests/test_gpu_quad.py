@@ -49,3 +49,38 @@ def test_every_kind_and_general_stoichiometry():
     rx[3].reactants, rx[3].products = {s[4]: 1.0}, {s[5]: 2.0, s[6]: 1.0, s[7]: 1.0}
     rx[3].reversible = False
     _check(mech, 83)
+
+
+def _derivatives(mech, ng, seed=0):
+    """(Jacobian, adjoint) of the kernels and of autograd through the FP64 law."""
+    import torch
+    from oracle import torch_ref
+    P, T, Y = _cuda(*synthetic.states(mech.ns, ng, seed=seed))
+    gm = GpuMechanism(mech)
+    G = torch.randn(mech.ns, ng, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(seed))
+    p, t, y = (x.clone().requires_grad_(True) for x in (P, T, Y))
+    w = torch_ref.getrates(mech, p, t, y)
+    gP, gT, gY = torch.autograd.grad(w, (p, t, y), G, retain_graph=True)
+    J = torch.empty(mech.ns, mech.ns + 1, ng, dtype=torch.float64, device="cuda")
+    for k in range(mech.ns):
+        J[k, 0], J[k, 1:] = torch.autograd.grad(w[k].sum(), (t, y), retain_graph=True)
+    return (gm.jacobian(P, T, Y), gm.jacobian(P, T, Y, precision="fp32").double(), gm.vjp(P, T, Y, G)), (J, (gT, gY, gP))
+
+
+def _rel(x, ref):
+    # per point, relative to the point's largest value (columns of J by column T and the rest)
+    d = (x - ref).abs().reshape(-1, ref.shape[-1]).amax(0)
+    return float((d / ref.abs().reshape(-1, ref.shape[-1]).amax(0).clamp_min(1e-300)).max())
+
+
+@pytest.mark.parametrize("name,ng", [("all_kinds", 1), ("all_kinds", 19), ("chunks", 9)])
+def test_derivatives_of_every_kind(name, ng):
+    # 1e-9: the bar of the derivative tests; FP32 storage 1e-6 (half an ulp is 6e-8)
+    mech = synthetic.all_kinds() if name == "all_kinds" else synthetic.synthetic_mechanism(30, 900, 30, 30, seed=3)
+    (J64, J32, v), (J, r) = _derivatives(mech, ng, seed=ng)
+    for sl in (slice(0, 1), slice(1, None)):
+        assert _rel(J64[:, sl], J[:, sl]) <= 1e-9
+        assert _rel(J32[:, sl], J[:, sl]) <= 1e-6
+    gT, gY, gP = v
+    assert _rel(gY, r[1]) <= 1e-9
+    assert _rel(gT[None], r[0][None]) <= 1e-7 and _rel(gP[None], r[2][None]) <= 1e-7
