@@ -22,7 +22,9 @@ int fp64_smem_block(int ns, size_t smem_per_sm, size_t smem_per_block, long* pts
 size_t fp64_global_slice_bytes(int ns);
 int fp64_global_blocks_per_sm();
 struct QuadPlan;
-cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, int mixed, QuadPlan** out);
+cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, int mixed, int latency,
+                         QuadPlan** out);
+int quad_tile_points();
 void quad_release(QuadPlan* p);
 cudaError_t launch_getrates_quad(const QuadPlan* p, const DevMech& m, const double* P, const double* T,
                                  const double* Y, double* wdot, int64_t i0, int64_t ng, int64_t n1, cudaStream_t s,
@@ -62,6 +64,8 @@ struct chemgen_handle {
     // kernels generated for this exact mechanism (generate_chemistry.py --language cuda)
     chemgen_kernel_fn gen_fn = nullptr;
     unsigned gen_modes = 0;
+    chemgen_kernel_range_fn gen_range[2] = {nullptr, nullptr};   // [mode] the same kernels over a range of points
+    int gen_block[2] = {0, 0};                                   // points per SM and wave
     int use_generated = 1;
     int gen_version = -1;
     int ns = 0, nr = 0;
@@ -70,7 +74,10 @@ struct chemgen_handle {
     void* dbuf = nullptr;
     int sm_count = 0;
     int fp64_block = 0;             // 32/64/128: shared-memory state; 0: quad kernel or global scratch
-    cg::QuadPlan* quad = nullptr;       // FP64 kernel on eight-point tiles (state on chip)
+    // kernels on eight-point tiles (state on chip): [mode][0] for throughput,
+    // [mode][1] the same with more warps to a tile, for batches of few tiles;
+    // mode 1 (the generated mixed kernel's arithmetic) serves generated handles
+    cg::QuadPlan* quad[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     cg::GradPlan* jacq = nullptr;       // Jacobian on eight-point tiles when every reaction's rows fit
     cg::GradPlan* vjpq = nullptr;       // adjoint on eight-point tiles
     cg::JacPlan* jac = nullptr;         // row-owner Jacobian (J written once) otherwise, when its tile fits
@@ -114,8 +121,10 @@ bool aligned8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0
 struct Registered {
     uint64_t fp;
     int ns, nr;
-    unsigned modes;
+    unsigned modes;                 // fn: bit per mode; range: the mode
     chemgen_kernel_fn fn;
+    chemgen_kernel_range_fn range;
+    int block;
 };
 std::mutex& reg_mu() {
     static std::mutex m;
@@ -143,8 +152,13 @@ void refresh_generated(chemgen_handle* h) {
     h->gen_version = g_reg_version;
     for (const Registered& r : registry())
         if (r.fp == h->fingerprint && r.ns == h->ns && r.nr == h->nr) {
-            h->gen_fn = r.fn;
-            h->gen_modes = r.modes;
+            if (r.fn) {
+                h->gen_fn = r.fn;
+                h->gen_modes = r.modes;
+            } else {
+                h->gen_range[r.modes] = r.range;
+                h->gen_block[r.modes] = r.block;
+            }
         }
 }
 
@@ -159,6 +173,14 @@ struct Builder {
         return off;
     }
 };
+
+void release_quads(chemgen_handle* h) {
+    for (auto& mode : h->quad)
+        for (cg::QuadPlan*& p : mode) {
+            cg::quad_release(p);
+            p = nullptr;
+        }
+}
 
 int build_tables(const cg_mech_view& v, chemgen_handle* h) {
     using namespace cg;
@@ -361,7 +383,7 @@ int ensure_ws_locked(chemgen_handle* h, size_t bytes) {
 }
 
 size_t fp64_ws_bytes(const chemgen_handle* h, int64_t ng) {
-    if (h->fp64_block || h->quad) return 0;
+    if (h->fp64_block || h->quad[0][0]) return 0;
     int64_t chunks = (ng + 63) / 64;
     int64_t slices = std::min<int64_t>(chunks, h->fp64_slices);
     return (size_t)slices * cg::fp64_global_slice_bytes(h->ns);
@@ -383,6 +405,44 @@ int check_args(const chemgen_handle* h, const double* P, const double* T, int64_
     return CHEMGEN_OK;
 }
 
+// Points [i0, ng) on the tile kernel: the plan with more warps to a tile when
+// every tile has an SM to itself.
+int launch_tiles(chemgen_handle* h, int mode, const double* P, const double* T, int64_t i0, int64_t ng,
+                 const double* Y, double* w, cudaStream_t s) {
+    const int64_t tiles = (ng - i0 + cg::quad_tile_points() - 1) / cg::quad_tile_points();
+    const cg::QuadPlan* p = h->quad[mode][1] && tiles <= h->sm_count ? h->quad[mode][1] : h->quad[mode][0];
+    return status_of(cg::launch_getrates_quad(p, h->m, P, T, Y, w, i0, ng, ng, s));
+}
+
+// The generated kernel, one point per thread, takes about as long for one
+// block as for a whole wave of one block per SM; the tile kernel takes time
+// in proportion to its tiles.  So the points past the last whole wave (all of
+// a small batch) run on the tile kernel when that is faster.  Both times,
+// fitted to B200 measurements at 9/23 and 53/325 (us):
+//   wave: FP64 12 and 103, mixed 10 and 68, linear in the reactions;
+//   eight-point tiles, one per SM at a time: FP64 1.6 and 4.7, mixed 1.5 and
+//   5.0, linear in the quads of four reactions (8 and 91).
+// (53/325 FP64: the line lies at 26000 of a wave's 75776 points; there the
+// tile kernel takes 99 us.)
+bool tiles_faster(const chemgen_handle* h, int mode, int64_t n) {
+    const double nr = h->nr, nq = 0.28 * nr, tiles = (double)n / cg::quad_tile_points() / h->sm_count;
+    const double wave = mode ? 5.6 + 0.192 * nr : 5.1 + 0.301 * nr;
+    const double tile = mode ? 1.2 + 0.0418 * nq : 1.3 + 0.0373 * nq;
+    return tiles * tile < wave;
+}
+
+int launch_generated(chemgen_handle* h, int mode, const double* P, const double* T, int64_t ng, const double* Y,
+                     double* w, cudaStream_t s) {
+    if (h->gen_range[mode] && h->quad[mode][0]) {
+        const int64_t wave = (int64_t)h->gen_block[mode] * h->sm_count, full = ng / wave * wave;
+        if (ng > full && tiles_faster(h, mode, ng - full)) {
+            const int st = full ? h->gen_range[mode](mode, P, T, ng, Y, w, 0, full, s) : CHEMGEN_OK;
+            return st ? st : launch_tiles(h, mode, P, T, full, ng, Y, w, s);
+        }
+    }
+    return h->gen_fn(mode, P, T, ng, Y, w, s);
+}
+
 // One launch.  `ws` is scratch the caller provides (may be more or less than
 // ws_bytes_for: the FP64 global variant runs as many persistent blocks as
 // slices fit, at least one).
@@ -391,10 +451,9 @@ int launch(chemgen_handle* h, int mode, const double* P, const double* T, int64_
     refresh_generated(h);
     if (h->use_generated && h->gen_fn && (mode == CHEMGEN_MODE_FP64 || mode == CHEMGEN_MODE_MIXED) &&
         (h->gen_modes & (1u << mode)))
-        return h->gen_fn(mode, P, T, ng, Y, w, s);
+        return launch_generated(h, mode, P, T, ng, Y, w, s);
     if (mode == CHEMGEN_MODE_FP64) {
-        if (!h->fp64_block && h->quad)
-            return status_of(cg::launch_getrates_quad(h->quad, h->m, P, T, Y, w, 0, ng, ng, s));
+        if (!h->fp64_block && h->quad[0][0]) return launch_tiles(h, mode, P, T, 0, ng, Y, w, s);
         int64_t slices = 0;
         if (!h->fp64_block) {
             if (!ws || (reinterpret_cast<uintptr_t>(ws) & 255u)) return CHEMGEN_ERR_INVALID_ARGUMENT;
@@ -501,10 +560,13 @@ int chemgen_create(const void* blob, size_t nbytes, int device, chemgen_handle**
     // its latencies) or none, and it serves the batches whose size is known
     // only on the device (chemgen_getrates_counted).  Beyond it, the
     // global-scratch kernel.
-    e = cg::quad_prepare(h->m, v, device, 0, &h->quad);
-    if (e == cudaSuccess) {
-        if (smem_pts < 256) h->fp64_block = 0;
-    } else if (e != cudaErrorNotSupported) {
+    e = cudaSuccess;
+    for (int mode = 0; mode < 2; ++mode)
+        for (int lat = 0; lat < 2 && (e == cudaSuccess || e == cudaErrorNotSupported); ++lat)
+            e = cg::quad_prepare(h->m, v, device, mode, lat, &h->quad[mode][lat]);
+    if (h->quad[0][0] && smem_pts < 256) h->fp64_block = 0;
+    if (e != cudaSuccess && e != cudaErrorNotSupported) {
+        release_quads(h);
         cudaFree(h->dbuf);
         delete h;
         return status_of(e);
@@ -514,7 +576,7 @@ int chemgen_create(const void* blob, size_t nbytes, int device, chemgen_handle**
     if (e == cudaErrorNotSupported) e = cg::jac_prepare(h->m, v, device, &h->jac);
     if (e != cudaSuccess && e != cudaErrorNotSupported) {
         cg::grad_release(h->vjpq);
-        if (h->quad) cg::quad_release(h->quad);
+        release_quads(h);
         cudaFree(h->dbuf);
         delete h;
         return status_of(e);
@@ -530,7 +592,7 @@ int chemgen_destroy(chemgen_handle* h) {
     DeviceGuard g(h->device);
     cudaDeviceSynchronize();
     if (h->mixed) cg::mixed_release(h->mixed);
-    if (h->quad) cg::quad_release(h->quad);
+    release_quads(h);
     if (h->jac) cg::jac_release(h->jac);
     cg::grad_release(h->jacq);
     cg::grad_release(h->vjpq);
@@ -550,7 +612,17 @@ int chemgen_num_species(const chemgen_handle* h) { return h ? h->ns : -1; }
 int chemgen_register_kernels(uint64_t fingerprint, int ns, int nr, unsigned modes, chemgen_kernel_fn fn) {
     if (!fn || ns <= 0 || nr < 0) return CHEMGEN_ERR_INVALID_ARGUMENT;
     std::lock_guard<std::mutex> lk(reg_mu());
-    registry().push_back(Registered{fingerprint, ns, nr, modes, fn});
+    registry().push_back(Registered{fingerprint, ns, nr, modes, fn, nullptr, 0});
+    ++g_reg_version;
+    return CHEMGEN_OK;
+}
+
+int chemgen_register_kernel_range(uint64_t fingerprint, int ns, int nr, int mode, int block,
+                                  chemgen_kernel_range_fn fn) {
+    if (!fn || ns <= 0 || nr < 0 || block <= 0 || (mode != CHEMGEN_MODE_FP64 && mode != CHEMGEN_MODE_MIXED))
+        return CHEMGEN_ERR_INVALID_ARGUMENT;
+    std::lock_guard<std::mutex> lk(reg_mu());
+    registry().push_back(Registered{fingerprint, ns, nr, (unsigned)mode, nullptr, fn, block});
     ++g_reg_version;
     return CHEMGEN_OK;
 }
@@ -628,9 +700,9 @@ int chemgen_getrates_counted(chemgen_handle* h, const double* P, const double* T
     if (st || ng == 0) return st;
     if (!count) return CHEMGEN_ERR_INVALID_ARGUMENT;
     if (reinterpret_cast<uintptr_t>(count) & 7u) return CHEMGEN_ERR_MISALIGNED;
-    if (!h->quad) return CHEMGEN_ERR_UNSUPPORTED;
+    if (!h->quad[0][0]) return CHEMGEN_ERR_UNSUPPORTED;
     DeviceGuard g(h->device);
-    return status_of(cg::launch_getrates_quad(h->quad, h->m, P, T, Y, wdot, 0, ng, ng, (cudaStream_t)stream,
+    return status_of(cg::launch_getrates_quad(h->quad[0][0], h->m, P, T, Y, wdot, 0, ng, ng, (cudaStream_t)stream,
                                               reinterpret_cast<const unsigned long long*>(count)));
 }
 
@@ -793,7 +865,7 @@ void wrapper_body(double* P, double* Temp, int ng, double* Ysp, double* wdot, do
     // Large mechanisms keep per-point state in scratch: the caller's log_c
     // (ng*ns doubles) when it holds at least one block's slice, otherwise
     // library-owned scratch.
-    if (!h->fp64_block && !h->quad && log_c) {
+    if (!h->fp64_block && !h->quad[0][0] && log_c) {
         uintptr_t a = reinterpret_cast<uintptr_t>(log_c);
         uintptr_t al = (a + 255) & ~(uintptr_t)255;
         size_t bytes = (size_t)ng * h->ns * sizeof(double);

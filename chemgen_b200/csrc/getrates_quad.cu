@@ -19,8 +19,11 @@
 // one reaction a warp, 13 chunks with two barriers each); JetSurf 2.0 3.6 ms;
 // 53/325 on the table-driven path 191 -> 272 Mpts/s.  A loop per class (build_runs)
 // is 18 % faster than a dispatch per quad (3.31 against 4.04 ms at 348/2163).
-// The mixed form repeats the generated mixed kernel's arithmetic reaction by
-// reaction (FP64 exponents and sums, FP32 2^f, products and falloff blend).
+// The mixed form repeats the generated mixed kernel's arithmetic to the last
+// bit: FP64 exponents, FP32 2^f, products and falloff blend, the sums over
+// species and reactions in the generated code's order.  It runs the batches
+// (and the remainders past whole waves) that would leave the generated
+// kernel's wave mostly empty: 53/325, 4096 points, FP64 98 -> 27 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -156,8 +159,11 @@ __device__ __forceinline__ float mix_c(const double2& s) { return __int_as_float
 
 // Net rate of progress, mixed precision: the generated mixed kernel's
 // expressions (emit_cuda.py reaction32, falloff32) with molecules as slots.
-__device__ __forceinline__ double quad_rate_mixed(const QuadView& v, int cls, int q, const QRec& R, int g,
+// CLS: the class when it is known at compile time, else -1.
+template <int CLS>
+__device__ __forceinline__ double quad_rate_mixed(const QuadView& v, int rcls, int q, const QRec& R, int g,
                                                   const MixPt& pt, const double2* ce) {
+    const int cls = CLS < 0 ? rcls : CLS;
     const int kind = cls & 15;
     float Ms = pt.ctot32;
     if (kind != CG_STANDARD) {
@@ -193,22 +199,24 @@ __device__ __forceinline__ double quad_rate_mixed(const QuadView& v, int cls, in
         const float l2m = cgg::lg2f(mpr), l2pr = (float)npr + l2m;
         cgg::falloff_blend(mpr, npr, l2m, l2r, nfix);
         constexpr float kL = 0.30102999566398119521f, kIL = (float)(1.0 / 0.30102999566398119521);
-        float l2F = 0.0f;
+        float l2k = l2r;               // log2 of Pr/(1+Pr) F / 2^nfix
         if (kind == CG_TROE) {
             float Fc = fmaf(c0, cgg::ex2f(c1 * pt.Tf), c2 * cgg::ex2f(c3 * pt.Tf));
             if (c4 != 0.0f) Fc = Fc + cgg::ex2f(c4 * pt.invTf);
             const float lFc = kL * cgg::lg2f(Fc);
             const float lp = kL * l2pr + fmaf(-0.67f, lFc, -0.4f);
             const float f = __fdividef(lp, fmaf(-0.14f, lp, fmaf(-1.27f, lFc, 0.75f)));
-            l2F = kIL * __fdividef(lFc, fmaf(f, f, 1.0f));
+            l2k = fmaf(kIL, __fdividef(lFc, fmaf(f, f, 1.0f)), l2r);
         } else if (kind == CG_SRI) {
             const float lp = kL * l2pr;
             const float X = __fdividef(1.0f, fmaf(lp, lp, 1.0f));
             const float base = fmaf(c0, cgg::ex2f(c1 * pt.invTf), cgg::ex2f(c2 * pt.Tf));
-            l2F = c3 + X * cgg::lg2f(base) + c4 * pt.lnT2f;
+            l2k = l2r + (c3 + X * cgg::lg2f(base) + c4 * pt.lnT2f);
         }
-        akf = ainf + ((double)nfix + (double)(l2r + l2F));
+        akf = ainf + ((double)nfix + (double)l2k);
     }
+    // products and Gibbs sums in the generated code's order: a species that
+    // is on a side twice adds 2 G in one rounding
     const float mf = kind == CG_THIRD_BODY ? Ms : 1.0f;
     const double2 a0 = quad_row(ce, R.s[0]), a1 = quad_row(ce, R.s[1]);
     float cf = mix_c(a0) * mix_c(a1);
@@ -216,21 +224,65 @@ __device__ __forceinline__ double quad_rate_mixed(const QuadView& v, int cls, in
     if (cls & kQWide) {
         const double2 a2 = quad_row(ce, R.s2);
         cf *= mix_c(a2);
-        gs += a2.x;
+        gs = R.s[1] == R.s2 ? a0.x + (a1.x + a2.x) : gs + a2.x;
     }
-    double rr = cgg::rate2(akf, cf * mf, -32 * (int)(R.ord & 0xffu));
+    int n;
+    float f;
+    cgg::split2(akf, n, f);
+    const float e2 = kind <= CG_THIRD_BODY && R.aux ? __uint_as_float(R.aux) : cgg::ex2f(f);
+    double rr = (double)(e2 * (cf * mf)) * cgg::exp2i(n - 32 * (int)(R.ord & 0xffu));   // rate2
+
     if (cls & kQRev) {
         const double2 b0 = quad_row(ce, R.p[0]), b1 = quad_row(ce, R.p[1]);
         float cb = mix_c(b0) * mix_c(b1);
-        gs = (gs - b0.x) - b1.x;
+        const double g0 = R.p[0] == R.p[1] ? gs - (b0.x + b1.x) : (gs - b0.x) - b1.x;
         if (cls & kQWide) {
             const double2 b2 = quad_row(ce, R.p2);
             cb *= mix_c(b2);
-            gs -= b2.x;
+            gs = R.p[1] != R.p2 ? g0 - b2.x : R.p[0] == R.p2 ? fma(-3.0, b0.x, gs) : (gs - b0.x) - (b1.x + b2.x);
+        } else {
+            gs = g0;
         }
         rr -= cgg::rate2(akf + gs, cb * mf, -32 * (int)((R.ord >> 8) & 0xffu));
     }
     return rr;
+}
+
+// The n quads of a run, mixed (see quad_standard).
+template <int W, int CLS>
+__device__ __forceinline__ void quad_run_mixed(const QuadView& v, int cls, int q, int n, int g, const MixPt& pt,
+                                               const double2* ce, double* out) {
+    const QRec* rec = v.rec + kQG * q + g;
+    QRec N = load_qrec(rec);
+    for (; n > 0; --n, q += W, out += 32 * W) {
+        const QRec R = N;
+        rec += kQG * W;
+        if (n > 1) N = load_qrec(rec);
+        *out = quad_rate_mixed<CLS>(v, cls, q, R, g, pt, ce);
+    }
+}
+
+// wdot of this quarter-warp's species, mixed: the reactions' rates added one by
+// one in file order as the generated kernel does (its bits: the two serve
+// batches of different sizes).  Entries: row | {0, 2, 3 for coefficients
+// 1, 2, 3} << 13 | minus << 15.
+__device__ __forceinline__ double sequence_sum(const QLists& L, const QOwn& o, int g, const double* rows) {
+    double acc = 0.0;
+    auto add = [&](unsigned e) {
+        // 1.0, 2.0, 3.0 are 0x3ff00000 + 0x80000 {0, 2, 3}: the entry holds {0, 2, 3}
+        const int hi = (int)((((e & 0x6000u) << 6) + 0x3ff00000u) | ((e & 0x8000u) << 16));
+        acc = fma(__hiloint2double(hi, 0), rows[(e & 0x1fffu) * kQP], acc);
+    };
+    const uint4* q = L.ent + o.ptr + g;
+    const int n = (int)o.cnt;
+    uint4 w = o.rows;
+    for (int k = 0; k < n; ++k) {
+        const uint4 c = w;
+        if (k + 1 < n) w = __ldg(q + kQG * k);
+        add(c.x & 0xffffu), add(c.x >> 16), add(c.y & 0xffffu), add(c.y >> 16);
+        add(c.z & 0xffffu), add(c.z >> 16), add(c.w & 0xffffu), add(c.w >> 16);
+    }
+    return acc;
 }
 
 template <int W, int MINB, bool MIXED>
@@ -287,22 +339,44 @@ __global__ void __launch_bounds__(32 * W, MINB)
             if (MIXED) sCE[k * kQP + p] = make_double2(fma(smh, cgg::kLog2e, lpfac2), c);
             else sCE[k * kQP + p] = make_double2(c, q_exp(smh, sTab) * pfac);
         }
-        part += __shfl_xor_sync(0xffffffffu, part, 8);
-        part += __shfl_xor_sync(0xffffffffu, part, 16);
-        if (g == 0) sRed[warp * kQP + p] = part;
-        __syncthreads();
-        const double csum = quad_total<W>(sRed, g);
-        const double fac = Pp * cgm::cg_rcp(kR0 * csum * T);   // ytoc.j2:3-18
-        const double ctot = csum * fac;
+        double fac, ctot;
+        if (MIXED) {
+            // the generated kernel's order of summation: one warp adds species
+            // after species
+            __syncthreads();
+            if (warp == 0) {
+                double csum = 0.0, ct = 0.0;
+#pragma unroll 4
+                for (int k = 0; k < ns; ++k) csum += sCE[k * kQP + p].y;
+                const double facs = Pp * cgm::cg_rcp(kR0 * csum * T) * 4294967296.0;
+#pragma unroll 4
+                for (int k = 0; k < ns; ++k) ct += sCE[k * kQP + p].y * facs;
+                if (g == 0) {
+                    sRed[p] = facs;
+                    sRed[kQP + p] = ct;
+                }
+            }
+            __syncthreads();
+            fac = sRed[p];             // times 2^32
+            ctot = sRed[kQP + p];
+        } else {
+            part += __shfl_xor_sync(0xffffffffu, part, 8);
+            part += __shfl_xor_sync(0xffffffffu, part, 16);
+            if (g == 0) sRed[warp * kQP + p] = part;
+            __syncthreads();
+            const double csum = quad_total<W>(sRed, g);
+            fac = Pp * cgm::cg_rcp(kR0 * csum * T);            // ytoc.j2:3-18
+            ctot = csum * fac;
+        }
         for (int k = 4 * warp + g; k < ns; k += 4 * W) {
             if (MIXED) {
-                const float c = (float)(sCE[k * kQP + p].y * (fac * 4294967296.0));
+                const float c = (float)(sCE[k * kQP + p].y * fac);
                 sCE[k * kQP + p].y = __hiloint2double(0, __float_as_int(c));
             } else {
                 sCE[k * kQP + p].x *= fac;
             }
         }
-        mp.ctot32 = (float)(ctot * 4294967296.0);
+        mp.ctot32 = (float)ctot;           // mixed: scaled by 2^32
         mp.Tf = (float)T;
         mp.invTf = (float)pt.invT;
         mp.lnT2f = (float)mp.lnT2;
@@ -316,8 +390,13 @@ __global__ void __launch_bounds__(32 * W, MINB)
                 const int cls = __shfl_sync(0xffffffffu, rn.x, 0), n = __shfl_sync(0xffffffffu, rn.z, 0);
                 double* out = sQ + rn.w + lane;
                 if (MIXED) {
-                    for (int j = 0, q = rn.y; j < n; ++j, q += W)
-                        out[j * 32 * W] = quad_rate_mixed(v, cls, q, load_qrec(v.rec + kQG * q + g), g, mp, ce);
+                    switch (cls) {
+                        case 0: quad_run_mixed<W, 0>(v, cls, rn.y, n, g, mp, ce, out); break;
+                        case kQRev: quad_run_mixed<W, kQRev>(v, cls, rn.y, n, g, mp, ce, out); break;
+                        case kQWide: quad_run_mixed<W, kQWide>(v, cls, rn.y, n, g, mp, ce, out); break;
+                        case kQWide | kQRev: quad_run_mixed<W, (kQWide | kQRev)>(v, cls, rn.y, n, g, mp, ce, out); break;
+                        default: quad_run_mixed<W, -1>(v, cls, rn.y, n, g, mp, ce, out); break;
+                    }
                 } else {
                     const QuadCtx qc{pt, Pp, lnP, ctot, ce, sTab, g};
                     quad_run<W>(m, v, qc, cls, rn.y, n, out);
@@ -334,7 +413,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
                     const QOwn o = N;
                     op += kQG * W;
                     if (s + W < v.nsq) N = load_qown(op);
-                    double acc = list_sum(v.lists, o, g, sQ + p);
+                    double acc = MIXED ? sequence_sum(v.lists, o, g, sQ + p) : list_sum(v.lists, o, g, sQ + p);
                     const int k = o.own;
                     if (k >= 0) {
                         if (c > 0) acc += sW[k * kQP + p];
@@ -363,13 +442,17 @@ static QuadKernel quad_kernel(int warps, int mixed) {
 // runs the global-scratch kernel.
 constexpr int kQuadMaxSpecies = 434;
 
-cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, int mixed, QuadPlan** out) {
+int quad_tile_points() { return kQP; }
+
+// latency: 24 warps to a tile whatever its size, for batches of few tiles.
+cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, int mixed, int latency,
+                         QuadPlan** out) {
     *out = nullptr;
     const int ns = m.ns, nr = m.nr;
     if (nr == 0 || ns > kQuadMaxSpecies) return cudaErrorNotSupported;
     HostQuads h;
     build_quads(v, h);
-    if (mixed && !h.mixed_ok) return cudaErrorNotSupported;
+    if (mixed && (!h.mixed_ok || 4 * h.nquad >= 0x1fff)) return cudaErrorNotSupported;
     cudaDeviceProp prop;
     cudaError_t e = cudaGetDeviceProperties(&prop, device);
     if (e != cudaSuccess) return e;
@@ -392,7 +475,8 @@ cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     // warps per CTA and CTAs per SM: 24 resident warps of 80 registers, in as
     // many CTAs as shared memory allows
     const int fit = (int)(per_sm / (bytes(pl.rows, pl.nchunk, 24) + 1024));
-    pl.warps = fit >= 3 ? 8 : fit == 2 ? 12 : 24;
+    if (latency && fit < 2) return cudaErrorNotSupported;   // the plan for throughput is the same
+    pl.warps = latency || fit < 2 ? 24 : fit == 2 ? 12 : 8;
     pl.smem = bytes(pl.rows, pl.nchunk, pl.warps);
     const int resident = std::max(1, std::min((int)(per_sm / (pl.smem + 1024)), 24 / pl.warps));
     pl.grid = prop.multiProcessorCount * resident;
@@ -442,6 +526,44 @@ cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
             lb.add_quad(own, q, pl.rows);
         }
     if (!lb.fits) return cudaErrorNotSupported;
+    if (mixed) {
+        // every coefficient of every side, in file order; one chunk
+        if (pl.nchunk > 1) return cudaErrorNotSupported;
+        const int32_t* orig = (const int32_t*)v.a[CG_ORIG];
+        std::vector<int> file(nr);
+        for (int r = 0; r < nr; ++r) file[r] = r;
+        std::sort(file.begin(), file.end(), [&](int a, int b) { return orig[a] < orig[b]; });
+        std::vector<std::vector<unsigned>> seq(ns);
+        for (int r : file)
+            for (int side = 0; side < 2; ++side)
+                for (int j = side ? pp[r] : rp[r]; j < (side ? pp[r + 1] : rp[r + 1]); ++j) {
+                    const double nu = side ? pnu[j] : rnu[j];
+                    const unsigned mult = nu == 1.0 ? 0u : nu == 2.0 ? 0x4000u : 0x6000u;   // integers up to 3: a fast form
+                    seq[side ? psp[j] : rsp[j]].push_back((unsigned)h.at[r] | mult | (side ? 0u : 0x8000u));
+                }
+        std::vector<int> sp(ns);
+        for (int k = 0; k < ns; ++k) sp[k] = k;
+        std::stable_sort(sp.begin(), sp.end(), [&](int a, int b) { return seq[a].size() > seq[b].size(); });
+        lb = ListBuilder();
+        pl.nsq = (ns + kQG - 1) / kQG;
+        for (int s = 0; s < pl.nsq; ++s) {
+            const unsigned n8 = std::max<unsigned>((unsigned)(seq[sp[kQG * s]].size() + 7) / 8, 1);
+            QOwn own[kQG];
+            const int ptr = (int)lb.ent.size();
+            for (unsigned k = 0; k < n8; ++k)
+                for (int g = 0; g < kQG; ++g) {
+                    const int i = kQG * s + g;
+                    unsigned e[8];
+                    for (unsigned u = 0; u < 8; ++u)
+                        e[u] = i < ns && 8 * k + u < seq[sp[i]].size() ? seq[sp[i]][8 * k + u] : (unsigned)pl.rows;
+                    const uint4 w =
+                        make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
+                    if (k == 0) own[g] = QOwn{i < ns ? sp[i] : -1, n8, ptr, 0u, w};
+                    else lb.ent.push_back(w);
+                }
+            lb.own.insert(lb.own.end(), own, own + kQG);
+        }
+    }
     Image im;
     const size_t o_rec = im.put(mixed ? h.rec2 : h.rec), o_run = im.put(run), o_efl = im.put(h.efl), o_eff = im.put(h.eff);
     const size_t o_fall = im.put(mixed ? h.fall2 : h.fall), o_rb = im.put(rbeg), o_th = im.put(quad_thermo_rows(v));

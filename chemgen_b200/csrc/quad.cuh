@@ -95,7 +95,7 @@ struct __align__(16) QRec {
     unsigned short s[2], p[2];         // the first two molecules of each side
     unsigned short s2, p2;             // the third ones
     unsigned int r;                    // reaction in kernel order
-    unsigned int aux;                  // falloff row
+    unsigned int aux;                  // falloff row; mixed: 2^f of a constant rate as FP32 bits, else 0
     unsigned int ord;                  // molecules a side, << 0 / << 8 (M included)
 };
 static_assert(sizeof(QRec) == 48, "QRec must stay 48 bytes");
@@ -392,6 +392,12 @@ inline void build_quads(const cg_mech_view& v, HostQuads& h, bool products = fal
         if (ok) {
             it.b.lnA = std::log2(std::fabs(arh[3 * r]));
             it.b.th = it.a.th * kLog2e;
+            if (kind <= CG_THIRD_BODY && it.b.b == 0.0 && it.b.th == 0.0) {
+                // a constant rate: in generated code the compiler evaluates its
+                // 2^f, to the nearest float and not as the hardware does
+                const float f = (float)(it.b.lnA - std::nearbyint(it.b.lnA)), e = (float)std::exp2((double)f);
+                std::memcpy(&it.b.aux, &e, sizeof(e));
+            }
             const bool wide = n[0] > 2 || ((rev || products) && n[1] > 2);
             it.key = kind | (wide ? kQWide : 0) | (rev ? kQRev : 0);
         } else {

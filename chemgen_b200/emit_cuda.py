@@ -538,8 +538,9 @@ class _Emitter:
         ns, B = self.ns, self.block
         L = []
         L.append("const int t = threadIdx.x;")
+        # n points of arrays whose species stride is ng
         L.append(f"const int64_t i = (int64_t)blockIdx.x * {B} + t;")
-        L.append("const bool act = i < ng;")
+        L.append("const bool act = i < n;")
         L.append(f"const double Tv = act ? {self.ld('T', 'i')} : 1000.0;")
         L.append(f"const double Pv = act ? {self.ld('P', 'i')} : {_d(1013250.0)};")
         L.append("const double lnT = cgm::cg_log(Tv), invT = rcp(Tv);")
@@ -624,7 +625,8 @@ class _Emitter:
         ns, B = self.ns, self.block
         name = "cg_gen_mixed" if mixed else "cg_gen_fp64"
         L = [f"__global__ void __launch_bounds__({B}, 1) {name}(const double* __restrict__ P, "
-             "const double* __restrict__ T, const double* __restrict__ Y, double* __restrict__ wdot, int64_t ng) {"]
+             "const double* __restrict__ T, const double* __restrict__ Y, double* __restrict__ wdot, int64_t ng, "
+             "int64_t n) {"]
         # dynamic shared memory: [array][species][thread]
         L.append("  extern __shared__ __align__(16) unsigned char dsm[];")
         if not mixed and self.tmem:
@@ -786,7 +788,7 @@ def emit(mech: Mechanism, name: Optional[str] = None, block: Optional[int] = Non
         "using cgg::rcp;",
         "namespace {",
     ]
-    attrs, dispatch = [], []
+    attrs, dispatch, blocks = [], [], {}
     for want, em, mixed, kname, mname in ((want64, em64, False, "cg_gen_fp64", "CHEMGEN_MODE_FP64"),
                                           (want32, em32, True, "cg_gen_mixed", "CHEMGEN_MODE_MIXED")):
         if not want:
@@ -795,13 +797,16 @@ def emit(mech: Mechanism, name: Optional[str] = None, block: Optional[int] = Non
         src += [em.kernel(mixed), ""]
         attrs.append(f"cudaFuncSetAttribute({kname}, cudaFuncAttributeMaxDynamicSharedMemorySize, "
                      f"{em.smem_bytes(mixed)}) != cudaSuccess")
-        dispatch.append(f"  if (mode == {mname}) {{ {kname}<<<(unsigned)((ng + {B - 1}) / {B}), {B}, "
+        dispatch.append(f"  if (mode == {mname}) {{ {kname}<<<(unsigned)((i1 - i0 + {B - 1}) / {B}), {B}, "
                         f"{em.smem_bytes(mixed)}, st>>>"
-                        "(P, T, Y, wdot, ng); return cudaGetLastError() == cudaSuccess ? CHEMGEN_OK : CHEMGEN_ERR_CUDA; }")
+                        "(P + i0, T + i0, Y + i0, wdot + i0, ng, i1 - i0); return cudaGetLastError() == cudaSuccess ? CHEMGEN_OK : "
+                        "CHEMGEN_ERR_CUDA; }")
+        blocks[mname] = B
     modes = (1 if want64 else 0) | (2 if want32 else 0)
     src += [
-        "int launch(int mode, const double* P, const double* T, int64_t ng, const double* Y, double* wdot, void* s) {",
-        "  if (ng <= 0) return CHEMGEN_OK;",
+        "int launch_range(int mode, const double* P, const double* T, int64_t ng, const double* Y, double* wdot,",
+        "                 int64_t i0, int64_t i1, void* s) {",
+        "  if (i1 <= i0) return CHEMGEN_OK;",
         "  static bool attrs = false;",
         "  if (!attrs) {",
         "    if (" + " ||\n        ".join(attrs) + ")",
@@ -813,8 +818,16 @@ def emit(mech: Mechanism, name: Optional[str] = None, block: Optional[int] = Non
         "  return CHEMGEN_ERR_INVALID_ARGUMENT;",
         "}",
         "",
+        "int launch(int mode, const double* P, const double* T, int64_t ng, const double* Y, double* wdot, void* s) {",
+        "  return launch_range(mode, P, T, ng, Y, wdot, 0, ng, s);",
+        "}",
+        "",
         "struct Register {",
-        f"  Register() {{ chemgen_register_kernels(0x{fp:016x}ull, {mech.ns}, {mech.nr}, {modes}u, &launch); }}",
+        "  Register() {",
+        f"    chemgen_register_kernels(0x{fp:016x}ull, {mech.ns}, {mech.nr}, {modes}u, &launch);",
+    ] + [f"    chemgen_register_kernel_range(0x{fp:016x}ull, {mech.ns}, {mech.nr}, {m}, {b}, &launch_range);"
+         for m, b in blocks.items()] + [
+        "  }",
         "} register_once;",
         "}  // namespace",
         "",

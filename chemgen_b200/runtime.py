@@ -112,7 +112,8 @@ def lib() -> ctypes.CDLL:
     L.chemgen_use_generated.argtypes = [vp, ci]
     L.chemgen_kernel_kind.argtypes = [vp, ci]
     L.chemgen_register_kernels.argtypes = [ctypes.c_uint64, ci, ci, ctypes.c_uint, vp]
-    for f in ("chemgen_create", "chemgen_destroy", "chemgen_num_species", "chemgen_num_reactions",
+    L.chemgen_register_kernel_range.argtypes = [ctypes.c_uint64, ci, ci, ci, ci, vp]
+    for f in ("chemgen_register_kernel_range", "chemgen_create", "chemgen_destroy", "chemgen_num_species", "chemgen_num_reactions",
               "chemgen_getrates", "chemgen_getrates_ex", "chemgen_getrates_counted", "chemgen_workspace_bytes",
               "chemgen_getrates_ws",
               "chemgen_getrates_host", "chemgen_init_constants", "chemgen_free_constants",

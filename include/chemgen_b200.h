@@ -107,6 +107,14 @@ int chemgen_getrates_host(chemgen_handle* h, int mode, const double* P, const do
 typedef int (*chemgen_kernel_fn)(int mode, const double* P, const double* T, int64_t ng, const double* Y,
                                  double* wdot, void* stream);
 int chemgen_register_kernels(uint64_t fingerprint, int ns, int nr, unsigned modes, chemgen_kernel_fn fn);
+/* A generated module's kernel of one mode over the points [i0, i1) of arrays
+ * laid out for ng points, `block` points per SM and wave.  With it, a batch
+ * that leaves most of its last wave empty runs that remainder (or all of a
+ * small batch) on the table-driven tile kernel of the same arithmetic. */
+typedef int (*chemgen_kernel_range_fn)(int mode, const double* P, const double* T, int64_t ng, const double* Y,
+                                       double* wdot, int64_t i0, int64_t i1, void* stream);
+int chemgen_register_kernel_range(uint64_t fingerprint, int ns, int nr, int mode, int block,
+                                  chemgen_kernel_range_fn fn);
 int chemgen_use_generated(chemgen_handle* h, int enable);
 int chemgen_kernel_kind(chemgen_handle* h, int mode);
 

@@ -84,3 +84,30 @@ def test_derivatives_of_every_kind(name, ng):
     gT, gY, gP = v
     assert _rel(gY, r[1]) <= 1e-9
     assert _rel(gT[None], r[0][None]) <= 1e-7 and _rel(gP[None], r[2][None]) <= 1e-7
+
+
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+@pytest.mark.parametrize("name", ["gri30", "h2_burke", "synthetic_53_325", "all_kinds"])
+def test_small_batches_and_remainders_equal_the_generated_kernel(name, mode):
+    # a batch of one wave runs the generated kernel, its first points alone the
+    # tile kernel, and a wave plus a few points both: the same arithmetic, with
+    # FP64 mode's sums in another order (1e-12 covers 300 terms of rounding; a mixed
+    # rate off by one FP32 ulp would show as 6e-8)
+    from conftest import load_golden
+    mech = synthetic.all_kinds() if name == "all_kinds" else load_golden(name)[0]
+    gm = GpuMechanism(mech, generated=True)
+    assert gm.kernel_kind(mode) == "generated"
+    wave = 148 * 512
+    P, T, Y = _cuda(*synthetic.states(mech.ns, wave + 77, seed=4))
+
+    def run(a, b):
+        return gm.getrates(P[a:b].contiguous(), T[a:b].contiguous(), Y[:, a:b].contiguous(), mode=mode)
+    ref = run(0, wave)
+    for n in (1, 8 * 148, 8 * 148 + 1, 3001):
+        assert _rel(run(0, n), ref[:, :n]) <= 1e-12, n
+    both = run(0, wave + 77)
+    assert _rel(both[:, :wave], ref) <= 1e-12
+    assert _rel(both[:, wave:], run(wave, wave + 77)) <= 1e-12
+    if mode == "mixed":
+        # the mixed tile kernel repeats the generated one to the last bit
+        assert all(bool((run(0, n) == ref[:, :n]).all()) for n in (1, 1184, 1185, 3001))
