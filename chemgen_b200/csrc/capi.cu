@@ -36,7 +36,8 @@ void mixed_release(MixedPlan* p);
 cudaError_t launch_getrates_mixed(const MixedPlan* p, const DevMech& m, const double* P, const double* T,
                                   const double* Y, double* wdot, int64_t ng, void* scratch, size_t scratch_bytes,
                                   cudaStream_t s);
-size_t mixed_workspace_bytes(const MixedPlan* p, int64_t ng);
+size_t mixed_workspace_bytes(const MixedPlan* p, int64_t ng);   // what a caller is asked for
+size_t mixed_scratch_bytes(const MixedPlan* p, int64_t ng);     // what the kernel needs
 size_t deriv_workspace_bytes(int ns, int64_t ng);
 struct GradPlan;
 cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, int adjoint, GradPlan** out);
@@ -389,10 +390,12 @@ size_t fp64_ws_bytes(const chemgen_handle* h, int64_t ng) {
     return (size_t)slices * cg::fp64_global_slice_bytes(h->ns);
 }
 
-size_t ws_bytes_for(const chemgen_handle* h, int mode, int64_t ng) {
+// Scratch of a launch; with `asked`, what chemgen_workspace_bytes asks for.
+size_t ws_bytes_for(const chemgen_handle* h, int mode, int64_t ng, bool asked = false) {
     if (h->use_generated && h->gen_fn && (mode == 0 || mode == 1) && (h->gen_modes & (1u << mode))) return 0;
     if (mode == CHEMGEN_MODE_FP64) return fp64_ws_bytes(h, ng);
-    if (mode == CHEMGEN_MODE_MIXED && h->mixed) return cg::mixed_workspace_bytes(h->mixed, ng);
+    if (mode == CHEMGEN_MODE_MIXED && h->mixed)
+        return asked ? cg::mixed_workspace_bytes(h->mixed, ng) : cg::mixed_scratch_bytes(h->mixed, ng);
     return 0;
 }
 
@@ -465,7 +468,7 @@ int launch(chemgen_handle* h, int mode, const double* P, const double* T, int64_
     }
     if (mode == CHEMGEN_MODE_MIXED) {
         if (!h->mixed) return h->mixed_err == cudaSuccess ? CHEMGEN_ERR_UNSUPPORTED : status_of(h->mixed_err);
-        size_t need = cg::mixed_workspace_bytes(h->mixed, ng);
+        size_t need = cg::mixed_scratch_bytes(h->mixed, ng);
         if (need && (!ws || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 255u)))
             return CHEMGEN_ERR_INVALID_ARGUMENT;
         return status_of(cg::launch_getrates_mixed(h->mixed, h->m, P, T, Y, w, ng, ws, ws_bytes, s));
@@ -710,7 +713,7 @@ int chemgen_workspace_bytes(const chemgen_handle* h, int mode, int64_t ng, size_
     if (!h || !bytes || ng < 0) return CHEMGEN_ERR_INVALID_ARGUMENT;
     if (mode == CHEMGEN_MODE_MIXED && !h->mixed) return CHEMGEN_ERR_UNSUPPORTED;
     if (mode != CHEMGEN_MODE_FP64 && mode != CHEMGEN_MODE_MIXED) return CHEMGEN_ERR_INVALID_ARGUMENT;
-    *bytes = ws_bytes_for(h, mode, ng);
+    *bytes = ws_bytes_for(h, mode, ng, true);
     return CHEMGEN_OK;
 }
 
@@ -719,6 +722,12 @@ int chemgen_getrates_ws(chemgen_handle* h, int mode, const double* P, const doub
     int st = check_args(h, P, T, ng, Y, wdot);
     if (st || ng == 0) return st;
     DeviceGuard g(h->device);
+    refresh_generated(h);
+    if (mode == CHEMGEN_MODE_MIXED) {
+        const size_t need = ws_bytes_for(h, mode, ng, true);
+        if (need && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255u)))
+            return CHEMGEN_ERR_INVALID_ARGUMENT;
+    }
     return launch(h, mode, P, T, ng, Y, wdot, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 

@@ -36,6 +36,7 @@
 
 #include "cg_math.cuh"
 #include "gen_common.cuh"
+#include "quad.cuh"
 #include "rates_common.cuh"
 #include "umma.cuh"
 
@@ -53,12 +54,17 @@ struct __align__(16) TcFast {
     double l2A, b, th2;          // log2|A|, b, (Ea/Rc) log2 e
     unsigned short sr[3], sp[3]; // reactant / product molecules (species ns = none)
     unsigned char ordf, ordb;    // concentration factors of each side (M included)
-    unsigned char flags;         // kFastOn | kFastRev | kFastThird | kFastNeg
-    unsigned char pad0;
-    int pad1[2];
+    unsigned char flags;         // kFastOn | kFastRev | kFastThird | kFastNeg | kFastFall
+    unsigned char neff;          // efficiencies (255: look them up)
+    int eff0;                    // first efficiency
+    union {
+        int aux;                 // falloff row
+        int ngen;                // species entries of a general row
+    };
 };
 static_assert(sizeof(TcFast) == 48, "TcFast must stay 48 bytes");
 constexpr unsigned kFastOn = 1, kFastRev = 2, kFastThird = 4, kFastNeg = 8;
+constexpr unsigned kFastFall = 16;   // falloff with positive A's, decoded for the 32-point kernel only
 
 struct MixedPlan {
     int ns = 0, nr = 0, npad = 0, nhalf = 0, nchunk = 0;
@@ -70,6 +76,10 @@ struct MixedPlan {
     int nt = 1;             // threads per point (blockDim = 128 nt)
     int hot = 0;            // species with FP64 accumulators in spare tensor-memory columns
     int hot_every = 8;      // chunks between the hot species' FP64 flushes
+    int t32 = 0;            // the 32-point kernel's tile fits
+    const TcFast* fast32 = nullptr;   // its records: species as byte offsets
+    size_t smem32 = 0;
+    int grid32 = 0;
     const int* perm = nullptr;  // accumulator column -> species (-1: padding)
     void* dbuf = nullptr;
     const __nv_bfloat16* nu = nullptr;
@@ -101,8 +111,8 @@ __device__ __forceinline__ float rate32(double a, float prod, int eoff) {
 }
 
 struct TileCtx {
-    const float* C;      // C * 2^32, stride kTile
-    const double* G;     // log2 Gibbs terms, stride kTile
+    const float* C;      // C * 2^32, one row of points a species
+    const double* G;     // log2 Gibbs terms, likewise
     double T, Pv, lnT, lnT2, invT;
     float ctot32, Tf, invTf, lnT2f;
 };
@@ -169,6 +179,7 @@ __device__ double plog_kf64(const DevMech& m, int row, double P, double lnT, dou
 // FP64 evaluation of reaction r (PLOG, non-integer stoichiometry, falloff
 // with negative pre-exponential factors): kept out of line so that the
 // common FP32 path keeps few registers.
+template <int TS>
 __device__ __noinline__ float rate_of_progress_fp64(const DevMech& m, const DRxn& R, int kind, float Ms,
                                                     const TileCtx& c, int tid) {
     const bool compact = (R.flags & kFCompact) != 0;
@@ -186,14 +197,14 @@ __device__ __noinline__ float rate_of_progress_fp64(const DevMech& m, const DRxn
             if (compact) {
                 for (int j = 0; j < R.nre; ++j) {
                     const int s = slot_species(R.sp[j]);
-                    qf *= ipow3((double)c.C[s * kTile + tid] * cs, slot_nu(R.sp[j]));
-                    g = fma((double)slot_nu(R.sp[j]), c.G[s * kTile + tid], g);
+                    qf *= ipow3((double)c.C[s * TS + tid] * cs, slot_nu(R.sp[j]));
+                    g = fma((double)slot_nu(R.sp[j]), c.G[s * TS + tid], g);
                 }
                 double pb = 1.0;
                 for (int j = 0; j < R.npr; ++j) {
                     const int s = slot_species(R.sp[3 + j]);
-                    pb *= ipow3((double)c.C[s * kTile + tid] * cs, slot_nu(R.sp[3 + j]));
-                    g = fma(-(double)slot_nu(R.sp[3 + j]), c.G[s * kTile + tid], g);
+                    pb *= ipow3((double)c.C[s * TS + tid] * cs, slot_nu(R.sp[3 + j]));
+                    g = fma(-(double)slot_nu(R.sp[3 + j]), c.G[s * TS + tid], g);
                 }
                 if (R.flags & CG_F_REVERSIBLE) qb = kf * exp2(g) * pb;
             } else {
@@ -203,15 +214,15 @@ __device__ __noinline__ float rate_of_progress_fp64(const DevMech& m, const DRxn
                 for (int j = r0; j < r1; ++j) {
                     const int s = __ldg(m.gen_sp + j);
                     const double nu = __ldg(m.gen_nu + j);
-                    qf *= pow((double)c.C[s * kTile + tid] * cs, nu);
-                    g = fma(nu, c.G[s * kTile + tid], g);
+                    qf *= pow((double)c.C[s * TS + tid] * cs, nu);
+                    g = fma(nu, c.G[s * TS + tid], g);
                 }
                 double pb = 1.0;
                 for (int j = p0; j < p1; ++j) {
                     const int s = __ldg(m.gen_sp + j);
                     const double nu = __ldg(m.gen_nu + j);
-                    pb *= pow((double)c.C[s * kTile + tid] * cs, nu);
-                    g = fma(-nu, c.G[s * kTile + tid], g);
+                    pb *= pow((double)c.C[s * TS + tid] * cs, nu);
+                    g = fma(-nu, c.G[s * TS + tid], g);
                 }
                 if (R.flags & CG_F_REVERSIBLE) qb = kf * exp2(g) * pb;
             }
@@ -225,10 +236,10 @@ __device__ __noinline__ float rate_of_progress_fp64(const DevMech& m, const DRxn
 // Ms = ctot + sum_e (eff_e - 1) C[sp_e] of reaction r (third_body.j2:18-31) in
 // FP32 at point `tid`, the efficiencies taken four at a time so that their
 // loads are in flight together; the sum keeps the table's order.
-__device__ __forceinline__ float tc_third_body(const DevMech& m, int r, const TileCtx& c, int tid) {
-    float Ms = c.ctot32;
-    const int e1 = __ldg(m.eff_ptr + r + 1);
-    for (int e = __ldg(m.eff_ptr + r); e < e1; e += 4) {
+template <int TS>
+__device__ __forceinline__ float tc_third_body(const DevMech& m, int e0, int e1, const float* C, float ctot32, int tid) {
+    float Ms = ctot32;
+    for (int e = e0; e < e1; e += 4) {
         int sp[4];
         float ev[4];
 #pragma unroll
@@ -239,23 +250,29 @@ __device__ __forceinline__ float tc_third_body(const DevMech& m, int r, const Ti
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const float cv = c.C[sp[u] * kTile + tid];
+            const float cv = C[sp[u] * TS + tid];
             if (e + u < e1) Ms = fmaf(ev[u], cv, Ms);
         }
     }
     return Ms;
 }
 
+template <int TS>
+__device__ __forceinline__ float tc_third_body(const DevMech& m, int r, const TileCtx& c, int tid) {
+    return tc_third_body<TS>(m, __ldg(m.eff_ptr + r), __ldg(m.eff_ptr + r + 1), c.C, c.ctot32, tid);
+}
+
 // Net rate of progress of reaction r at point `tid` of the tile, FP32.
+template <int TS>
 __device__ float rate_of_progress(const DevMech& m, int r, const TileCtx& c, int tid) {
     const DRxn R = load_rxn(m.rxn + r);
     int kind = CG_STANDARD;
     while (kind < CG_PLOG && r >= m.seg[kind + 1]) ++kind;
     float Ms = 0.0f;
-    if (kind >= CG_THIRD_BODY && kind <= CG_SRI) Ms = tc_third_body(m, r, c, tid);
+    if (kind >= CG_THIRD_BODY && kind <= CG_SRI) Ms = tc_third_body<TS>(m, r, c, tid);
     const bool compact = (R.flags & kFCompact) != 0;
     const bool neg_falloff = kind >= CG_LINDEMANN && kind <= CG_SRI && (R.flags & (CG_F_A_NEG | CG_F_LOW_NEG));
-    if (!compact || kind == CG_PLOG || neg_falloff) return rate_of_progress_fp64(m, R, kind, Ms, c, tid);
+    if (!compact || kind == CG_PLOG || neg_falloff) return rate_of_progress_fp64<TS>(m, R, kind, Ms, c, tid);
     double a;
     float sgn = 1.0f;
     if (kind <= CG_THIRD_BODY) {
@@ -270,10 +287,10 @@ __device__ float rate_of_progress(const DevMech& m, int r, const TileCtx& c, int
     double g = 0.0;
     for (int j = 0; j < R.nre; ++j) {
         const int s = slot_species(R.sp[j]), nu = slot_nu(R.sp[j]);
-        const float x = c.C[s * kTile + tid];
+        const float x = c.C[s * TS + tid];
         cf *= (nu == 1) ? x : (nu == 2 ? x * x : x * x * x);
         of += nu;
-        g = fma((double)nu, c.G[s * kTile + tid], g);
+        g = fma((double)nu, c.G[s * TS + tid], g);
     }
     if (kind == CG_THIRD_BODY) {
         cf *= Ms;
@@ -285,10 +302,10 @@ __device__ float rate_of_progress(const DevMech& m, int r, const TileCtx& c, int
         int ob = 0;
         for (int j = 0; j < R.npr; ++j) {
             const int s = slot_species(R.sp[3 + j]), nu = slot_nu(R.sp[3 + j]);
-            const float x = c.C[s * kTile + tid];
+            const float x = c.C[s * TS + tid];
             cb *= (nu == 1) ? x : (nu == 2 ? x * x : x * x * x);
             ob += nu;
-            g = fma(-(double)nu, c.G[s * kTile + tid], g);
+            g = fma(-(double)nu, c.G[s * TS + tid], g);
         }
         if (kind == CG_THIRD_BODY) {
             cb *= Ms;
@@ -300,16 +317,17 @@ __device__ float rate_of_progress(const DevMech& m, int r, const TileCtx& c, int
 }
 
 // Net rate of progress of a pre-decoded reaction (TcFast) at point `tid`, FP32.
+template <int TS>
 __device__ __forceinline__ float rate_fast(const DevMech& m, int r, const TcFast& F, const TileCtx& c, int tid) {
     const double a = fma(F.b, c.lnT2, F.l2A) - F.th2 * c.invT;
     float Ms = 1.0f;
-    if (F.flags & kFastThird) Ms = tc_third_body(m, r, c, tid);
-    const float cf = c.C[F.sr[0] * kTile + tid] * c.C[F.sr[1] * kTile + tid] * c.C[F.sr[2] * kTile + tid] * Ms;
+    if (F.flags & kFastThird) Ms = tc_third_body<TS>(m, r, c, tid);
+    const float cf = c.C[F.sr[0] * TS + tid] * c.C[F.sr[1] * TS + tid] * c.C[F.sr[2] * TS + tid] * Ms;
     float q = rate32(a, cf, -32 * (int)F.ordf);
     if (F.flags & kFastRev) {
-        const double g = (c.G[F.sr[0] * kTile + tid] + c.G[F.sr[1] * kTile + tid] + c.G[F.sr[2] * kTile + tid]) -
-                         (c.G[F.sp[0] * kTile + tid] + c.G[F.sp[1] * kTile + tid] + c.G[F.sp[2] * kTile + tid]);
-        const float cb = c.C[F.sp[0] * kTile + tid] * c.C[F.sp[1] * kTile + tid] * c.C[F.sp[2] * kTile + tid] * Ms;
+        const double g = (c.G[F.sr[0] * TS + tid] + c.G[F.sr[1] * TS + tid] + c.G[F.sr[2] * TS + tid]) -
+                         (c.G[F.sp[0] * TS + tid] + c.G[F.sp[1] * TS + tid] + c.G[F.sp[2] * TS + tid]);
+        const float cb = c.C[F.sp[0] * TS + tid] * c.C[F.sp[1] * TS + tid] * c.C[F.sp[2] * TS + tid] * Ms;
         q -= rate32(a + g, cb, -32 * (int)F.ordb);
     }
     return (F.flags & kFastNeg) ? -q : q;
@@ -326,7 +344,8 @@ __device__ __forceinline__ TcFast load_fast(const TcFast* p) {
 }
 
 // One TcFast per reaction (flags 0 where the generic path is needed).
-__global__ void build_fast_kernel(DevMech m, TcFast* out) {
+// Species are stored times `scale` (the 32-point kernel's byte offsets).
+__global__ void build_fast_kernel(DevMech m, TcFast* out, int scale) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= m.nr) return;
     const DRxn R = load_rxn(m.rxn + r);
@@ -336,28 +355,34 @@ __global__ void build_fast_kernel(DevMech m, TcFast* out) {
     f.l2A = R.lnA * kLog2eD;
     f.b = R.b;
     f.th2 = R.theta * kLog2eD;
-    f.pad0 = 0;
-    f.pad1[0] = f.pad1[1] = 0;
+    f.eff0 = __ldg(m.eff_ptr + r);
+    f.neff = (unsigned char)min(__ldg(m.eff_ptr + r + 1) - f.eff0, 255);
+    f.aux = R.aux;
+    if (!(R.flags & kFCompact) && R.gen >= 0)
+        f.ngen = __ldg(m.gen_rptr + R.gen + 1) - __ldg(m.gen_rptr + R.gen) + __ldg(m.gen_pptr + R.gen + 1) -
+                 __ldg(m.gen_pptr + R.gen);
     f.flags = 0;
     f.ordf = f.ordb = 0;
-    for (int j = 0; j < 3; ++j) f.sr[j] = f.sp[j] = (unsigned short)m.ns;
-    bool ok = (kind == CG_STANDARD || kind == CG_THIRD_BODY) && (R.flags & kFCompact) && R.sgn != 0.0;
+    for (int j = 0; j < 3; ++j) f.sr[j] = f.sp[j] = (unsigned short)(m.ns * scale);
+    const bool fall = scale > 1 && kind >= CG_LINDEMANN && kind <= CG_SRI && !(R.flags & (CG_F_A_NEG | CG_F_LOW_NEG)) &&
+                      R.sgn > 0.0;
+    bool ok = (kind == CG_STANDARD || kind == CG_THIRD_BODY || fall) && (R.flags & kFCompact) && R.sgn != 0.0;
     int nf = 0, nb = 0;
     for (int j = 0; ok && j < R.nre; ++j)
         for (int k = 0; k < slot_nu(R.sp[j]); ++k) {
             if (nf == 3) ok = false;
-            else f.sr[nf++] = (unsigned short)slot_species(R.sp[j]);
+            else f.sr[nf++] = (unsigned short)(slot_species(R.sp[j]) * scale);
         }
     for (int j = 0; ok && j < R.npr; ++j)
         for (int k = 0; k < slot_nu(R.sp[3 + j]); ++k) {
             if (nb == 3) ok = false;
-            else f.sp[nb++] = (unsigned short)slot_species(R.sp[3 + j]);
+            else f.sp[nb++] = (unsigned short)(slot_species(R.sp[3 + j]) * scale);
         }
     if (ok) {
         const bool third = kind == CG_THIRD_BODY;
         f.ordf = (unsigned char)(nf + (third ? 1 : 0));
         f.ordb = (unsigned char)(nb + (third ? 1 : 0));
-        f.flags = (unsigned char)(kFastOn | ((R.flags & CG_F_REVERSIBLE) ? kFastRev : 0) | (third ? kFastThird : 0) |
+        f.flags = (unsigned char)((fall ? kFastFall : kFastOn) | ((R.flags & CG_F_REVERSIBLE) ? kFastRev : 0) | (third ? kFastThird : 0) |
                                   (R.sgn < 0.0 ? kFastNeg : 0));
     }
     out[r] = f;
@@ -487,7 +512,7 @@ __global__ void __launch_bounds__(kTile * NT, 1)
                     const TcFast F = load_fast(fast + r);
                     // this thread's next record moves into L1 meanwhile (no registers held)
                     if (u + 1 < kPer && r + 1 < m.nr) asm volatile("prefetch.global.L1 [%0];" ::"l"(fast + r + 1));
-                    q = (F.flags & kFastOn) ? rate_fast(m, r, F, c, pt) : rate_of_progress(m, r, c, pt);
+                    q = (F.flags & kFastOn) ? rate_fast<kTile>(m, r, F, c, pt) : rate_of_progress<kTile>(m, r, c, pt);
                 }
                 if (!act) q = 0.0f;
                 const __nv_bfloat16 h = __float2bfloat16_rn(q);
@@ -611,6 +636,433 @@ __global__ void __launch_bounds__(kTile * NT, 1)
     if (warp == 0) um::tmem_dealloc(tbase, tcols);
 }
 
+// ------------------------------------------------------------ 32-point tile
+//
+// One point per lane and one reaction per warp: every lane of a warp runs the
+// same reaction (no divergence, records read once per warp), and the tile's
+// C (FP32) and G (FP64) fit in shared memory up to ~410 species, where the
+// 128-point tile had to read G from L2 for every molecule.  The 16 warps take
+// the 32 reactions of two chunks, two each; lane p's rates are row p of the A
+// operands.  The MMAs stay M = 128 (the tensor memory's lanes): rows 32..127
+// read whatever follows in shared memory, and nobody reads their sums.  A batch
+// of 20011 points is 5 rounds of 626 tiles instead of two waves of 157.  The
+// order of every sum -- reactions in K, chunks, splits, hot flushes -- is the
+// 128-point kernel's, and so is every bit of the result.
+// Bound by latency (34 % of issue slots; FP64 chains, shared loads, records
+// from L1) with 17 warps of 96 registers.  Measured on B200: JetSurf 2.0, 20011
+// points 2.30 -> 1.53 ms, 256 points 1.11 -> 0.30 ms; 348/2163, 20011 points
+// 1.71 -> 1.22 ms, 65536 points 3.43 ms both.
+constexpr int kTP = 32, kTWarps = 16;
+constexpr int kA32 = 1024;             // bytes of a split's 32 rows
+
+// A tile's per-point values that only the slow path reads, in shared memory.
+struct Tile32 {
+    double T[kTP], P[kTP], lnT[kTP], invT[kTP];
+    float ctot[kTP];
+    double tab[16];
+};
+
+// M of a pre-decoded reaction.
+__device__ __forceinline__ float third_body32(const DevMech& m, int r, const TcFast& F, float ctot32, const float* sC) {
+    const int lane = threadIdx.x & 31;
+    const int e1 = F.neff < 255 ? F.eff0 + F.neff : __ldg(m.eff_ptr + r + 1);
+    return tc_third_body<kTP>(m, F.eff0, e1, sC, ctot32, lane);
+}
+
+__device__ __forceinline__ float c_at(const char* C, unsigned off) {
+    return *reinterpret_cast<const float*>(C + off);
+}
+__device__ __forceinline__ double g_at(const char* G, unsigned off) {
+    return *reinterpret_cast<const double*>(G + 2 * off);
+}
+
+// q = 2^a cf - 2^(a + g) cb of a pre-decoded reaction (offsets of 128-byte rows
+// of C, twice that of G).  pow2: a species' square is formed first, as
+// rate_of_progress does.
+__device__ __forceinline__ float net32(const TcFast& F, double a, float Ms, const char* C, const char* G, bool pow2) {
+    const float x0 = c_at(C, F.sr[0]), x1 = c_at(C, F.sr[1]), x2 = c_at(C, F.sr[2]);
+    float cf = x0 * x1 * x2;
+    if (pow2 && F.sr[1] == F.sr[2]) cf = x0 * (x1 * x2);
+    float q = rate32(a, cf * Ms, -32 * (int)F.ordf);
+    if (F.flags & kFastRev) {
+        const double g = (g_at(G, F.sr[0]) + g_at(G, F.sr[1]) + g_at(G, F.sr[2])) -
+                         (g_at(G, F.sp[0]) + g_at(G, F.sp[1]) + g_at(G, F.sp[2]));
+        const float y0 = c_at(C, F.sp[0]), y1 = c_at(C, F.sp[1]), y2 = c_at(C, F.sp[2]);
+        float cb = y0 * y1 * y2;
+        if (pow2 && F.sp[1] == F.sp[2]) cb = y0 * (y1 * y2);
+        q -= rate32(a + g, cb * Ms, -32 * (int)F.ordb);
+    }
+    return (F.flags & kFastNeg) ? -q : q;
+}
+
+// An elementary or three-body reaction.
+__device__ __forceinline__ float rate_common32(const DevMech& m, int r, const TcFast& F, double lnT2, double invT,
+                                               float ctot32, const float* sC, const double* sG) {
+    const int lane = threadIdx.x & 31;
+    const float Ms = (F.flags & kFastThird) ? third_body32(m, r, F, ctot32, sC) : 1.0f;
+    return net32(F, fma(F.b, lnT2, F.l2A) - F.th2 * invT, Ms, reinterpret_cast<const char*>(sC + lane),
+                 reinterpret_cast<const char*>(sG + lane), false);
+}
+
+// A reaction with general stoichiometry that is no falloff and no PLOG, FP64
+// (rate_of_progress_fp64 with one reaction per warp): each lane fetches one
+// entry of the reaction's row, so the row is one load deep instead of two per
+// entry.
+__device__ __noinline__ float rate_general32(const DevMech& m, int r, int kind, float Ms, TileCtx c) {
+    const int lane = threadIdx.x & 31;
+    const DRxn R = load_rxn(m.rxn + r);
+    const int r0 = __ldg(m.gen_rptr + R.gen), r1 = __ldg(m.gen_rptr + R.gen + 1);
+    const int p0 = __ldg(m.gen_pptr + R.gen), p1 = __ldg(m.gen_pptr + R.gen + 1);
+    const int nr = r1 - r0, n = nr + p1 - p0, at = lane < nr ? r0 + lane : p0 + (lane - nr);
+    const int sp = lane < n ? __ldg(m.gen_sp + at) : 0;
+    const double nu = lane < n ? __ldg(m.gen_nu + at) : 0.0;
+    const double kf = R.sgn * cgm::cg_exp_clamped(fma(R.b, c.lnT, R.lnA) - R.theta * c.invT);
+    const double cs = 2.3283064365386963e-10;   // 2^-32
+    double qf = kf, pb = 1.0, g = 0.0;
+    for (int j = 0; j < n; ++j) {
+        const int k = __shfl_sync(0xffffffffu, sp, j);
+        const double v = __shfl_sync(0xffffffffu, nu, j);
+        const double x = (double)c.C[k * kTP + lane] * cs, y = v == 1.0 ? x : pow(x, v);
+        if (j < nr) qf *= y;
+        else pb *= y;
+        g = fma(j < nr ? v : -v, c.G[k * kTP + lane], g);
+    }
+    const double qb = (R.flags & CG_F_REVERSIBLE) ? kf * exp2(g) * pb : 0.0;
+    double rr = qf - qb;
+    if (kind == CG_THIRD_BODY) rr *= (double)Ms * cs;
+    return (float)rr;
+}
+
+// Falloff and reactions without a pre-decoded form.  Out of line, and with
+// its context in shared memory, so that the common path keeps its values in
+// registers (inline, they went through local memory: 374 instructions a
+// reaction).  The falloff blend is falloff_l2 with the quad kernels' exp.
+__device__ __noinline__ float rate_other32(const DevMech& m, const TcFast* fast, int r, const Tile32* t,
+                                           const float* sC, const double* sG) {
+    const int lane = threadIdx.x & 31;
+    TileCtx c;
+    c.C = sC;
+    c.G = sG;
+    c.T = t->T[lane];
+    c.Pv = t->P[lane];
+    c.lnT = t->lnT[lane];
+    c.invT = t->invT[lane];
+    c.ctot32 = t->ctot[lane];
+    const TcFast F = load_fast(fast + r);
+    const double* tab = t->tab;
+    const DRxn R = load_rxn(m.rxn + r);
+    if (!(F.flags & kFastFall)) {
+        if ((R.flags & kFCompact) || r >= m.seg[CG_LINDEMANN] || F.ngen > 32) return rate_of_progress<kTP>(m, r, c, lane);
+        return rate_general32(m, r, r >= m.seg[CG_THIRD_BODY] ? CG_THIRD_BODY : CG_STANDARD,
+                              r >= m.seg[CG_THIRD_BODY] ? third_body32(m, r, F, c.ctot32, sC) : 0.0f, c);
+    }
+    const DFall f = load_fall(m.fall + F.aux);
+    const double x2 = __ldg(&m.fall2[F.aux].T2);
+    int kind = CG_LINDEMANN;
+    while (kind < CG_SRI && r >= m.seg[kind + 1]) ++kind;
+    const float Ms = third_body32(m, r, F, c.ctot32, sC);
+    constexpr double kLog10_2 = 0.30102999566398119521, kLn2 = 0.69314718055994530942;
+    const double ainf = (fma(R.b, c.lnT, R.lnA) - R.theta * c.invT) * kLog2eD;
+    const double a0 = (fma(f.b0, c.lnT, f.lnA0) - f.theta0 * c.invT) * kLog2eD;
+    const double M = (double)Ms * 2.3283064365386963e-10;   // Ms = M * 2^32
+    const double l2pr = (a0 - ainf) + cgm::cg_log(M) * kLog2eD;
+    const double x = q_exp(fmax(-fabs(l2pr) * kLn2, kQMinArg), tab);   // min(Pr, 1/Pr)
+    const double l2r = fmin(l2pr, 0.0) - cgm::cg_log(1.0 + x) * kLog2eD;
+    double l2F = 0.0;
+    if (kind == CG_TROE) {
+        double Fc = fma(f.p[0], q_exp(fmax(-c.T * f.p[1], kQMinArg), tab),
+                        f.p[2] * q_exp(fmax(-c.T * f.p[3], kQMinArg), tab));
+        if (R.flags & CG_F_TROE_T2) Fc += q_exp(fmax(-x2 * c.invT, kQMinArg), tab);
+        const double lFc = cgm::cg_log10(Fc);
+        const double lp = fma(kLog10_2, l2pr, fma(-0.67, lFc, -0.4));
+        const double f1 = lp * q_rcp(fma(-0.14, lp, fma(-1.27, lFc, 0.75)));
+        l2F = lFc * q_rcp(fma(f1, f1, 1.0)) / kLog10_2;
+    } else if (kind == CG_SRI) {
+        const double lp = kLog10_2 * l2pr;
+        const double X = q_rcp(fma(lp, lp, 1.0));
+        const double base = fma(f.p[0], q_exp(fmax(-f.p[1] * c.invT, kQMinArg), tab),
+                                q_exp(fmax(-c.T * f.p[2], kQMinArg), tab));
+        l2F = (cgm::cg_log(f.p[3]) + fma(X, cgm::cg_log(base), x2 * c.lnT)) * kLog2eD;
+    }
+    return net32(F, ainf + (l2r + l2F), 1.0f, reinterpret_cast<const char*>(sC + lane),
+                 reinterpret_cast<const char*>(sG + lane), true);
+}
+
+// The two reactions r, r + 1 of a warp when one of them has no common form, or
+// does not exist.
+__device__ __noinline__ float2 rate_pair32(const DevMech& m, const TcFast* fast, int r, const Tile32* t,
+                                           const float* sC, const double* sG) {
+    const int lane = threadIdx.x & 31;
+    float q[2] = {0.0f, 0.0f};
+    for (int j = 0; j < 2; ++j) {
+        if (r + j >= m.nr) break;
+        const TcFast F = load_fast(fast + r + j);
+        if (!(F.flags & kFastOn)) {
+            q[j] = rate_other32(m, fast, r + j, t, sC, sG);
+            continue;
+        }
+        q[j] = rate_common32(m, r + j, F, t->lnT[lane] * kLog2eD, t->invT[lane], t->ctot[lane], sC, sG);
+    }
+    return make_float2(q[0], q[1]);
+}
+
+// The sums of a group leave tensor memory (lanes 0..31) for wdot, or, for a hot
+// flush, the most-touched species' FP32 sums move into their FP64 accumulators.
+// w: this point's wdot, or NULL.  Out of line: 48 registers of columns beside
+// the main loop's values would spill to local memory, whose 512 x 370 bytes do
+// not stay in the L1 that the tile leaves (83 spills a pair of chunks cost 10k
+// cycles).
+__device__ __noinline__ void flush32(bool hot_end, bool first_group, int nhot, uint32_t tbase, int warp, int npad,
+                 int hot, const int* __restrict__ perm, double* w, int64_t ng) {
+    if (hot_end) {
+        for (int blk = warp >> 2; blk < hot / 16; blk += kTWarps / 4) {
+            float v[16];
+            uint32_t d[32];
+            um::tmem_ld16(um::tmem_lane_addr(tbase, 0, 16 * blk), v);
+            if (nhot > 0) um::tmem_ld32(um::tmem_lane_addr(tbase, 0, npad + 32 * blk), d);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const double a = (nhot > 0 ? __hiloint2double((int)d[2 * j + 1], (int)d[2 * j]) : 0.0) +
+                                 (double)v[j];
+                d[2 * j] = (uint32_t)__double2loint(a);
+                d[2 * j + 1] = (uint32_t)__double2hiint(a);
+            }
+            um::tmem_st32(um::tmem_lane_addr(tbase, 0, npad + 32 * blk), d);
+            uint32_t z[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) z[j] = 0u;
+            um::tmem_st16(um::tmem_lane_addr(tbase, 0, 16 * blk), z);
+        }
+        um::tmem_wait_st();
+        return;
+    }
+    for (int col = 16 * (warp >> 2); col < npad; col += 4 * kTWarps) {
+        float v[16];
+        uint32_t d[32];
+        um::tmem_ld16(um::tmem_lane_addr(tbase, 0, col), v);
+        const bool h64 = col < hot && nhot > 0;
+        if (h64) um::tmem_ld32(um::tmem_lane_addr(tbase, 0, npad + 2 * col), d);
+        if (!w) continue;
+        int sp[16];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) reinterpret_cast<int4*>(sp)[j] = __ldg(reinterpret_cast<const int4*>(perm + col) + j);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            if (sp[j] < 0) continue;
+            double x = (double)v[j];
+            if (h64) x += __hiloint2double((int)d[2 * j + 1], (int)d[2 * j]);
+            double* o = w + (int64_t)sp[j] * ng;
+            if (first_group) __stcs(o, x);
+            else *o += x;
+        }
+    }
+}
+
+// 16 warps compute, a 17th loads the stoichiometry and issues the MMAs.  The
+// compute warps meet only at a tile's prologue: a pair's operands are handed
+// over by mbarriers (full: one arrival a warp; done: the MMAs' commit), so a
+// warp runs up to two pairs ahead of the slowest.  With a block barrier each
+// pair, and the MMAs issued by a compute warp, a pair took 3.5 us instead of
+// 2.9 (348 species, elementary reactions).
+__global__ void __launch_bounds__(32 * (kTWarps + 1), 1)
+    getrates_tc32_kernel(const __grid_constant__ DevMech m, const __nv_bfloat16* __restrict__ nu,
+                         const TcFast* __restrict__ fast, int npad, int nhalf, int nchunk, uint32_t tcols,
+                         const double* __restrict__ P, const double* __restrict__ Tg, const double* __restrict__ Y,
+                         double* __restrict__ wdot, int64_t ng, int* err, int group, const int* __restrict__ perm,
+                         int hot, int hot_every) {
+    extern __shared__ __align__(1024) unsigned char sm[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int ns = m.ns, rows = ns + 1;
+    unsigned char* sA = sm;                                     // [2 buffers][2 chunks][3 splits][32 x 16] BF16
+    unsigned char* sB = sA + 12 * kA32;                         // [2 buffers][2 chunks][npad x 16] BF16
+    // (the A operands' rows 32..127 run into sB, at most 3 KB of it and of sG)
+    double* sG = reinterpret_cast<double*>(sB + 4 * npad * 32);    // [rows][32]
+    float* sC = reinterpret_cast<float*>(sG + rows * kTP);      // [rows][32]
+    double* sRed = reinterpret_cast<double*>(sC + rows * kTP);  // [16][32]
+    Tile32* sT = reinterpret_cast<Tile32*>(sRed + kTWarps * kTP);
+    uint64_t* full = reinterpret_cast<uint64_t*>(sT + 1);       // [2] A written
+    uint64_t* done = full + 2;                                  // [2] MMAs done
+    uint64_t* bfull = full + 4;                                 // [2] B loaded
+    uint64_t* flushed = full + 6;                               // sums taken out of tensor memory
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(full + 7);
+    if (tid == 0) {
+        for (int j = 0; j < 2; ++j) {
+            um::mbar_init(&full[j], kTWarps);
+            um::mbar_init(&done[j], 1);
+            um::mbar_init(&bfull[j], 1);
+        }
+        um::mbar_init(flushed, kTWarps / 4);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (tid < 16) sT->tab[tid] = kQExpTab[tid];
+    if (warp == 0) um::tmem_alloc(tslot, tcols);
+    um::fence_before_sync();
+    __syncthreads();
+    um::fence_after_sync();
+    const uint32_t tbase = *tslot;
+    const int npair = (nchunk + 1) / 2;
+    const int64_t ntiles = (ng + kTP - 1) / kTP;
+    // A wait that runs out clears ok; the warp goes on without waiting (and the
+    // issuing warp without loads and MMAs), so that every warp reaches the end.
+    bool ok = true;
+    uint32_t n = 0, nflush = 0;        // pairs and flushes so far, of all tiles
+    auto wait = [&](uint64_t* bar, uint32_t use) { ok = ok && um::mbar_wait(bar, use & 1u); };
+    // group and hot_every are even, so a flush falls on the end of a pair
+    auto flush_after = [&](int ch, bool& hot_end) {
+        const bool group_end = (ch % group) == group - 1 || ch == nchunk - 1;
+        hot_end = hot > 0 && !group_end && (ch % hot_every) == hot_every - 1;
+        return group_end || hot_end;
+    };
+    if (warp == kTWarps) {
+        if (lane == 0) {
+            const uint32_t idesc = um::idesc_bf16(kTile, nhalf);
+            const int nh = npad / nhalf;
+            auto load = [&](int pr, uint32_t k) {               // pair pr of a tile, pair k of all
+                const uint32_t bytes = (uint32_t)(min(2, nchunk - 2 * pr) * npad * 32);
+                um::mbar_expect_tx(&bfull[k & 1], bytes);
+                um::bulk_g2s(sB + (k & 1) * 2 * npad * 32, nu + (int64_t)2 * pr * npad * kChunk, bytes, &bfull[k & 1]);
+            };
+            const bool any = (int64_t)blockIdx.x < ntiles && npair > 0;
+            bool inflight = any;
+            if (any) load(0, 0);
+            for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
+                for (int pr = 0; pr < npair; ++pr, ++n) {
+                    const uint32_t buf = n & 1;
+                    const int ch0 = 2 * pr, nc = min(2, nchunk - ch0);
+                    // the other buffers are free when the last pair's MMAs are done
+                    if (n > 0) wait(&done[buf ^ 1], (n - 1) >> 1);
+                    const bool more = pr + 1 < npair || tile + gridDim.x < ntiles;
+                    if (inflight) ok = um::mbar_wait(&bfull[buf], (n >> 1) & 1u) && ok;   // even after a time-out
+                    inflight = ok && more;
+                    if (inflight) load(pr + 1 < npair ? pr + 1 : 0, n + 1);
+                    wait(&full[buf], n >> 1);
+                    um::fence_after_sync();
+                    for (int cc = 0; cc < nc && ok; ++cc) {
+                        const bool start = ((ch0 + cc) % group) == 0;
+                        const uint32_t ab = um::smem_addr(sA + (buf * 2 + cc) * 3 * kA32);
+                        const uint32_t bs = um::smem_addr(sB + (buf * 2 + cc) * npad * 32);
+                        for (int s = 0; s < 3; ++s) {
+                            const uint64_t ad = um::desc_kmajor(ab + (uint32_t)(s * kA32), kChunk, 0);
+                            for (int h = 0; h < nh; ++h)
+                                um::mma_bf16(tbase + (uint32_t)(h * nhalf), ad,
+                                             um::desc_kmajor(bs + (uint32_t)(h * nhalf * 32), kChunk, 0), idesc,
+                                             (!start || s > 0) ? 1u : 0u);
+                        }
+                    }
+                    um::commit(&done[buf]);
+                    bool hot_end;
+                    if (flush_after(ch0 + nc - 1, hot_end)) {
+                        wait(flushed, nflush);
+                        ++nflush;
+                        um::fence_after_sync();
+                    }
+                }
+        }
+    } else {
+        const int rsub = (warp >> 3) * kChunk + 2 * (warp & 7);     // this warp's two reactions of a pair
+        for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+            const int64_t i = tile * kTP + lane;
+            const bool act = i < ng;
+            const double T = act ? __ldcs(Tg + i) : 1000.0, Pv = act ? __ldcs(P + i) : kPatm;
+            const double lnT = cgm::cg_log(T), invT = fmin(1.0 / T, kQMaxInvT), lnT2 = lnT * kLog2eD;
+            um::bar_sync(1, 32 * kTWarps);                      // the last tile's rates are done
+            double part = 0.0;
+#pragma unroll 8
+            for (int k = warp; k < ns; k += kTWarps) {
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(m.thermo + 16 * k));
+                const double yk = (act ? __ldcs(Y + (int64_t)k * ng + i) : 1.0) * __ldg(m.inv_mw + k);
+                sG[k * kTP + lane] = yk;
+                part += yk;
+            }
+            sRed[warp * kTP + lane] = part;
+            um::bar_sync(1, 32 * kTWarps);
+            double csum = 0.0;
+#pragma unroll
+            for (int q = 0; q < kTWarps; ++q) csum += sRed[q * kTP + lane];
+            const double facs = Pv / (kR0 * csum * T) * 4294967296.0;
+            const float ctot32 = (float)(csum * facs);
+            if (warp == 0) {
+                sT->T[lane] = T;
+                sT->P[lane] = Pv;
+                sT->lnT[lane] = lnT;
+                sT->invT[lane] = invT;
+                sT->ctot[lane] = ctot32;
+                sC[ns * kTP + lane] = 1.0f;
+                sG[ns * kTP + lane] = 0.0;
+            }
+            const double lpfac2 = -6.35856916300311 - lnT2;     // log2(Patm/R0) - log2 T
+#pragma unroll 4
+            for (int k = warp; k < ns; k += kTWarps) {
+                sC[k * kTP + lane] = (float)(sG[k * kTP + lane] * facs);
+                const double* th = m.thermo + 16 * k;
+                th += T < __ldg(th) ? 1 : 8;
+                double cf[7];
+#pragma unroll
+                for (int j = 0; j < 7; ++j) cf[j] = __ldg(th + j);
+                sG[k * kTP + lane] = fma(smh_poly(cf, T, lnT, invT), kLog2eD, lpfac2);
+            }
+            um::bar_sync(1, 32 * kTWarps);
+            bool first_group = true;
+            int nhot = 0;
+            for (int pr = 0; pr < npair; ++pr, ++n) {
+                const uint32_t buf = n & 1;
+                const int ch0 = 2 * pr, nc = min(2, nchunk - ch0), r0 = ch0 * kChunk + rsub;
+                // (records come from L1, where the last pair's turn has put them: held in
+                // registers across the calls below they would go through local memory)
+                const TcFast F0 = load_fast(fast + min(r0, m.nr - 1)), F1 = load_fast(fast + min(r0 + 1, m.nr - 1));
+                float q0, q1;
+                if ((F0.flags & F1.flags & kFastOn) && r0 + 1 < m.nr) {
+                    q0 = rate_common32(m, r0, F0, lnT2, invT, ctot32, sC, sG);
+                    q1 = rate_common32(m, r0 + 1, F1, lnT2, invT, ctot32, sC, sG);
+                } else {
+                    const float2 q = rate_pair32(m, fast, r0, sT, sC, sG);
+                    q0 = q.x;
+                    q1 = q.y;
+                }
+                if (lane < 2 && r0 + 2 * kChunk + lane < m.nr)
+                    asm volatile("prefetch.global.L1 [%0];" ::"l"(fast + r0 + 2 * kChunk + lane));
+                if (!act) q0 = q1 = 0.0f;
+                // q = hi + mid + lo in BF16
+                uint32_t w[3];
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    const __nv_bfloat16 b0 = __float2bfloat16_rn(q0), b1 = __float2bfloat16_rn(q1);
+                    w[j] = (uint32_t)__bfloat16_as_ushort(b0) | (uint32_t)__bfloat16_as_ushort(b1) << 16;
+                    q0 -= __bfloat162float(b0);
+                    q1 -= __bfloat162float(b1);
+                }
+                if (n > 1) wait(&done[buf], (n - 2) >> 1);      // the buffer's last MMAs
+                unsigned char* a0 = sA + (buf * 2 + (warp >> 3)) * 3 * kA32 +
+                                    um::kmajor_offset(lane, 2 * (warp & 7), kChunk);
+#pragma unroll
+                for (int j = 0; j < 3; ++j) *reinterpret_cast<uint32_t*>(a0 + j * kA32) = w[j];
+                um::fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) um::mbar_arrive(&full[buf]);
+                bool hot_end;
+                if (!flush_after(ch0 + nc - 1, hot_end)) continue;
+                // the tile's sums are in lanes 0..31: the warps of that quadrant take
+                // them out while the others go on
+                if ((warp & 3) == 0) {
+                    wait(&done[buf], n >> 1);
+                    ok = __all_sync(0xffffffffu, ok);
+                    um::fence_after_sync();
+                    if (ok) flush32(hot_end, first_group, nhot, tbase, warp, npad, hot, perm, act ? wdot + i : nullptr, ng);
+                    um::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) um::mbar_arrive(flushed);
+                }
+                if (hot_end) ++nhot;
+                else first_group = false;
+            }
+        }
+    }
+    if (!ok && lane == 0) atomicExch(err, 1);
+    um::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) um::tmem_dealloc(tbase, tcols);
+}
+
 const void* kernel_for(int g_smem, int nt) {
     if (g_smem) return nt == 4 ? (const void*)getrates_tc_kernel<true, 4>
                                : nt == 2 ? (const void*)getrates_tc_kernel<true, 2> : (const void*)getrates_tc_kernel<true, 1>;
@@ -681,6 +1133,13 @@ cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, M
         }
     }
     p->grid = prop.multiProcessorCount * per_sm;
+    // the 32-point kernel whenever its tile's state fits
+    const size_t t32 = 12 * (size_t)kA32 + 4 * (size_t)npad * 32 + rows * kTP * 12 + kTWarps * kTP * 8 + sizeof(Tile32) + 64;
+    if (t32 <= limit) {
+        p->t32 = 1;
+        p->smem32 = t32;
+        p->grid32 = prop.multiProcessorCount;
+    }
     // nu chunks in the canonical K-major layout: B[n][k] = nu of species n in reaction 16*chunk + k
     std::vector<float> nuf((size_t)ns * nr, 0.0f);
     const int32_t* rp = (const int32_t*)v.a[CG_RPTR];
@@ -726,12 +1185,12 @@ cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, M
     const size_t img_bytes = (img.size() * sizeof(__nv_bfloat16) + 255) / 256 * 256;
     const size_t fast_bytes = ((size_t)nr * sizeof(TcFast) + 255) / 256 * 256;
     const size_t perm_bytes = ((size_t)npad * sizeof(int) + 255) / 256 * 256;
-    const size_t bytes = img_bytes + fast_bytes + perm_bytes + 256;
+    const size_t bytes = img_bytes + 2 * fast_bytes + perm_bytes + 256;
     e = cudaMalloc(&p->dbuf, bytes);
     if (e == cudaSuccess) e = cudaMemcpy(p->dbuf, img.data(), img.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset((char*)p->dbuf + bytes - 256, 0, 256);
     if (e == cudaSuccess)
-        e = cudaMemcpy((char*)p->dbuf + img_bytes + fast_bytes, perm.data(), perm.size() * sizeof(int),
+        e = cudaMemcpy((char*)p->dbuf + img_bytes + 2 * fast_bytes, perm.data(), perm.size() * sizeof(int),
                        cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel_for(p->g_smem, p->nt),
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
@@ -742,9 +1201,11 @@ cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, M
     }
     p->nu = (const __nv_bfloat16*)p->dbuf;
     p->fast = (const TcFast*)((char*)p->dbuf + img_bytes);
-    p->perm = (const int*)((char*)p->dbuf + img_bytes + fast_bytes);
+    p->fast32 = (const TcFast*)((char*)p->dbuf + img_bytes + fast_bytes);
+    p->perm = (const int*)((char*)p->dbuf + img_bytes + 2 * fast_bytes);
     if (nr > 0) {
-        build_fast_kernel<<<(nr + 127) / 128, 128>>>(m, (TcFast*)p->fast);
+        build_fast_kernel<<<(nr + 127) / 128, 128>>>(m, (TcFast*)p->fast, 1);
+        if (p->t32) build_fast_kernel<<<(nr + 127) / 128, 128>>>(m, (TcFast*)p->fast32, kTP * 4);
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
         if (e != cudaSuccess) {
@@ -764,6 +1225,12 @@ void mixed_release(MixedPlan* p) {
     delete p;
 }
 
+// Scratch the kernel that runs needs (none with 32-point tiles), and the
+// scratch a caller is asked for: the latter stays what the 128-point kernel
+// needs, so that programs that size and pass it see no change.
+size_t mixed_workspace_bytes(const MixedPlan* p, int64_t ng);
+size_t mixed_scratch_bytes(const MixedPlan* p, int64_t ng) { return p && p->t32 ? 0 : mixed_workspace_bytes(p, ng); }
+
 size_t mixed_workspace_bytes(const MixedPlan* p, int64_t ng) {
     if (!p || p->g_smem) return 0;
     int64_t tiles = (ng + kTile - 1) / kTile;
@@ -775,6 +1242,26 @@ cudaError_t launch_getrates_mixed(const MixedPlan* p, const DevMech& m, const do
                                   const double* Y, double* wdot, int64_t ng, void* scratch, size_t scratch_bytes,
                                   cudaStream_t s) {
     if (ng <= 0) return cudaSuccess;
+    // the kernel's shared-memory limit is this plan's, set under one lock with
+    // the launch (a plan made later for a smaller mechanism sets it lower)
+    static std::mutex mu;
+    // Mechanisms whose Gibbs terms fit beside the 128-point tile run the faster
+    // of the two: on B200 at 53/325 a round of 32-point tiles takes 47 us and a
+    // wave of 128-point tiles 121 us.  Larger ones always run 32-point tiles
+    // (348/2163: a round 0.22 ms, a wave 0.82 ms).
+    const int64_t rounds = (ng + (int64_t)kTP * p->grid32 - 1) / std::max<int64_t>(1, (int64_t)kTP * p->grid32);
+    const int64_t waves = (ng + (int64_t)kTile * p->grid - 1) / ((int64_t)kTile * p->grid);
+    if (p->t32 && (!p->g_smem || (double)rounds * 0.39 <= (double)waves)) {
+        const unsigned g32 = (unsigned)std::min<int64_t>((ng + kTP - 1) / kTP, p->grid32);
+        std::lock_guard<std::mutex> lk(mu);
+        const cudaError_t e = cudaFuncSetAttribute(getrates_tc32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)p->smem32);
+        if (e != cudaSuccess) return e;
+        getrates_tc32_kernel<<<g32, 32 * (kTWarps + 1), p->smem32, s>>>(m, p->nu, p->fast32, p->npad, p->nhalf, p->nchunk,
+                                                                  p->tcols, P, T, Y, wdot, ng, p->err, p->group,
+                                                                  p->perm, p->hot, p->hot_every);
+        return cudaGetLastError();
+    }
     int64_t tiles = (ng + kTile - 1) / kTile;
     int64_t grid = std::min<int64_t>(tiles, p->grid);
     if (!p->g_smem) {
@@ -783,9 +1270,6 @@ cudaError_t launch_getrates_mixed(const MixedPlan* p, const DevMech& m, const do
         if (grid < 1 || !scratch) return cudaErrorInvalidValue;
     }
     double* gs = p->g_smem ? nullptr : (double*)scratch;
-    // the kernel's shared-memory limit is this plan's, set under one lock with
-    // the launch (a plan made later for a smaller mechanism sets it lower)
-    static std::mutex mu;
     std::lock_guard<std::mutex> lk(mu);
     const cudaError_t e = cudaFuncSetAttribute(kernel_for(p->g_smem, p->nt),
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);

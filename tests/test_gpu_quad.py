@@ -111,3 +111,17 @@ def test_small_batches_and_remainders_equal_the_generated_kernel(name, mode):
     if mode == "mixed":
         # the mixed tile kernel repeats the generated one to the last bit
         assert all(bool((run(0, n) == ref[:, :n]).all()) for n in (1, 1184, 1185, 3001))
+
+
+@pytest.mark.parametrize("ng", [1, 31, 33, 32 * 148 + 7])
+def test_mixed_32_point_tiles(ng):
+    # part tiles and more tiles than SMs on the 32-point tensor-core kernel; 1e-6
+    # is the mixed kernels' bar
+    from conftest import load_golden
+    mech = load_golden("jetsurf2")[0]
+    blob = pack.pack(mech).to_blob()
+    P, T, Y = synthetic.states(mech.ns, ng, seed=ng)
+    w = GpuMechanism(blob).getrates(*_cuda(P, T, Y), mode="mixed").cpu().numpy()
+    idx = np.unique(np.concatenate([np.arange(min(ng, 40)), np.arange(max(0, ng - 40), ng)]))
+    r = oracle.rates(blob, P[idx], T[idx], np.ascontiguousarray(Y[:, idx]), mech.nr)
+    assert oracle.errors(w[:, idx], r["wdot"], r["S"])["norm_max"] <= 1e-6
