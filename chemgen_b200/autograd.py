@@ -8,7 +8,7 @@ from __future__ import annotations
 
 import torch
 
-from .runtime import GpuMechanism
+from .runtime import GpuMechanism, transposed
 
 
 class Getrates(torch.autograd.Function):
@@ -19,20 +19,20 @@ class Getrates(torch.autograd.Function):
         if layout not in ("species_major", "point_major"):
             raise ValueError("layout must be 'species_major' or 'point_major'")
         P, T = P.contiguous(), T.contiguous()
-        Ys = Y.t().contiguous() if layout == "point_major" else Y.contiguous()
+        Ys = transposed(Y) if layout == "point_major" else Y.contiguous()
         ctx.gm = gm
         ctx.layout = layout
         ctx.save_for_backward(P, T, Ys)
         w = gm.getrates(P, T, Ys, mode=mode)
-        return w.t().contiguous() if layout == "point_major" else w
+        return transposed(w) if layout == "point_major" else w
 
     @staticmethod
     def backward(ctx, g):
         P, T, Ys = ctx.saved_tensors
-        gs = g.t().contiguous() if ctx.layout == "point_major" else g.contiguous()
+        gs = transposed(g) if ctx.layout == "point_major" else g.contiguous()
         gT, gY, gP = ctx.gm.vjp(P, T, Ys, gs)
         if ctx.layout == "point_major":
-            gY = gY.t().contiguous()
+            gY = transposed(gY)
         return None, gP, gT, gY, None, None
 
 

@@ -96,6 +96,10 @@ int chemgen_getrates_ws(chemgen_handle* h, int mode, const double* P, const doub
 int chemgen_getrates_host(chemgen_handle* h, int mode, const double* P, const double* T, int64_t ng,
                           const double* Y, double* wdot);
 
+/* dst[c*rows + r] = src[r*cols + c]: point-major states [ng, ns] to
+ * species-major [ns, ng] and back (device pointers, asynchronous). */
+int chemgen_transpose(const double* src, int64_t rows, int64_t cols, double* dst, void* stream);
+
 /* Kernels generated for one mechanism (generate_chemistry.py --language cuda
  * emits them; the reference's counterpart is its per-mechanism generated
  * getrates, chemgen/chemistry.py:326-341).  A generated module calls

@@ -125,3 +125,15 @@ def test_mixed_32_point_tiles(ng):
     idx = np.unique(np.concatenate([np.arange(min(ng, 40)), np.arange(max(0, ng - 40), ng)]))
     r = oracle.rates(blob, P[idx], T[idx], np.ascontiguousarray(Y[:, idx]), mech.nr)
     assert oracle.errors(w[:, idx], r["wdot"], r["S"])["norm_max"] <= 1e-6
+
+
+@pytest.mark.parametrize("rows,cols", [(1 << 19, 1), (1, 1 << 19), (9893, 53), (53, 9893), (8129, 65), (348, 1507)])
+def test_transposed_copies(rows, cols):
+    # tiles of 64 x 64: whole, part and single-row ones; the values are moved, not computed
+    import torch
+    from chemgen_b200.runtime import transposed
+    x = torch.arange(rows * cols, dtype=torch.float64, device="cuda").reshape(rows, cols)
+    assert torch.equal(transposed(x), x.t())
+    out = torch.empty(cols, rows, dtype=torch.float64, device="cuda")
+    assert transposed(x, out) is out and torch.equal(out, x.t())
+    assert torch.equal(transposed(x[:, ::2]), x[:, ::2].t())
