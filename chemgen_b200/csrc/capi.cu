@@ -746,7 +746,14 @@ int chemgen_getrates_host(chemgen_handle* h, int mode, const double* P, const do
     // reused (its in-order queue waiting for chunk c's copy back) only three
     // chunks later: both copy directions stay busy.
     constexpr int NS = chemgen_handle::kIoStreams;
-    const int64_t chunk = std::min<int64_t>(ng, std::max<int64_t>(1 << 16, (ng + 15) / 16));
+    // An eighth of the points a chunk, so that both copy directions overlap
+    // from ~10^4 points on (53 species: 30000 points 0.57 -> 0.49 ms, 80000
+    // points 1.28 -> 1.20 ms against one or two chunks of 65536), not under
+    // 8192 (64 KB a species' row: more chunks cost more row copies than they
+    // hide; 16 chunks at 200000 points 2.41 -> 2.8 ms) and not over 65536 or a
+    // sixteenth (2^20 points and up).
+    const int64_t most = std::max<int64_t>(1 << 16, (ng + 15) / 16);
+    const int64_t chunk = std::min<int64_t>(ng, std::max<int64_t>(8192, std::min((ng + 7) / 8, most)));
     const size_t per = (size_t)(2 + 2 * ns) * chunk;       // P, T, Y, wdot doubles of one chunk
     std::lock_guard<std::mutex> lk(h->mu);
     cudaError_t e = cudaSuccess;
