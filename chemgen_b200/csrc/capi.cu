@@ -423,14 +423,14 @@ int launch_tiles(chemgen_handle* h, int mode, const double* P, const double* T, 
 // a small batch) run on the tile kernel when that is faster.  Both times,
 // fitted to B200 measurements at 9/23 and 53/325 (us):
 //   wave: FP64 12 and 103, mixed 10 and 68, linear in the reactions;
-//   eight-point tiles, one per SM at a time: FP64 1.6 and 4.7, mixed 1.5 and
-//   5.0, linear in the quads of four reactions (8 and 91).
-// (53/325 FP64: the line lies at 26000 of a wave's 75776 points; there the
-// tile kernel takes 99 us.)
+//   eight-point tiles, one per SM at a time: FP64 1.6 and 4.4, mixed 1.5 and
+//   4.8, linear in the quads of four reactions (8 and 91).
+// (53/325 FP64: the line lies at 27500 of a wave's 75776 points; 25000 take the
+// tile kernel 92 us.)
 bool tiles_faster(const chemgen_handle* h, int mode, int64_t n) {
     const double nr = h->nr, nq = 0.28 * nr, tiles = (double)n / cg::quad_tile_points() / h->sm_count;
     const double wave = mode ? 5.6 + 0.192 * nr : 5.1 + 0.301 * nr;
-    const double tile = mode ? 1.2 + 0.0418 * nq : 1.3 + 0.0373 * nq;
+    const double tile = mode ? 1.2 + 0.0400 * nq : 1.3 + 0.0341 * nq;
     return tiles * tile < wave;
 }
 
