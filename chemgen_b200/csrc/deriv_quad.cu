@@ -169,13 +169,14 @@ __device__ __forceinline__ void quad_falloff_d(int kind, const QRec& R, const QF
     dlkf = fma(gpr, dlPr, dlkinf) + dlF_T;
 }
 
-// The rows of one reaction.  kf is the forward rate constant times the
-// reaction's three-body factor M; scale: dq/dM = scale (qf - qb) (0: the
-// reaction has no M), add: its share of s = add (qf - qb) beside the
-// molecules' (ord counts M of a three-body reaction).
+// The rows of one reaction with q = mul (qf - qb): mul is M for a three-body
+// reaction, otherwise 1.  scale: dq/dM = scale (qf - qb) (M itself is no
+// divisor here: it is zero where a species without efficiency stands alone),
+// add: the reaction's share of s = add (qf - qb) beside the molecules' (ord
+// counts M of a three-body reaction).
 template <bool ADJ, bool WIDE, bool REV>
 __device__ __forceinline__ void grad_rows(const GradCtx& c, const QRec& R, double kf, double dlkf, bool usesM,
-                                          double scale, double add, double* out, AdjSums& sum) {
+                                          double mul, double scale, double add, double* out, AdjSums& sum) {
     constexpr int N = WIDE ? 3 : 2;
     unsigned so[3] = {R.s[0], R.s[1], R.s2}, po[3] = {R.p[0], R.p[1], R.p2};
     double x[N], d[N];
@@ -217,10 +218,16 @@ __device__ __forceinline__ void grad_rows(const GradCtx& c, const QRec& R, doubl
         for (int j = 0; j < N; ++j) gq += quad_row(c.dg, po[j]).y;
     }
     const double net = qf - qb;
-    const double dT = net * dlkf - (REV ? qb * dlKc : 0.0);
-    const double s = fma((double)(R.ord & 0xffu), qf, fma(add, net, -(double)((R.ord >> 8) & 0xffu) * qb));
+    double dT = net * dlkf - (REV ? qb * dlKc : 0.0);
+    double s = fma((double)(R.ord & 0xffu), qf, fma(add, net, -(double)((R.ord >> 8) & 0xffu) * qb));
     const double m = scale * net;
-    const double f = ADJ ? gq * kf : kf, b = ADJ ? -gq * kb : -kb;
+    double f = ADJ ? gq * kf : kf, b = ADJ ? -gq * kb : -kb;
+    if (usesM) {
+        dT *= mul;
+        s *= mul;
+        f *= mul;
+        b *= mul;
+    }
     int o = 0;
 #pragma unroll
     for (int j = 0; j < N; ++j) out[32 * o++] = f * d[j];
@@ -306,7 +313,7 @@ __device__ __forceinline__ void grad_standard(const GradCtx& c, const QRec* rec,
             row = __ldg(qrow);
         }
         const double kf = q_exp(fma(R.b, c.pt.lnT, R.lnA) - R.th * c.pt.invT, c.tab);
-        grad_rows<ADJ, WIDE, REV>(c, R, kf, fma(R.th, c.pt.invT, R.b) * c.pt.invT, false, 0.0, 0.0, out, sum);
+        grad_rows<ADJ, WIDE, REV>(c, R, kf, fma(R.th, c.pt.invT, R.b) * c.pt.invT, false, 1.0, 0.0, 0.0, out, sum);
     }
 }
 
@@ -338,20 +345,20 @@ __device__ __forceinline__ void grad_run(const DevMech& m, const GradView& v, co
         }
         const QRec R = load_qrec(rec);
         const double M = quad_m(v.eff, __ldg(v.efl + q), c.g, c.ctot, c.ce);
-        double kf, dlkf, scale = q_rcp(M), add = 0.0;
+        double kf, dlkf, mul = 1.0, scale = 1.0, add = 0.0;
         if (kind == CG_THIRD_BODY) {
-            // q = M (qf - qb): dq/dM = net / M with kf scaled by M
-            kf = M * q_exp(fma(R.b, c.pt.lnT, R.lnA) - R.th * c.pt.invT, c.tab);
+            kf = q_exp(fma(R.b, c.pt.lnT, R.lnA) - R.th * c.pt.invT, c.tab);
             dlkf = fma(R.th, c.pt.invT, R.b) * c.pt.invT;
+            mul = M;
         } else {
             quad_falloff_d(kind, R, v.fall, M, c.pt, c.tab, kf, dlkf, add);
-            scale *= add;
+            scale = add * cgm::cg_rcp(M);
         }
         switch (cls & (kQWide | kQRev)) {
-            case 0: grad_rows<ADJ, false, false>(c, R, kf, dlkf, true, scale, add, out, sum); break;
-            case kQRev: grad_rows<ADJ, false, true>(c, R, kf, dlkf, true, scale, add, out, sum); break;
-            case kQWide: grad_rows<ADJ, true, false>(c, R, kf, dlkf, true, scale, add, out, sum); break;
-            default: grad_rows<ADJ, true, true>(c, R, kf, dlkf, true, scale, add, out, sum); break;
+            case 0: grad_rows<ADJ, false, false>(c, R, kf, dlkf, true, mul, scale, add, out, sum); break;
+            case kQRev: grad_rows<ADJ, false, true>(c, R, kf, dlkf, true, mul, scale, add, out, sum); break;
+            case kQWide: grad_rows<ADJ, true, false>(c, R, kf, dlkf, true, mul, scale, add, out, sum); break;
+            default: grad_rows<ADJ, true, true>(c, R, kf, dlkf, true, mul, scale, add, out, sum); break;
         }
     }
 }

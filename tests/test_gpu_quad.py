@@ -51,11 +51,11 @@ def test_every_kind_and_general_stoichiometry():
     _check(mech, 83)
 
 
-def _derivatives(mech, ng, seed=0):
+def _derivatives(mech, ng, seed=0, states=None):
     """(Jacobian, adjoint) of the kernels and of autograd through the FP64 law."""
     import torch
     from oracle import torch_ref
-    P, T, Y = _cuda(*synthetic.states(mech.ns, ng, seed=seed))
+    P, T, Y = _cuda(*(states or synthetic.states(mech.ns, ng, seed=seed)))
     gm = GpuMechanism(mech)
     G = torch.randn(mech.ns, ng, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(seed))
     p, t, y = (x.clone().requires_grad_(True) for x in (P, T, Y))
@@ -84,6 +84,21 @@ def test_derivatives_of_every_kind(name, ng):
     gT, gY, gP = v
     assert _rel(gY, r[1]) <= 1e-9
     assert _rel(gT[None], r[0][None]) <= 1e-7 and _rel(gP[None], r[2][None]) <= 1e-7
+
+
+def test_derivatives_where_a_third_body_is_zero():
+    # a species without efficiency alone: M = 0, and nothing divides by it
+    mech = synthetic.synthetic_mechanism(10, 24, 10, 0, seed=5)
+    for r in mech.reactions:
+        if r.kind == "third_body":
+            r.efficiencies = {**r.efficiencies, "S3": -1.0}
+    P, T, Y = synthetic.states(mech.ns, 9, seed=1)
+    Y[:] = 0.0
+    Y[3] = 1.0
+    (J64, J32, v), (J, r) = _derivatives(mech, 9, states=(P, T, Y))
+    # (column T is zero but for rounding: relative to the rest)
+    assert _rel(J64, J) <= 1e-9 and _rel(J32, J) <= 1e-6
+    assert _rel(v[1], r[1]) <= 1e-9
 
 
 @pytest.mark.parametrize("mode", ["fp64", "mixed"])
