@@ -40,7 +40,7 @@ size_t mixed_workspace_bytes(const MixedPlan* p, int64_t ng);   // what a caller
 size_t mixed_scratch_bytes(const MixedPlan* p, int64_t ng);     // what the kernel needs
 size_t deriv_workspace_bytes(int ns, int64_t ng);
 struct GradPlan;
-cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, int adjoint, GradPlan** out);
+cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, int adjoint, int f32, GradPlan** out);
 void grad_release(GradPlan* p);
 cudaError_t launch_jacobian_quad(const GradPlan* p, const DevMech& m, int precision, const double* P, const double* T,
                                  const double* Y, void* J, int64_t ng, cudaStream_t s);
@@ -80,6 +80,7 @@ struct chemgen_handle {
     // mode 1 (the generated mixed kernel's arithmetic) serves generated handles
     cg::QuadPlan* quad[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     cg::GradPlan* jacq = nullptr;       // Jacobian on eight-point tiles when every reaction's rows fit
+    cg::GradPlan* jacq32 = nullptr;     // the same for FP32 storage where it differs
     cg::GradPlan* vjpq = nullptr;       // adjoint on eight-point tiles
     cg::JacPlan* jac = nullptr;         // row-owner Jacobian (J written once) otherwise, when its tile fits
     int64_t fp64_slices = 0;        // persistent blocks of the global variant
@@ -574,10 +575,12 @@ int chemgen_create(const void* blob, size_t nbytes, int device, chemgen_handle**
         delete h;
         return status_of(e);
     }
-    e = cg::grad_prepare(h->m, v, device, 1, &h->vjpq);
-    if (e == cudaSuccess || e == cudaErrorNotSupported) e = cg::grad_prepare(h->m, v, device, 0, &h->jacq);
-    if (e == cudaErrorNotSupported) e = cg::jac_prepare(h->m, v, device, &h->jac);
+    e = cg::grad_prepare(h->m, v, device, 1, 0, &h->vjpq);
+    if (e == cudaSuccess || e == cudaErrorNotSupported) e = cg::grad_prepare(h->m, v, device, 0, 0, &h->jacq);
+    if (e == cudaSuccess) e = cg::grad_prepare(h->m, v, device, 0, 1, &h->jacq32);
+    if (e == cudaErrorNotSupported && !h->jacq) e = cg::jac_prepare(h->m, v, device, &h->jac);
     if (e != cudaSuccess && e != cudaErrorNotSupported) {
+        cg::grad_release(h->jacq);
         cg::grad_release(h->vjpq);
         release_quads(h);
         cudaFree(h->dbuf);
@@ -598,6 +601,7 @@ int chemgen_destroy(chemgen_handle* h) {
     release_quads(h);
     if (h->jac) cg::jac_release(h->jac);
     cg::grad_release(h->jacq);
+    cg::grad_release(h->jacq32);
     cg::grad_release(h->vjpq);
     if (h->ws) cudaFree(h->ws);
     if (h->dbuf) cudaFree(h->dbuf);
@@ -637,8 +641,8 @@ int chemgen_jacobian(chemgen_handle* h, int precision, const double* P, const do
     if (precision != 0 && precision != 1) return CHEMGEN_ERR_INVALID_ARGUMENT;
     DeviceGuard g(h->device);
     if (h->max_side > 16) return CHEMGEN_ERR_UNSUPPORTED;
-    if (h->jacq)
-        return status_of(cg::launch_jacobian_quad(h->jacq, h->m, precision, P, T, Y, J, ng, (cudaStream_t)stream));
+    if (const cg::GradPlan* q = precision && h->jacq32 ? h->jacq32 : h->jacq)
+        return status_of(cg::launch_jacobian_quad(q, h->m, precision, P, T, Y, J, ng, (cudaStream_t)stream));
     std::lock_guard<std::mutex> lk(h->mu);
     if (h->jac) {
         st = ensure_ws_locked(h, cg::jac_rows_workspace_bytes(h->jac, h->m, ng));

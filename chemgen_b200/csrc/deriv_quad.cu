@@ -18,12 +18,12 @@
 //   Adjoint: rho = sum_j dL/dC_j C_j = sum_r gq_r s_r, so dL/dY_j needs no
 //     second pass over the species either.
 // What bounds them: the load/store unit (60-70 % busy: state, records, rows)
-// and the issue rate (47 %), with one CTA of 24 warps per SM for the Jacobian
-// (its 2000 rows take 130 KB), two of 12 for the adjoint.  J itself is written
-// once, in 64-byte pieces.  Measured on B200 at 53/325, 65536 points, against
+// and the issue rate (47 %), with one CTA per SM for the Jacobian (its 2000
+// rows take 130 KB; 24 warps, or 32 for FP32 storage), two of 12 for the
+// adjoint.  J itself is written once, in 64-byte pieces.  Measured on B200 at 53/325, 65536 points, against
 // the kernels they replaced (32-point tiles; the Jacobian's derivatives cached
 // in L2 and gathered row by row, the adjoint added into per-warp copies):
-// Jacobian FP64 3.17 -> 1.18 ms, FP32 3.10 -> 1.16 ms, adjoint 1.66 -> 0.42 ms.
+// Jacobian FP64 3.17 -> 1.16 ms, FP32 3.10 -> 1.14 ms, adjoint 1.66 -> 0.42 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -43,7 +43,7 @@ namespace cg {
 // sum itself; an entry of at most four rows is one 16-byte load here.
 struct __align__(16) JEnt {
     unsigned at;                       // k (ns + 1) + j + 1
-    unsigned short k, j;               // byte offsets of bk and of 1/(W_j S): 64 k, 128 j
+    unsigned short k, j;               // byte offsets of bk and of 1/(W_j S): 64 k, 64 j
     unsigned short row[8];
     unsigned short grow[2];
     unsigned pad;
@@ -55,7 +55,7 @@ constexpr int kJRows[] = {1, 2, 3, 4, 6, 8};           // rows of class c / 3; c
 struct __align__(16) JZero {
     unsigned at;                       // k (ns + 1) + 1
     unsigned short k, n;               // 64 k
-    unsigned short j[4];               // 128 j
+    unsigned short j[4];               // 64 j
 };
 static_assert(sizeof(JZero) == 16, "JZero must stay 16 bytes");
 
@@ -105,11 +105,19 @@ struct GradCtx {
     PointT pt;
     double P, lnP, ctot;
     const double2* ce;                 // {C, EGp}
-    const double2* dg;                 // {dE, G}
+    const double* dg;                  // adjoint: pairs {dE, G}; Jacobian: dE
     const double* tab;
     double* out;                       // this lane's slot of row 0
     int g;
 };
+
+// {dE, G} of the species at byte offset `off` of the state.  The Jacobian has
+// no G, and its dE rows are half as long.
+template <bool ADJ>
+__device__ __forceinline__ double2 grad_row(const GradCtx& c, unsigned off) {
+    if (ADJ) return quad_row(reinterpret_cast<const double2*>(c.dg), off);
+    return make_double2(*reinterpret_cast<const double*>(reinterpret_cast<const char*>(c.dg) + (off >> 1)), 0.0);
+}
 
 // Adjoint sums of a lane's reactions.
 struct AdjSums {
@@ -187,7 +195,7 @@ __device__ __forceinline__ void grad_rows(const GradCtx& c, const QRec& R, doubl
         x[j] = a.x;
         if (REV) num = j ? num * a.y : a.y;
         if (REV || ADJ) {
-            const double2 b = quad_row(c.dg, so[j]);
+            const double2 b = grad_row<ADJ>(c, so[j]);
             if (REV) dlKc += b.x;
             if (ADJ) gq -= b.y;
         }
@@ -202,7 +210,7 @@ __device__ __forceinline__ void grad_rows(const GradCtx& c, const QRec& R, doubl
 #pragma unroll
         for (int j = 0; j < N; ++j) {
             const double2 a = quad_row(c.ce, po[j]);
-            const double2 b = quad_row(c.dg, po[j]);
+            const double2 b = grad_row<ADJ>(c, po[j]);
             y[j] = a.x;
             den = j ? den * a.y : a.y;
             dlKc -= b.x;
@@ -215,7 +223,7 @@ __device__ __forceinline__ void grad_rows(const GradCtx& c, const QRec& R, doubl
         qb = kb * (e[0] * y[0]);
     } else if (ADJ) {
 #pragma unroll
-        for (int j = 0; j < N; ++j) gq += quad_row(c.dg, po[j]).y;
+        for (int j = 0; j < N; ++j) gq += grad_row<ADJ>(c, po[j]).y;
     }
     const double net = qf - qb;
     double dT = net * dlkf - (REV ? qb * dlKc : 0.0);
@@ -256,9 +264,9 @@ __device__ __noinline__ AdjSums grad_rows_generic(const DevMech& m, GradCtx c, u
     AdjSums sum;
     if (r == kQNone) return sum;
     const double* s0 = reinterpret_cast<const double*>(c.ce);
-    const double* d0 = reinterpret_cast<const double*>(c.dg);
+    const double* d0 = c.dg;
     const DState st{const_cast<double*>(s0), const_cast<double*>(s0 + 1), const_cast<double*>(d0), nullptr, 2 * kQP,
-                    2 * kQP};
+                    ADJ ? 2 * kQP : kQP};
     Side re, pr;
     RxnGrad rg;
     reaction_grad<16>(m, (int)r, load_rxn(m.rxn + r), c.pt, c.ctot, c.P, c.lnP, st, re, pr, rg);
@@ -376,13 +384,13 @@ __device__ __forceinline__ void grad_chunk(const DevMech& m, const GradView& v, 
     }
 }
 
-// The tile's state {C, EGp}, {dE, G} (for the Jacobian {dE, 1/(W S)}) from its
-// head, Y and G; leaves ctot, P and the temperature functions in c and
+// The tile's state {C, EGp}, {dE, G} (for the Jacobian dE, and 1/(W S) in rows
+// of their own after dE's) from its head, Y and G; leaves ctot, P and the temperature functions in c and
 // returns 1/S, S = sum Y/W.
 template <int W, bool ADJ>
 __device__ __forceinline__ double grad_state(const DevMech& m, const GradView& v, GradCtx& c, bool act, int64_t i,
                                              int64_t ng, const double* h, const double* __restrict__ Y,
-                                             const double* __restrict__ G, int warp, int p, double2* sCE, double2* sDG,
+                                             const double* __restrict__ G, int warp, int p, double2* sCE, double* sDG,
                                              double* sRed) {
     const int ns = m.ns;
     c.pt.T = h[p];
@@ -402,8 +410,12 @@ __device__ __forceinline__ double grad_state(const DevMech& m, const GradView& v
         const double dp = fma(fma(fma(4.0 * cf[5], T, 3.0 * cf[4]), T, 2.0 * cf[3]), T, cf[2]);
         part += x;
         sCE[k * kQP + p] = make_double2(x, q_exp(smh, c.tab) * pfac);
-        sDG[k * kQP + p].x = dp + fma(cf[6], c.pt.invT, cf[1]) * c.pt.invT - c.pt.invT;
-        if (ADJ) sDG[k * kQP + p].y = act ? __ldcs(G + (int64_t)k * ng + i) : 0.0;
+        const double dE = dp + fma(cf[6], c.pt.invT, cf[1]) * c.pt.invT - c.pt.invT;
+        if (ADJ)
+            reinterpret_cast<double2*>(sDG)[k * kQP + p] =
+                make_double2(dE, act ? __ldcs(G + (int64_t)k * ng + i) : 0.0);
+        else
+            sDG[k * kQP + p] = dE;
     }
     part += __shfl_xor_sync(0xffffffffu, part, 8);
     part += __shfl_xor_sync(0xffffffffu, part, 16);
@@ -415,7 +427,7 @@ __device__ __forceinline__ double grad_state(const DevMech& m, const GradView& v
     for (int k = 4 * warp + c.g; k < ns; k += 4 * W) {
         sCE[k * kQP + p].x *= fac;
         // (written after the barrier: the last tile's entries read it before)
-        if (!ADJ) sDG[k * kQP + p].y = __ldg(m.inv_mw + k) * iS;
+        if (!ADJ) sDG[(ns + 1 + k) * kQP + p] = __ldg(m.inv_mw + k) * iS;
     }
     __syncthreads();
     return iS;
@@ -489,15 +501,15 @@ __global__ void __launch_bounds__(32 * W, MINB)
     double* sH = sTab + 16;                                // [2][4][8] heads of this tile and the next
     double* sRed = sH + 8 * kQP;                           // [W][8]
     double2* sCE = reinterpret_cast<double2*>(sRed + W * kQP);   // [ns + 1][8]
-    double2* sDG = sCE + (ns + 1) * kQP;                   // [ns + 1][8]
-    double* sB = reinterpret_cast<double*>(sDG + (ns + 1) * kQP);   // [ns][8] bk
+    double* sDG = reinterpret_cast<double*>(sCE + (ns + 1) * kQP);  // [ns + 1][8] dE, [ns][8] 1/(W S)
+    double* sB = sDG + (2 * ns + 1) * kQP;                 // [ns][8] bk
     double* sV = sB + ns * kQP;                            // [rows + 1][8]
     if (threadIdx.x < 16) sTab[threadIdx.x] = kQExpTab[threadIdx.x];
     if (warp == W - 1 && g == 0) quad_head(sH, (int64_t)blockIdx.x * kQP + p, ng, P, Tg);
     if (threadIdx.x < kQP) {
         sV[v.rows * kQP + p] = 0.0;
         sCE[ns * kQP + p] = make_double2(1.0, 1.0);
-        sDG[ns * kQP + p] = make_double2(0.0, 0.0);
+        sDG[ns * kQP + p] = 0.0;
     }
     __syncthreads();
     GradCtx c;
@@ -522,14 +534,14 @@ __global__ void __launch_bounds__(32 * W, MINB)
         });
         __syncthreads();
         const double* bk = sB + p;
-        const double* wj = reinterpret_cast<const double*>(sDG + p) + 1;   // 1/(W_j S), stride 2 kQP
+        const double* wj = sDG + (ns + 1) * kQP + p;
         const unsigned n32 = (unsigned)ng;                 // the launch function keeps ng below 2^32
         JT* Ji = J + i;
         for_owners<W>(v.lists, v.nown, 0, warp, g, [&](const QOwn& o) {
             const double x = list_sum(v.lists, o, g, sV + p);
             if (o.own < 0 || !act) return;
             const int k = o.own >> 16, col = o.own & 0xffff;   // column 0: T
-            const double y = col ? fma(c.ctot, x, bk[k * kQP]) * wj[(col - 1) * 2 * kQP] : x;
+            const double y = col ? fma(c.ctot, x, bk[k * kQP]) * wj[(col - 1) * kQP] : x;
             __stcs(Ji + (uint64_t)(unsigned)(k * ncol + col) * n32, (JT)y);
         });
         const int r1 = __ldg(v.ebeg + warp + 1);
@@ -561,7 +573,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const double y = b0 * at_byte(wj, j[u]);
-                if (act && u < n) __stcs(Jk + (uint64_t)(j[u] >> 7) * n32, (JT)y);
+                if (act && u < n) __stcs(Jk + (uint64_t)(j[u] >> 6) * n32, (JT)y);
             }
         }
         // the next tile's rows are written after two more barriers
@@ -582,20 +594,20 @@ __global__ void __launch_bounds__(32 * W, MINB)
     double* sH = sTab + 16;                                // [2][4][8] heads of this tile and the next
     double* sRed = sH + 8 * kQP;                           // [4][W][8]
     double2* sCE = reinterpret_cast<double2*>(sRed + 4 * W * kQP);   // [ns + 1][8]
-    double2* sDG = sCE + (ns + 1) * kQP;                   // [ns + 1][8]
-    double* sV = reinterpret_cast<double*>(sDG + (ns + 1) * kQP);   // [rows + 1][8]
+    double* sDG = reinterpret_cast<double*>(sCE + (ns + 1) * kQP);  // [ns + 1][8] pairs
+    double* sV = sDG + 2 * (ns + 1) * kQP;                 // [rows + 1][8]
     double* sW = sV + (v.rows + 1) * kQP;                  // [ns][8], several chunks only
     if (threadIdx.x < 16) sTab[threadIdx.x] = kQExpTab[threadIdx.x];
     if (warp == W - 1 && g == 0) quad_head(sH, (int64_t)blockIdx.x * kQP + p, ng, P, Tg);
     if (threadIdx.x < kQP) {
         sV[v.rows * kQP + p] = 0.0;
         sCE[ns * kQP + p] = make_double2(1.0, 1.0);
-        sDG[ns * kQP + p] = make_double2(0.0, 0.0);
+        reinterpret_cast<double2*>(sDG)[ns * kQP + p] = make_double2(0.0, 0.0);
     }
     __syncthreads();
     GradCtx c;
     c.ce = sCE + p;
-    c.dg = sDG + p;
+    c.dg = sDG + 2 * p;
     c.tab = sTab;
     c.out = sV + lane;
     c.g = g;
@@ -653,6 +665,7 @@ const void* grad_kernel(const GradPlan* p, int precision) {
     if (p->adjoint)
         return p->warps == 8 ? (const void*)vjp_quad<8, 3>
                              : p->warps == 12 ? (const void*)vjp_quad<12, 2> : (const void*)vjp_quad<24, 1>;
+    if (p->warps == 32) return (const void*)jacobian_quad<32, 1, float>;
     if (precision == 0)
         return p->warps == 8 ? (const void*)jacobian_quad<8, 3, double>
                              : p->warps == 12 ? (const void*)jacobian_quad<12, 2, double>
@@ -666,8 +679,10 @@ const void* grad_kernel(const GradPlan* p, int precision) {
 
 // adjoint: any mechanism whose state fits (the reactions run in chunks).
 // Jacobian: the rows of every reaction at once (about 520 reactions), and at
-// most 32767 species-pair codes.  cudaErrorNotSupported otherwise.
-cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, int adjoint, GradPlan** out) {
+// most 32767 species-pair codes.  cudaErrorNotSupported otherwise.  f32: the
+// Jacobian's plan for FP32 storage where it has one of its own (the FP64 plan
+// serves both otherwise, and this returns cudaErrorNotSupported).
+cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, int adjoint, int f32, GradPlan** out) {
     *out = nullptr;
     const int ns = m.ns, nr = m.nr;
     if (nr == 0 || ns >= 0x10000 / kQRow) return cudaErrorNotSupported;
@@ -742,8 +757,15 @@ cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     qbeg.push_back(h.nquad);
     const int fit = (int)(per_sm / (bytes(pl.rows, pl.nchunk, 24) + 1024));
     pl.warps = fit >= 3 ? 8 : fit == 2 ? 12 : 24;
+    if (f32) {
+        // one CTA per SM: 32 warps of 64 registers.  FP32 J at 53/325: 106 -> 97 us
+        // for 5003 points, 581 -> 540 for 32768; FP64 J, whose stores weigh more,
+        // goes from 579 to 599 us there and stays with 24 warps of 80
+        if (pl.warps != 24 || bytes(pl.rows, pl.nchunk, 32) > limit) return cudaErrorNotSupported;
+        pl.warps = 32;
+    }
     pl.smem = bytes(pl.rows, pl.nchunk, pl.warps);
-    const int resident = std::max(1, std::min((int)(per_sm / (pl.smem + 1024)), 24 / pl.warps));
+    const int resident = std::max(1, std::min((int)(per_sm / (pl.smem + 1024)), f32 ? 1 : 24 / pl.warps));
     pl.grid = prop.multiProcessorCount * resident;
     std::vector<int4> run;
     std::vector<int> rbeg;
@@ -839,7 +861,7 @@ cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
             std::memset(&e, 0, sizeof(e));
             e.at = (unsigned)(k * (ns + 1) + col);
             e.k = (unsigned short)(k * 8 * kQP);
-            e.j = (unsigned short)((col - 1) * 16 * kQP);
+            e.j = (unsigned short)((col - 1) * 8 * kQP);
             size_t nr_ = 0, ng_ = 0;
             for (const auto& y : x.second) {
                 const double a = std::fabs(y.second);
@@ -896,7 +918,7 @@ cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
             JZero z;
             z.n = 0;
             for (int j = 0; j <= ns; ++j) {
-                if (j < ns && !ent.count(k << 16 | (j + 1))) z.j[z.n++] = (unsigned short)(j * 16 * kQP);
+                if (j < ns && !ent.count(k << 16 | (j + 1))) z.j[z.n++] = (unsigned short)(j * 8 * kQP);
                 if (z.n == 4 || (j == ns && z.n > 0)) {
                     z.at = (unsigned)(k * (ns + 1) + 1);
                     z.k = (unsigned short)(k * 8 * kQP);

@@ -73,10 +73,14 @@ def _rel(x, ref):
     return float((d / ref.abs().reshape(-1, ref.shape[-1]).amax(0).clamp_min(1e-300)).max())
 
 
-@pytest.mark.parametrize("name,ng", [("all_kinds", 1), ("all_kinds", 19), ("chunks", 9)])
+@pytest.mark.parametrize("name,ng", [("all_kinds", 1), ("all_kinds", 19), ("one_cta", 17), ("chunks", 9)])
 def test_derivatives_of_every_kind(name, ng):
     # 1e-9: the bar of the derivative tests; FP32 storage 1e-6 (half an ulp is 6e-8)
-    mech = synthetic.all_kinds() if name == "all_kinds" else synthetic.synthetic_mechanism(30, 900, 30, 30, seed=3)
+    mech = {"all_kinds": synthetic.all_kinds,
+            # rows for one CTA per SM: 24 warps, 32 for FP32 storage
+            "one_cta": lambda: synthetic.synthetic_mechanism(30, 330, 30, 10, seed=3, n_lindemann=10, n_sri=10,
+                                                             n_plog=10),
+            "chunks": lambda: synthetic.synthetic_mechanism(30, 900, 30, 30, seed=3)}[name]()
     (J64, J32, v), (J, r) = _derivatives(mech, ng, seed=ng)
     for sl in (slice(0, 1), slice(1, None)):
         assert _rel(J64[:, sl], J[:, sl]) <= 1e-9
