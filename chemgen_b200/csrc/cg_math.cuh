@@ -70,11 +70,15 @@ __device__ __forceinline__ double cg_rcp(double x) {
 // of it at every call site.
 static __device__ __noinline__ double cg_log_special(double x) { return log(x); }
 
-__device__ __forceinline__ double cg_log(double x) {
+// normal, finite, positive: biased exponent in [1, 2046], sign clear
+__device__ __forceinline__ bool cg_log_normal(double x) {
+    const int hi = __double2hiint(x);
+    return hi >= 0x00100000 && hi < 0x7ff00000;
+}
+
+__device__ __forceinline__ double cg_log_of_normal(double x) {
     const int hi = __double2hiint(x);
     const int lo = __double2loint(x);
-    // normal, finite, positive: biased exponent in [1, 2046], sign clear
-    if (hi < 0x00100000 || hi >= 0x7ff00000) return cg_log_special(x);
     int e = (hi >> 20) - 1023;
     int mh = (hi & 0x000fffff) | 0x3ff00000;          // m in [1, 2)
     if (mh > 0x3ff6a09e) {                            // m > sqrt(2): use m/2
@@ -97,6 +101,10 @@ __device__ __forceinline__ double cg_log(double x) {
     const double lm = fma(2.0 * s * z, p, 2.0 * s);   // 2 s (1 + z p)
     const double de = (double)e;
     return fma(de, kLn2Hi, fma(de, kLn2Lo, lm));
+}
+
+__device__ __forceinline__ double cg_log(double x) {
+    return cg_log_normal(x) ? cg_log_of_normal(x) : cg_log_special(x);
 }
 
 __device__ __forceinline__ double cg_log10(double x) { return cg_log(x) * 0.4342944819032518; }

@@ -650,8 +650,8 @@ __global__ void __launch_bounds__(kTile * NT, 1)
 // 128-point kernel's, and so is every bit of the result.
 // Bound by latency (34 % of issue slots; FP64 chains, shared loads, records
 // from L1) with 17 warps of 96 registers.  Measured on B200: JetSurf 2.0, 20011
-// points 2.30 -> 1.53 ms, 256 points 1.11 -> 0.30 ms; 348/2163, 20011 points
-// 1.71 -> 1.22 ms, 65536 points 3.43 ms both.
+// points 2.30 -> 1.12 ms, 256 points 1.11 -> 0.22 ms; 348/2163, 20011 points
+// 1.71 -> 0.89 ms, 65536 points 3.43 -> 2.47 ms.
 constexpr int kTP = 32, kTWarps = 16;
 constexpr int kA32 = 1024;             // bytes of a split's 32 rows
 
@@ -733,10 +733,10 @@ __device__ __noinline__ float rate_general32(const DevMech& m, int r, int kind, 
     return (float)rr;
 }
 
-// Falloff and reactions without a pre-decoded form.  Out of line, and with
-// its context in shared memory, so that the common path keeps its values in
-// registers (inline, they went through local memory: 374 instructions a
-// reaction).  The falloff blend is falloff_l2 with the quad kernels' exp.
+// A reaction without a pre-decoded form.  Out of line, like the falloff, and
+// with its context in shared memory, so that the common path keeps its values
+// in registers (inline, they went through local memory: 374 instructions a
+// reaction).
 __device__ __noinline__ float rate_other32(const DevMech& m, const TcFast* fast, int r, const Tile32* t,
                                            const float* sC, const double* sG) {
     const int lane = threadIdx.x & 31;
@@ -749,43 +749,124 @@ __device__ __noinline__ float rate_other32(const DevMech& m, const TcFast* fast,
     c.invT = t->invT[lane];
     c.ctot32 = t->ctot[lane];
     const TcFast F = load_fast(fast + r);
-    const double* tab = t->tab;
     const DRxn R = load_rxn(m.rxn + r);
-    if (!(F.flags & kFastFall)) {
-        if ((R.flags & kFCompact) || r >= m.seg[CG_LINDEMANN] || F.ngen > 32) return rate_of_progress<kTP>(m, r, c, lane);
-        return rate_general32(m, r, r >= m.seg[CG_THIRD_BODY] ? CG_THIRD_BODY : CG_STANDARD,
-                              r >= m.seg[CG_THIRD_BODY] ? third_body32(m, r, F, c.ctot32, sC) : 0.0f, c);
+    if ((R.flags & kFCompact) || r >= m.seg[CG_LINDEMANN] || F.ngen > 32) return rate_of_progress<kTP>(m, r, c, lane);
+    return rate_general32(m, r, r >= m.seg[CG_THIRD_BODY] ? CG_THIRD_BODY : CG_STANDARD,
+                          r >= m.seg[CG_THIRD_BODY] ? third_body32(m, r, F, c.ctot32, sC) : 0.0f, c);
+}
+
+// log of both values, the one's chain beside the other's.
+__device__ __forceinline__ void log_pair(double (&x)[2]) {
+    const double y0 = cgm::cg_log_of_normal(x[0]), y1 = cgm::cg_log_of_normal(x[1]);
+    const bool s0 = !cgm::cg_log_normal(x[0]), s1 = !cgm::cg_log_normal(x[1]);
+    if (s0 || s1) {
+        x[0] = s0 ? cgm::cg_log_special(x[0]) : y0;
+        x[1] = s1 ? cgm::cg_log_special(x[1]) : y1;
+        return;
     }
-    const DFall f = load_fall(m.fall + F.aux);
-    const double x2 = __ldg(&m.fall2[F.aux].T2);
-    int kind = CG_LINDEMANN;
-    while (kind < CG_SRI && r >= m.seg[kind + 1]) ++kind;
-    const float Ms = third_body32(m, r, F, c.ctot32, sC);
+    x[0] = y0;
+    x[1] = y1;
+}
+
+// Two falloff reactions of one kind (STEP 0: one, twice), falloff_l2's blend with
+// the quad kernels' exp, each step of one beside the same step of the other: a
+// chain of FP64 logarithms, exponentials and loads bounds them (JetSurf 2.0,
+// 20011 points: 1.57 ms one after the other, 1.49 ms so).
+template <int STEP>
+__device__ __noinline__ float2 falloff_pair32(const DevMech& m, const TcFast* fast, int r, int kind, const Tile32* t,
+                                              const float* sC, const double* sG) {
+    const int lane = threadIdx.x & 31;
+    const double T = t->T[lane], lnT = t->lnT[lane], invT = t->invT[lane];
+    const double* tab = t->tab;
     constexpr double kLog10_2 = 0.30102999566398119521, kLn2 = 0.69314718055994530942;
-    const double ainf = (fma(R.b, c.lnT, R.lnA) - R.theta * c.invT) * kLog2eD;
-    const double a0 = (fma(f.b0, c.lnT, f.lnA0) - f.theta0 * c.invT) * kLog2eD;
-    const double M = (double)Ms * 2.3283064365386963e-10;   // Ms = M * 2^32
-    const double l2pr = (a0 - ainf) + cgm::cg_log(M) * kLog2eD;
-    const double x = q_exp(fmax(-fabs(l2pr) * kLn2, kQMinArg), tab);   // min(Pr, 1/Pr)
-    const double l2r = fmin(l2pr, 0.0) - cgm::cg_log(1.0 + x) * kLog2eD;
-    double l2F = 0.0;
-    if (kind == CG_TROE) {
-        double Fc = fma(f.p[0], q_exp(fmax(-c.T * f.p[1], kQMinArg), tab),
-                        f.p[2] * q_exp(fmax(-c.T * f.p[3], kQMinArg), tab));
-        if (R.flags & CG_F_TROE_T2) Fc += q_exp(fmax(-x2 * c.invT, kQMinArg), tab);
-        const double lFc = cgm::cg_log10(Fc);
-        const double lp = fma(kLog10_2, l2pr, fma(-0.67, lFc, -0.4));
-        const double f1 = lp * q_rcp(fma(-0.14, lp, fma(-1.27, lFc, 0.75)));
-        l2F = lFc * q_rcp(fma(f1, f1, 1.0)) / kLog10_2;
-    } else if (kind == CG_SRI) {
-        const double lp = kLog10_2 * l2pr;
-        const double X = q_rcp(fma(lp, lp, 1.0));
-        const double base = fma(f.p[0], q_exp(fmax(-f.p[1] * c.invT, kQMinArg), tab),
-                                q_exp(fmax(-c.T * f.p[2], kQMinArg), tab));
-        l2F = (cgm::cg_log(f.p[3]) + fma(X, cgm::cg_log(base), x2 * c.lnT)) * kLog2eD;
+    float Ms[2];
+    {
+        int e0[2], n[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const TcFast F = load_fast(fast + r + j * STEP);
+            e0[j] = F.eff0;
+            n[j] = F.neff < 255 ? F.neff : __ldg(m.eff_ptr + r + j * STEP + 1) - F.eff0;
+            Ms[j] = t->ctot[lane];
+        }
+        for (int e = 0; e < max(n[0], n[1]); e += 4) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                int sp[4];
+                float ev[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const bool ok = e + u < n[j];
+                    sp[u] = ok ? __ldg(m.eff_sp + e0[j] + e + u) : 0;
+                    ev[u] = ok ? (float)__ldg(m.eff_val + e0[j] + e + u) : 0.0f;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float cv = sC[sp[u] * kTP + lane];
+                    if (e + u < n[j]) Ms[j] = fmaf(ev[u], cv, Ms[j]);
+                }
+            }
+        }
     }
-    return net32(F, ainf + (l2r + l2F), 1.0f, reinterpret_cast<const char*>(sC + lane),
-                 reinterpret_cast<const char*>(sG + lane), true);
+    double ainf[2], l2pr[2], x[2], l2r[2], l2F[2] = {0.0, 0.0};
+    const DFall* fr[2];
+    int fl[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const DRxn R = load_rxn(m.rxn + r + j * STEP);
+        fr[j] = m.fall + R.aux;
+        fl[j] = R.flags;
+        const double2 f0 = __ldg(reinterpret_cast<const double2*>(fr[j]));
+        ainf[j] = (fma(R.b, lnT, R.lnA) - R.theta * invT) * kLog2eD;
+        const double a0 = (fma(f0.y, lnT, f0.x) - __ldg(&fr[j]->theta0) * invT) * kLog2eD;
+        l2pr[j] = a0 - ainf[j];
+        x[j] = (double)Ms[j] * 2.3283064365386963e-10;
+    }
+    log_pair(x);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        l2pr[j] = l2pr[j] + x[j] * kLog2eD;
+        x[j] = 1.0 + q_exp(fmax(-fabs(l2pr[j]) * kLn2, kQMinArg), tab);   // 1 + min(Pr, 1/Pr)
+    }
+    log_pair(x);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) l2r[j] = fmin(l2pr[j], 0.0) - x[j] * kLog2eD;
+    if (kind == CG_TROE) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const double2 p01 = __ldg(reinterpret_cast<const double2*>(fr[j]->p));
+            const double2 p23 = __ldg(reinterpret_cast<const double2*>(fr[j]->p) + 1);
+            const double x2 = __ldg(&m.fall2[fr[j] - m.fall].T2);
+            double Fc = fma(p01.x, q_exp(fmax(-T * p01.y, kQMinArg), tab), p23.x * q_exp(fmax(-T * p23.y, kQMinArg), tab));
+            const double e2 = q_exp(fmax(-x2 * invT, kQMinArg), tab);
+            x[j] = (fl[j] & CG_F_TROE_T2) ? Fc + e2 : Fc;
+        }
+        log_pair(x);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const double lFc = x[j] * 0.4342944819032518;                // cg_log10
+            const double lp = fma(kLog10_2, l2pr[j], fma(-0.67, lFc, -0.4));
+            const double f1 = lp * q_rcp(fma(-0.14, lp, fma(-1.27, lFc, 0.75)));
+            l2F[j] = lFc * q_rcp(fma(f1, f1, 1.0)) / kLog10_2;
+        }
+    } else if (kind == CG_SRI) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const DFall f = load_fall(fr[j]);
+            const double lp = kLog10_2 * l2pr[j];
+            const double X = q_rcp(fma(lp, lp, 1.0));
+            const double base = fma(f.p[0], q_exp(fmax(-f.p[1] * invT, kQMinArg), tab),
+                                    q_exp(fmax(-T * f.p[2], kQMinArg), tab));
+            const double x2 = __ldg(&m.fall2[fr[j] - m.fall].T2);
+            l2F[j] = (cgm::cg_log(f.p[3]) + fma(X, cgm::cg_log(base), x2 * lnT)) * kLog2eD;
+        }
+    }
+    float q[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+        q[j] = net32(load_fast(fast + r + j * STEP), ainf[j] + (l2r[j] + l2F[j]), 1.0f,
+                     reinterpret_cast<const char*>(sC + lane), reinterpret_cast<const char*>(sG + lane), true);
+    return make_float2(q[0], q[1]);
 }
 
 // The two reactions r, r + 1 of a warp when one of them has no common form, or
@@ -794,9 +875,22 @@ __device__ __noinline__ float2 rate_pair32(const DevMech& m, const TcFast* fast,
                                            const float* sC, const double* sG) {
     const int lane = threadIdx.x & 31;
     float q[2] = {0.0f, 0.0f};
+    auto kind_of = [&](int k) {
+        int kind = CG_LINDEMANN;
+        while (kind < CG_SRI && k >= m.seg[kind + 1]) ++kind;
+        return kind;
+    };
+    if (r + 1 < m.nr && (load_fast(fast + r).flags & load_fast(fast + r + 1).flags & kFastFall)) {
+        const int kind = kind_of(r);
+        if (r + 1 < m.seg[kind + 1]) return falloff_pair32<1>(m, fast, r, kind, t, sC, sG);
+    }
     for (int j = 0; j < 2; ++j) {
         if (r + j >= m.nr) break;
         const TcFast F = load_fast(fast + r + j);
+        if (F.flags & kFastFall) {
+            q[j] = falloff_pair32<0>(m, fast, r + j, kind_of(r + j), t, sC, sG).x;
+            continue;
+        }
         if (!(F.flags & kFastOn)) {
             q[j] = rate_other32(m, fast, r + j, t, sC, sG);
             continue;
@@ -806,36 +900,36 @@ __device__ __noinline__ float2 rate_pair32(const DevMech& m, const TcFast* fast,
     return make_float2(q[0], q[1]);
 }
 
-// The sums of a group leave tensor memory (lanes 0..31) for wdot, or, for a hot
-// flush, the most-touched species' FP32 sums move into their FP64 accumulators.
-// w: this point's wdot, or NULL.  Out of line: 48 registers of columns beside
-// the main loop's values would spill to local memory, whose 512 x 370 bytes do
-// not stay in the L1 that the tile leaves (83 spills a pair of chunks cost 10k
-// cycles).
-__device__ __noinline__ void flush32(bool hot_end, bool first_group, int nhot, uint32_t tbase, int warp, int npad,
-                 int hot, const int* __restrict__ perm, double* w, int64_t ng) {
-    if (hot_end) {
-        for (int blk = warp >> 2; blk < hot / 16; blk += kTWarps / 4) {
-            float v[16];
-            uint32_t d[32];
-            um::tmem_ld16(um::tmem_lane_addr(tbase, 0, 16 * blk), v);
-            if (nhot > 0) um::tmem_ld32(um::tmem_lane_addr(tbase, 0, npad + 32 * blk), d);
+// The most-touched species' FP32 sums move into their FP64 accumulators
+// (tensor memory lanes 0..31), by the issuing warp.  Out of line, like the
+// function after it: 48 registers of columns beside a loop's values would
+// spill to local memory, whose 512 x 370 bytes do not stay in the L1 that the
+// tile leaves (83 spills a pair of chunks cost 10k cycles).
+__device__ __noinline__ void flush_hot32(int nhot, uint32_t tbase, int npad, int hot) {
+    for (int blk = 0; blk < hot / 16; ++blk) {
+        float v[16];
+        uint32_t d[32];
+        um::tmem_ld16(um::tmem_lane_addr(tbase, 0, 16 * blk), v);
+        if (nhot > 0) um::tmem_ld32(um::tmem_lane_addr(tbase, 0, npad + 32 * blk), d);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const double a = (nhot > 0 ? __hiloint2double((int)d[2 * j + 1], (int)d[2 * j]) : 0.0) +
-                                 (double)v[j];
-                d[2 * j] = (uint32_t)__double2loint(a);
-                d[2 * j + 1] = (uint32_t)__double2hiint(a);
-            }
-            um::tmem_st32(um::tmem_lane_addr(tbase, 0, npad + 32 * blk), d);
-            uint32_t z[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) z[j] = 0u;
-            um::tmem_st16(um::tmem_lane_addr(tbase, 0, 16 * blk), z);
+        for (int j = 0; j < 16; ++j) {
+            const double a = (nhot > 0 ? __hiloint2double((int)d[2 * j + 1], (int)d[2 * j]) : 0.0) + (double)v[j];
+            d[2 * j] = (uint32_t)__double2loint(a);
+            d[2 * j + 1] = (uint32_t)__double2hiint(a);
         }
-        um::tmem_wait_st();
-        return;
+        um::tmem_st32(um::tmem_lane_addr(tbase, 0, npad + 32 * blk), d);
+        uint32_t z[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) z[j] = 0u;
+        um::tmem_st16(um::tmem_lane_addr(tbase, 0, 16 * blk), z);
     }
+    um::tmem_wait_st();
+}
+
+// The sums of a group leave tensor memory for wdot.  w: this point's wdot, or
+// NULL.
+__device__ __noinline__ void flush32(bool first_group, int nhot, uint32_t tbase, int warp, int npad,
+                 int hot, const int* __restrict__ perm, double* w, int64_t ng) {
     for (int col = 16 * (warp >> 2); col < npad; col += 4 * kTWarps) {
         float v[16];
         uint32_t d[32];
@@ -858,12 +952,14 @@ __device__ __noinline__ void flush32(bool hot_end, bool first_group, int nhot, u
     }
 }
 
-// 16 warps compute, a 17th loads the stoichiometry and issues the MMAs.  The
-// compute warps meet only at a tile's prologue: a pair's operands are handed
-// over by mbarriers (full: one arrival a warp; done: the MMAs' commit), so a
-// warp runs up to two pairs ahead of the slowest.  With a block barrier each
-// pair, and the MMAs issued by a compute warp, a pair took 3.5 us instead of
-// 2.9 (348 species, elementary reactions).
+// 16 warps compute, a 17th loads the stoichiometry, issues the MMAs and moves
+// the hot species' sums.  The compute warps meet only at a tile's prologue: a
+// pair's operands are handed over by mbarriers (full: one arrival a warp; done:
+// the MMAs' commit), so a warp runs up to two pairs ahead of the slowest.  The
+// 17th warp's turn is the other half of the pipeline: with descriptors built for
+// every MMA (2000 cycles a pair) and the hot sums moved by compute warps (3900
+// cycles every four pairs) a pair of elementary reactions took 2.9 us, now 2.1
+// (348 species); with a block barrier each pair, 3.5.
 __global__ void __launch_bounds__(32 * (kTWarps + 1), 1)
     getrates_tc32_kernel(const __grid_constant__ DevMech m, const __nv_bfloat16* __restrict__ nu,
                          const TcFast* __restrict__ fast, int npad, int nhalf, int nchunk, uint32_t tcols,
@@ -907,56 +1003,83 @@ __global__ void __launch_bounds__(32 * (kTWarps + 1), 1)
     bool ok = true;
     uint32_t n = 0, nflush = 0;        // pairs and flushes so far, of all tiles
     auto wait = [&](uint64_t* bar, uint32_t use) { ok = ok && um::mbar_wait(bar, use & 1u); };
-    // group and hot_every are even, so a flush falls on the end of a pair
-    auto flush_after = [&](int ch, bool& hot_end) {
-        const bool group_end = (ch % group) == group - 1 || ch == nchunk - 1;
-        hot_end = hot > 0 && !group_end && (ch % hot_every) == hot_every - 1;
+    // chunks so far in the group and since the last hot flush, after nc more
+    // of them: group and hot_every are even, so a flush falls on the end of a
+    // pair (hot flushes: one group per tile)
+    int gpos = 0, hpos = 0;
+    auto flush_after = [&](int ch_end, int nc, bool& hot_end) {
+        gpos += nc;
+        hpos += nc;
+        const bool group_end = gpos == group || ch_end == nchunk;
+        hot_end = hot > 0 && !group_end && hpos == hot_every;
+        if (group_end) gpos = 0;
+        if (group_end || hot_end) hpos = 0;
         return group_end || hot_end;
     };
     if (warp == kTWarps) {
-        if (lane == 0) {
-            const uint32_t idesc = um::idesc_bf16(kTile, nhalf);
-            const int nh = npad / nhalf;
-            auto load = [&](int pr, uint32_t k) {               // pair pr of a tile, pair k of all
-                const uint32_t bytes = (uint32_t)(min(2, nchunk - 2 * pr) * npad * 32);
-                um::mbar_expect_tx(&bfull[k & 1], bytes);
-                um::bulk_g2s(sB + (k & 1) * 2 * npad * 32, nu + (int64_t)2 * pr * npad * kChunk, bytes, &bfull[k & 1]);
-            };
-            const bool any = (int64_t)blockIdx.x < ntiles && npair > 0;
-            bool inflight = any;
-            if (any) load(0, 0);
-            for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-                for (int pr = 0; pr < npair; ++pr, ++n) {
-                    const uint32_t buf = n & 1;
-                    const int ch0 = 2 * pr, nc = min(2, nchunk - ch0);
-                    // the other buffers are free when the last pair's MMAs are done
-                    if (n > 0) wait(&done[buf ^ 1], (n - 1) >> 1);
-                    const bool more = pr + 1 < npair || tile + gridDim.x < ntiles;
-                    if (inflight) ok = um::mbar_wait(&bfull[buf], (n >> 1) & 1u) && ok;   // even after a time-out
-                    inflight = ok && more;
-                    if (inflight) load(pr + 1 < npair ? pr + 1 : 0, n + 1);
-                    wait(&full[buf], n >> 1);
-                    um::fence_after_sync();
-                    for (int cc = 0; cc < nc && ok; ++cc) {
-                        const bool start = ((ch0 + cc) % group) == 0;
-                        const uint32_t ab = um::smem_addr(sA + (buf * 2 + cc) * 3 * kA32);
-                        const uint32_t bs = um::smem_addr(sB + (buf * 2 + cc) * npad * 32);
+        const uint32_t idesc = um::idesc_bf16(kTile, nhalf);
+        const int nh = npad / nhalf;
+        // descriptors of the first operands; others lie a multiple of 16 bytes further
+        const uint64_t ad0 = um::desc_kmajor(um::smem_addr(sA), kChunk, 0);
+        const uint64_t bd0 = um::desc_kmajor(um::smem_addr(sB), kChunk, 0);
+        const uint32_t bstep = (uint32_t)(npad * 32) >> 4, hstep = (uint32_t)(nhalf * 32) >> 4;
+        auto load = [&](int pr, uint32_t k) {                   // pair pr of a tile, pair k of all
+            const uint32_t bytes = (uint32_t)(min(2, nchunk - 2 * pr) * npad * 32);
+            um::mbar_expect_tx(&bfull[k & 1], bytes);
+            um::bulk_g2s(sB + (k & 1) * 2 * npad * 32, nu + (int64_t)2 * pr * npad * kChunk, bytes, &bfull[k & 1]);
+        };
+        const bool any = (int64_t)blockIdx.x < ntiles && npair > 0;
+        bool inflight = any;
+        if (any && lane == 0) load(0, 0);
+        for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+            int nhot = 0;
+            for (int pr = 0; pr < npair; ++pr, ++n) {
+                const uint32_t buf = n & 1;
+                const int ch0 = 2 * pr, nc = min(2, nchunk - ch0);
+                const bool start = gpos == 0;
+                // the other buffers are free when the last pair's MMAs are done
+                if (n > 0) wait(&done[buf ^ 1], (n - 1) >> 1);
+                const bool more = pr + 1 < npair || tile + gridDim.x < ntiles;
+                if (inflight) ok = um::mbar_wait(&bfull[buf], (n >> 1) & 1u) && ok;   // even after a time-out
+                ok = __all_sync(0xffffffffu, ok);
+                inflight = ok && more;
+                if (inflight && lane == 0) load(pr + 1 < npair ? pr + 1 : 0, n + 1);
+                __syncwarp();
+                wait(&full[buf], n >> 1);
+                ok = __all_sync(0xffffffffu, ok);
+                um::fence_after_sync();
+                if (lane == 0) {
+#pragma unroll
+                    for (int cc = 0; cc < 2; ++cc) {
+                        if (cc >= nc || !ok) break;
+                        const uint64_t ad = ad0 + (buf * 2 + cc) * 3 * (kA32 >> 4), bd = bd0 + (buf * 2 + cc) * bstep;
+#pragma unroll
                         for (int s = 0; s < 3; ++s) {
-                            const uint64_t ad = um::desc_kmajor(ab + (uint32_t)(s * kA32), kChunk, 0);
-                            for (int h = 0; h < nh; ++h)
-                                um::mma_bf16(tbase + (uint32_t)(h * nhalf), ad,
-                                             um::desc_kmajor(bs + (uint32_t)(h * nhalf * 32), kChunk, 0), idesc,
-                                             (!start || s > 0) ? 1u : 0u);
+                            const uint32_t acc = (!start || cc > 0 || s > 0) ? 1u : 0u;
+                            um::mma_bf16(tbase, ad + s * (kA32 >> 4), bd, idesc, acc);
+                            if (nh > 1) um::mma_bf16(tbase + (uint32_t)nhalf, ad + s * (kA32 >> 4), bd + hstep, idesc, acc);
                         }
                     }
                     um::commit(&done[buf]);
-                    bool hot_end;
-                    if (flush_after(ch0 + nc - 1, hot_end)) {
+                }
+                __syncwarp();
+                bool hot_end;
+                if (flush_after(ch0 + nc, nc, hot_end)) {
+                    if (hot_end) {
+                        wait(&done[buf], n >> 1);
+                        ok = __all_sync(0xffffffffu, ok);
+                        um::fence_after_sync();
+                        if (ok) flush_hot32(nhot, tbase, npad, hot);
+                        ++nhot;
+                        um::fence_before_sync();
+                        __syncwarp();
+                    } else {
                         wait(flushed, nflush);
                         ++nflush;
-                        um::fence_after_sync();
                     }
+                    um::fence_after_sync();
                 }
+            }
         }
     } else {
         const int rsub = (warp >> 3) * kChunk + 2 * (warp & 7);     // this warp's two reactions of a pair
@@ -1040,20 +1163,23 @@ __global__ void __launch_bounds__(32 * (kTWarps + 1), 1)
                 __syncwarp();
                 if (lane == 0) um::mbar_arrive(&full[buf]);
                 bool hot_end;
-                if (!flush_after(ch0 + nc - 1, hot_end)) continue;
+                if (!flush_after(ch0 + nc, nc, hot_end)) continue;
+                if (hot_end) {
+                    ++nhot;
+                    continue;
+                }
                 // the tile's sums are in lanes 0..31: the warps of that quadrant take
                 // them out while the others go on
                 if ((warp & 3) == 0) {
                     wait(&done[buf], n >> 1);
                     ok = __all_sync(0xffffffffu, ok);
                     um::fence_after_sync();
-                    if (ok) flush32(hot_end, first_group, nhot, tbase, warp, npad, hot, perm, act ? wdot + i : nullptr, ng);
+                    if (ok) flush32(first_group, nhot, tbase, warp, npad, hot, perm, act ? wdot + i : nullptr, ng);
                     um::fence_before_sync();
                     __syncwarp();
                     if (lane == 0) um::mbar_arrive(flushed);
                 }
-                if (hot_end) ++nhot;
-                else first_group = false;
+                first_group = false;
             }
         }
     }
@@ -1246,12 +1372,12 @@ cudaError_t launch_getrates_mixed(const MixedPlan* p, const DevMech& m, const do
     // the launch (a plan made later for a smaller mechanism sets it lower)
     static std::mutex mu;
     // Mechanisms whose Gibbs terms fit beside the 128-point tile run the faster
-    // of the two: on B200 at 53/325 a round of 32-point tiles takes 47 us and a
-    // wave of 128-point tiles 121 us.  Larger ones always run 32-point tiles
-    // (348/2163: a round 0.22 ms, a wave 0.82 ms).
+    // of the two: on B200 at 53/325 a round of 32-point tiles takes 40 us and a
+    // wave of 128-point tiles 121 us (9/21: 12 and 29).  Larger ones always run
+    // 32-point tiles (348/2163: a round 0.17 ms, a wave 0.82 ms).
     const int64_t rounds = (ng + (int64_t)kTP * p->grid32 - 1) / std::max<int64_t>(1, (int64_t)kTP * p->grid32);
     const int64_t waves = (ng + (int64_t)kTile * p->grid - 1) / ((int64_t)kTile * p->grid);
-    if (p->t32 && (!p->g_smem || (double)rounds * 0.39 <= (double)waves)) {
+    if (p->t32 && (!p->g_smem || (double)rounds * 0.35 <= (double)waves)) {
         const unsigned g32 = (unsigned)std::min<int64_t>((ng + kTP - 1) / kTP, p->grid32);
         std::lock_guard<std::mutex> lk(mu);
         const cudaError_t e = cudaFuncSetAttribute(getrates_tc32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -146,6 +146,18 @@ def test_mixed_32_point_tiles(ng):
     assert oracle.errors(w[:, idx], r["wdot"], r["S"])["norm_max"] <= 1e-6
 
 
+@pytest.mark.parametrize("kinds", [(5, 0, 0), (0, 1, 4), (3, 3, 3), (40, 33, 30)])
+def test_mixed_32_point_tiles_falloff(kinds):
+    # pairs of one falloff kind, pairs across two kinds and single ones; 1e-6 as above
+    n_lind, n_troe, n_sri = kinds
+    mech = synthetic.synthetic_mechanism(40, 60 + sum(kinds), 7, n_troe, seed=2, n_lindemann=n_lind, n_sri=n_sri)
+    blob = pack.pack(mech).to_blob()
+    P, T, Y = synthetic.states(mech.ns, 45, seed=1)
+    w = GpuMechanism(blob).getrates(*_cuda(P, T, Y), mode="mixed").cpu().numpy()
+    r = oracle.rates(blob, P, T, Y, mech.nr)
+    assert oracle.errors(w, r["wdot"], r["S"])["norm_max"] <= 1e-6
+
+
 @pytest.mark.parametrize("rows,cols", [(1 << 19, 1), (1, 1 << 19), (9893, 53), (53, 9893), (8129, 65), (348, 1507)])
 def test_transposed_copies(rows, cols):
     # tiles of 64 x 64: whole, part and single-row ones; the values are moved, not computed
