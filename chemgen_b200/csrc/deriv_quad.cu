@@ -28,7 +28,6 @@
 
 #include <algorithm>
 #include <map>
-#include <mutex>
 #include <utility>
 #include <vector>
 
@@ -677,6 +676,8 @@ const void* grad_kernel(const GradPlan* p, int precision) {
 
 }  // namespace
 
+void grad_release(GradPlan* p);
+
 // adjoint: any mechanism whose state fits (the reactions run in chunks).
 // Jacobian: the rows of every reaction at once (about 520 reactions), and at
 // most 32767 species-pair codes.  cudaErrorNotSupported otherwise.  f32: the
@@ -940,8 +941,10 @@ cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     const size_t o_je = im.put(jent), o_er = im.put(erun), o_eb = im.put(ebeg);
     GradPlan* p = new GradPlan(pl);
     e = im.upload(&p->dbuf);
+    for (int precision = 0; precision < 2 && e == cudaSuccess; ++precision)
+        e = raise_smem_limit(grad_kernel(p, precision), p->smem);
     if (e != cudaSuccess) {
-        delete p;
+        grad_release(p);
         return e;
     }
     char* d = (char*)p->dbuf;
@@ -975,17 +978,10 @@ GradView grad_view(const GradPlan* p) {
                     p->efl, p->eff, p->fall, p->th, p->lists, p->rlists, p->ent, p->erun, p->ebeg, p->zero};
 }
 
-// The shared-memory limit of a kernel instance is set and the kernel launched
-// under one lock (plans of several handles share the instances).
 cudaError_t launch_grad(const GradPlan* p, int precision, int64_t ng, void** args, cudaStream_t s) {
     const int64_t tiles = (ng + kQP - 1) / kQP;
-    static std::mutex mu;
-    std::lock_guard<std::mutex> lk(mu);
-    const void* fn = grad_kernel(p, precision);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
-    if (e != cudaSuccess) return e;
-    return cudaLaunchKernel(fn, dim3((unsigned)std::min<int64_t>(tiles, p->grid)), dim3(32u * (unsigned)p->warps), args,
-                            p->smem, s);
+    return cudaLaunchKernel(grad_kernel(p, precision), dim3((unsigned)std::min<int64_t>(tiles, p->grid)),
+                            dim3(32u * (unsigned)p->warps), args, p->smem, s);
 }
 }  // namespace
 

@@ -27,7 +27,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <mutex>
 #include <utility>
 #include <vector>
 
@@ -571,9 +570,7 @@ cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     const size_t o_li = im.put(lb.own), o_le = im.put(lb.ent), o_lg = im.put(lb.gen);
     QuadPlan* q = new QuadPlan(pl);
     e = im.upload(&q->dbuf);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(quad_kernel(q->warps, mixed), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)q->smem);
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)quad_kernel(q->warps, mixed), q->smem);
     if (e != cudaSuccess) {
         if (q->dbuf) cudaFree(q->dbuf);
         delete q;
@@ -606,15 +603,7 @@ cudaError_t launch_getrates_quad(const QuadPlan* p, const DevMech& m, const doub
     const int64_t tiles = (n1 - i0 + kQP - 1) / kQP;
     const unsigned grid = (unsigned)std::min<int64_t>(tiles, p->grid);
     const QuadView v{p->nchunk, p->nsq, p->rows, p->rec, p->run, p->efl, p->eff, p->fall, p->rbeg, p->th, p->lists};
-    // Every plan of the same kernel instance (one per handle) has its own
-    // shared-memory size: the limit is set and the kernel launched under one
-    // lock, so that a handle made later for a smaller mechanism cannot leave
-    // the limit below this plan's.
-    static std::mutex mu;
-    std::lock_guard<std::mutex> lk(mu);
     const QuadKernel fn = quad_kernel(p->warps, p->mixed);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
-    if (e != cudaSuccess) return e;
     fn<<<grid, 32u * (unsigned)p->warps, p->smem, s>>>(m, v, P, T, Y, wdot, i0, ng, n1, count);
     return cudaGetLastError();
 }

@@ -24,6 +24,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "cg_math.cuh"
@@ -655,6 +656,19 @@ inline void build_runs(const HostQuads& h, const std::vector<int>& qbeg, int war
             }
             beg.push_back((int)run.size());
         }
+}
+
+// Raises a kernel's limit of dynamic shared memory to `bytes` on the current
+// device.  Every plan of one kernel instance (one per handle) has its own size:
+// the limit is never lowered, so a launch needs no call and no lock for it
+// (0.5 us of a small batch's 12).
+inline cudaError_t raise_smem_limit(const void* fn, size_t bytes) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+    if (e != cudaSuccess || (size_t)fa.maxDynamicSharedSizeBytes >= bytes) return e;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 // Host image of a plan's tables, copied to the device in one piece.
