@@ -15,15 +15,15 @@
 // What bounds it: the load/store unit's 128 bytes per clock (70 % busy at
 // 348 species: the four 16-byte state loads of a reaction, its record, the
 // list rows) and the issue rate (53 %).  Measured on B200, FP64: 348/2163,
-// 2^17 points, 5.63 -> 3.29 ms against the kernel it replaced (32-point tiles,
+// 2^17 points, 5.63 -> 3.14 ms against the kernel it replaced (32-point tiles,
 // one reaction a warp, 13 chunks with two barriers each); JetSurf 2.0 3.6 ms;
-// 53/325 on the table-driven path 191 -> 272 Mpts/s.  A loop per class (build_runs)
-// is 18 % faster than a dispatch per quad (3.31 against 4.04 ms at 348/2163).
+// 53/325 on the table-driven path 191 -> 290 Mpts/s.  A loop per class (build_runs)
+// is 18 % faster than a dispatch per quad (3.31 against 4.04 ms at 348/2163, then).
 // The mixed form repeats the generated mixed kernel's arithmetic to the last
 // bit: FP64 exponents, FP32 2^f, products and falloff blend, the sums over
 // species and reactions in the generated code's order.  It runs the batches
 // (and the remainders past whole waves) that would leave the generated
-// kernel's wave mostly empty: 53/325, 4096 points, FP64 98 -> 27 us.
+// kernel's wave mostly empty: 53/325, 4096 points, FP64 98 -> 21 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
