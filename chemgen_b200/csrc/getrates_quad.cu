@@ -12,9 +12,9 @@
 //   3  species quads: wdot = sum nu q from per-species row lists
 //      (reactions/standard.j2:21-27), each species with one owner, so no
 //      atomics and one order of summation.
-// What bounds it: the load/store unit's 128 bytes per clock (70 % busy at
+// What bounds it: the load/store unit's 128 bytes per clock (76 % busy at
 // 348 species: the four 16-byte state loads of a reaction, its record, the
-// list rows) and the issue rate (53 %).  Measured on B200, FP64: 348/2163,
+// list rows) and the issue rate (59 %).  Measured on B200, FP64: 348/2163,
 // 2^17 points, 5.63 -> 3.14 ms against the kernel it replaced (32-point tiles,
 // one reaction a warp, 13 chunks with two barriers each); JetSurf 2.0 3.6 ms;
 // 53/325 on the table-driven path 191 -> 290 Mpts/s.  A loop per class (build_runs)
