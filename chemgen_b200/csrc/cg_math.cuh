@@ -103,8 +103,12 @@ __device__ __forceinline__ double cg_log_of_normal(double x) {
     return fma(de, kLn2Hi, fma(de, kLn2Lo, lm));
 }
 
+// (As an early return: written as a conditional expression, the compiler's
+// code for the generated FP64 kernel at 53/325 took 1480 instead of 1467 us
+// for 2^20 points.)
 __device__ __forceinline__ double cg_log(double x) {
-    return cg_log_normal(x) ? cg_log_of_normal(x) : cg_log_special(x);
+    if (!cg_log_normal(x)) return cg_log_special(x);
+    return cg_log_of_normal(x);
 }
 
 __device__ __forceinline__ double cg_log10(double x) { return cg_log(x) * 0.4342944819032518; }

@@ -112,7 +112,8 @@ typedef int (*chemgen_kernel_fn)(int mode, const double* P, const double* T, int
                                  double* wdot, void* stream);
 int chemgen_register_kernels(uint64_t fingerprint, int ns, int nr, unsigned modes, chemgen_kernel_fn fn);
 /* A generated module's kernel of one mode over the points [i0, i1) of arrays
- * laid out for ng points, `block` points per SM and wave.  With it, a batch
+ * laid out for ng points, `block` points per SM and wave.  The library calls
+ * it with i0 = 0 and i1 a multiple of `block`.  With it, a batch
  * that leaves most of its last wave empty runs that remainder (or all of a
  * small batch) on the table-driven tile kernel of the same arithmetic. */
 typedef int (*chemgen_kernel_range_fn)(int mode, const double* P, const double* T, int64_t ng, const double* Y,

@@ -135,3 +135,17 @@ def test_generated_53_species_kernels_fit_their_register_budget(tmp_path):
     for name, (regs, spill) in info.items():
         assert regs * shapes[name] <= E.REG_FILE, (name, regs)
         assert spill <= 64, (name, spill)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_kernels_test_their_points_against_the_stride(mixed):
+    # one count in the kernel: the array's.  A launch over fewer points covers whole blocks,
+    # whose threads all pass this test
+    name = "cg_gen_mixed" if mixed else "cg_gen_fp64"
+    src = E.emit(synthetic.h2o2_10sp(), precision="mixed" if mixed else "fp64")
+    params, body = src.split(name + "(", 1)[1].split(") {", 1)
+    assert params.replace("\n", " ").split(", ")[-1] == "int64_t ng" and params.count("int64_t") == 1
+    assert "const bool act = i < ng;" in body
+    block = int(re.search(r"__launch_bounds__\((\d+), 1\) " + name, src).group(1))
+    assert f"if (i1 < ng && i1 % {block}) return CHEMGEN_ERR_INVALID_ARGUMENT;" in src
+    assert f", {block}, &launch_range);" in src
