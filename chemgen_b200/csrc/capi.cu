@@ -25,6 +25,7 @@ struct QuadPlan;
 cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, int mixed, int latency,
                          QuadPlan** out);
 int quad_tile_points();
+int quad_general(const QuadPlan* p);   // reactions without a pre-decoded form
 void quad_release(QuadPlan* p);
 cudaError_t launch_getrates_quad(const QuadPlan* p, const DevMech& m, const double* P, const double* T,
                                  const double* Y, double* wdot, int64_t i0, int64_t ng, int64_t n1, cudaStream_t s,
@@ -421,25 +422,41 @@ int launch_tiles(chemgen_handle* h, int mode, const double* P, const double* T, 
 // The generated kernel, one point per thread, takes about as long for one
 // block as for a whole wave of one block per SM; the tile kernel takes time
 // in proportion to its tiles.  So the points past the last whole wave (all of
-// a small batch) run on the tile kernel when that is faster.  Both times,
-// fitted to B200 measurements at 9/23 and 53/325 (us):
-//   wave: FP64 12 and 103, mixed 10 and 68, linear in the reactions;
-//   eight-point tiles, one per SM at a time: FP64 1.6 and 4.4, mixed 1.5 and
-//   4.8, linear in the quads of four reactions (8 and 91).
-// (53/325 FP64: the line lies at 27500 of a wave's 75776 points; 25000 take the
-// tile kernel 92 us.)
-bool tiles_faster(const chemgen_handle* h, int mode, int64_t n) {
-    const double nr = h->nr, nq = 0.28 * nr, tiles = (double)n / cg::quad_tile_points() / h->sm_count;
-    const double wave = mode ? 5.6 + 0.192 * nr : 5.1 + 0.301 * nr;
-    const double tile = mode ? 1.2 + 0.0400 * nq : 1.3 + 0.0341 * nq;
-    return tiles * tile < wave;
+// a small batch) run on the tile kernel when that is faster.  Both times (us,
+// code in L2), fitted to B200 measurements of ten mechanisms of 9 to 53 species:
+//   wave: linear in the reactions, a falloff counted as three and a PLOG
+//   reaction as six (FP64 9/23 10, 20/60 of every kind 33, 30/150 with 20 PLOG
+//   66, 53/325 102, with 60 PLOG 160, with 60 of fractional coefficients 91);
+//   eight-point tiles, one per SM at a time: linear in the reactions, a falloff
+//   six times another's time, PLOG and the other reactions without a
+//   pre-decoded form five and two and a half times, and 0.5 us for the first of
+//   these (FP64 9/23 1.5, 20/60 2.9, 30/150 3.7, 53/325 4.4, 6.7 and 5.8).
+// Past a wave the tiles are a second launch, the generated kernel's points one
+// more wave of the same: 8 us (mixed, whose wave hides less of it, 4).  A wave
+// of under 16 us is little more than a launch: there the tiles serve four rounds
+// at most (9/23 FP64, 4736 points 10 us either way, 8192 points 14 against 10).  The FP64 lines lie at 27100 points
+// for 53/325 (24000: tiles 90, wave 102; 28000: 105 and 103) and 25000 past a
+// wave, at 20700 and 19000 with 60 fractional reactions (24227 past a wave:
+// tiles 118, wave 92).  With other data in L2 a wave takes twice the time
+// (53/325 223 us), the tiles a few us more: hence no margin on the tiles' side.
+bool tiles_faster(const chemgen_handle* h, int mode, int64_t n, bool remainder) {
+    const int* seg = h->m.seg;
+    const int nr = h->nr, nfall = seg[CG_PLOG] - seg[CG_LINDEMANN], nplog = nr - seg[CG_PLOG];
+    const int general = cg::quad_general(h->quad[mode][0]);    // PLOG among them
+    const double rounds = (double)n / cg::quad_tile_points() / h->sm_count;
+    const double wave = 5.0 + (mode ? 0.16 : 0.25) * (nr + 2 * nfall + 5 * nplog);
+    const double tile = mode ? 1.2 + 0.0101 * nr
+                             : 1.3 + 0.0065 * nr + 0.034 * nfall +
+                                   (general ? 0.5 + 0.0325 * nplog + 0.016 * (general - nplog) : 0.0);
+    if (wave < 16.0) return !remainder && rounds <= 4.0;
+    return rounds * tile + (remainder ? (mode ? 4.0 : 8.0) : 0.0) < wave;
 }
 
 int launch_generated(chemgen_handle* h, int mode, const double* P, const double* T, int64_t ng, const double* Y,
                      double* w, cudaStream_t s) {
     if (h->gen_range[mode] && h->quad[mode][0]) {
         const int64_t wave = (int64_t)h->gen_block[mode] * h->sm_count, full = ng / wave * wave;
-        if (ng > full && tiles_faster(h, mode, ng - full)) {
+        if (ng > full && tiles_faster(h, mode, ng - full, full > 0)) {
             const int st = full ? h->gen_range[mode](mode, P, T, ng, Y, w, 0, full, s) : CHEMGEN_OK;
             return st ? st : launch_tiles(h, mode, P, T, full, ng, Y, w, s);
         }

@@ -37,7 +37,7 @@ namespace cg {
 
 struct QuadPlan {
     int nquad = 0, nchunk = 0, nsq = 0, rows = 0, warps = 0;
-    int mixed = 0;
+    int mixed = 0, general = 0;        // general: reactions of kQKindGeneric
     size_t smem = 0;
     int grid = 0;
     const QRec* rec = nullptr;
@@ -442,6 +442,7 @@ static QuadKernel quad_kernel(int warps, int mixed) {
 constexpr int kQuadMaxSpecies = 434;
 
 int quad_tile_points() { return kQP; }
+int quad_general(const QuadPlan* p) { return p->general; }
 
 // latency: 32 warps to a tile whatever its size, for batches of few tiles.
 cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, int mixed, int latency,
@@ -459,6 +460,7 @@ cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     QuadPlan pl;
     pl.mixed = mixed;
     pl.nquad = h.nquad;
+    pl.general = h.ngeneric;
     // chunks: every reaction at once when the rates fit beside the state
     auto bytes = [&](int rows, int chunks, int warps) {
         return (16 + ((size_t)8 + 2 * (ns + 1) + rows + 1 + warps + (chunks > 1 ? ns : 0)) * kQP) * sizeof(double);

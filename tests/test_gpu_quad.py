@@ -132,6 +132,31 @@ def test_small_batches_and_remainders_equal_the_generated_kernel(name, mode):
         assert all(bool((run(0, n) == ref[:, :n]).all()) for n in (1, 1184, 1185, 3001))
 
 
+@pytest.mark.parametrize("name,waves,n,tiles", [
+    ("h2_burke", 0, 1000, True), ("h2_burke", 0, 8192, False), ("h2_burke", 1, 500, False), ("all_kinds", 0, 4000, True), ("all_kinds", 0, 16000, False),
+    ("gri30", 0, 20000, True), ("gri30", 0, 30000, False), ("all_kinds", 1, 2000, True), ("all_kinds", 1, 12000, False)])
+def test_which_kernel_a_batch_of_a_generated_mechanism_runs_on(name, waves, n, tiles):
+    # the FP64 tile kernel adds in another order than the generated one, so its bits
+    # tell which of them ran: the last n points of a batch against the same points
+    # in a whole wave (the generated kernel's)
+    import torch
+    from chemgen_b200 import emit_cuda as E
+    from conftest import load_golden
+    mech = synthetic.all_kinds() if name == "all_kinds" else load_golden(name)[0]
+    gm = GpuMechanism(mech, generated=True)
+    wave = (E.choose_block(mech.ns, False, E.use_tmem(mech.ns, False)) *
+            torch.cuda.get_device_properties(0).multi_processor_count)
+    P, T, Y = _cuda(*synthetic.states(mech.ns, wave + n, seed=8))
+    k = n + waves * wave                                   # the batch, and the wave that ends where it does
+
+    def run(a, b):
+        return gm.getrates(P[a:b].contiguous(), T[a:b].contiguous(), Y[:, a:b].contiguous())
+    w, ref = run(0, k)[:, k - n:], run(k - wave if waves else 0, k if waves else wave)
+    ref = ref[:, wave - n:] if waves else ref[:, :n]
+    assert bool((w == ref).all()) == (not tiles)
+    assert _rel(w, ref) <= 1e-12
+
+
 @pytest.mark.parametrize("ng", [1, 31, 33, 32 * 148 + 7])
 def test_mixed_32_point_tiles(ng):
     # part tiles and more tiles than SMs on the 32-point tensor-core kernel; 1e-6
