@@ -507,6 +507,36 @@ int run_owned(chemgen_handle* h, int mode, const double* P, const double* T, int
     return launch(h, mode, P, T, ng, Y, w, h->ws, h->ws_bytes, s);
 }
 
+bool is_pageable(const void* p) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return true;
+}
+
+// Points per chunk of the host pipeline: at most 65536 or a sixteenth of all.
+// From pinned memory more and smaller chunks overlap the two copy directions
+// and the kernel, but a chunk's six calls take the host ~30 us and its copies
+// are rows of one species each, so their number goes with the square root of
+// the input's size up to four, and to eight from 150 MB.  Measured in 1, 2, 4
+// and 8 chunks (FP64, us): 9 species 30000 points (2.6 MB) 131, 129, 160, 218;
+// 53 species 10000 points (4.4 MB) 235, 199, 217, 272, 200000 points (88 MB)
+// 3515, 2755, 2478, 2506, 400000 points 6990, 5350, 4760, 4620; 348 species
+// 16000 points (45 MB) 2150, 1570, 1510, 1450.
+// Pageable memory is staged by the driver while the host waits, so there is
+// nothing for more chunks to overlap (9 species, 30000 points: 0.70 ms in four
+// chunks, 0.33 in one; 53 species 2.1 and 1.5).
+int64_t host_chunk(int ns, int64_t ng, const void* in, const void* out) {
+    const int64_t most = std::max<int64_t>(1 << 16, (ng + 15) / 16);
+    const double bytes = 8.0 * (ns + 2) * (double)ng;
+    const int64_t n = bytes >= 150e6 ? 8 : std::min<int64_t>(4, std::llround(std::sqrt(bytes / 0.8e6)));
+    // (asked last: it takes 2 to 5 us a pointer)
+    if (n <= 1 || is_pageable(in) || is_pageable(out)) return std::min(ng, most);
+    // (whole 8 KB of a row; the last chunk, which nothing overlaps, is the short
+    // one: 53 species, 30000 points in four of 8192 495 us, in three of 10240 518)
+    return std::min(((ng + n - 1) / n + 1023) / 1024 * 1024, most);
+}
+
 std::mutex g_mu;
 chemgen_handle* g_handle = nullptr;
 
@@ -767,14 +797,7 @@ int chemgen_getrates_host(chemgen_handle* h, int mode, const double* P, const do
     // reused (its in-order queue waiting for chunk c's copy back) only three
     // chunks later: both copy directions stay busy.
     constexpr int NS = chemgen_handle::kIoStreams;
-    // An eighth of the points a chunk, so that both copy directions overlap
-    // from ~10^4 points on (53 species: 30000 points 0.57 -> 0.49 ms, 80000
-    // points 1.28 -> 1.20 ms against one or two chunks of 65536), not under
-    // 8192 (64 KB a species' row: more chunks cost more row copies than they
-    // hide; 16 chunks at 200000 points 2.41 -> 2.8 ms) and not over 65536 or a
-    // sixteenth (2^20 points and up).
-    const int64_t most = std::max<int64_t>(1 << 16, (ng + 15) / 16);
-    const int64_t chunk = std::min<int64_t>(ng, std::max<int64_t>(8192, std::min((ng + 7) / 8, most)));
+    const int64_t chunk = host_chunk(ns, ng, Y, wdot);
     const size_t per = (size_t)(2 + 2 * ns) * chunk;       // P, T, Y, wdot doubles of one chunk
     std::lock_guard<std::mutex> lk(h->mu);
     cudaError_t e = cudaSuccess;

@@ -157,6 +157,24 @@ def test_which_kernel_a_batch_of_a_generated_mechanism_runs_on(name, waves, n, t
     assert _rel(w, ref) <= 1e-12
 
 
+@pytest.mark.parametrize("name,ng,pinned", [("gri30", 60000, False), ("synthetic_plog_15_40", 50000, True)])
+def test_host_calls_that_gain_nothing_from_chunks_take_one(name, ng, pinned):
+    # pageable arrays and small states: one chunk, so the generated kernel serves all
+    # of it and the FP64 bits are the device call's (chunks of 8192 points run on the
+    # tile kernel)
+    import torch
+    from conftest import load_golden
+    mech = load_golden(name)[0]
+    gm = GpuMechanism(mech, generated=True)
+    P, T, Y = synthetic.states(mech.ns, ng, seed=9)
+    w = gm.getrates(*_cuda(P, T, Y)).cpu()
+    if pinned:
+        P, T, Y = (torch.from_numpy(x).pin_memory() for x in (P, T, Y))
+    out = torch.empty(mech.ns, ng, dtype=torch.float64, pin_memory=pinned)
+    gm.getrates_host(P, T, Y, out=out if pinned else out.numpy())
+    assert torch.equal(out, w)
+
+
 @pytest.mark.parametrize("ng", [1, 31, 33, 32 * 148 + 7])
 def test_mixed_32_point_tiles(ng):
     # part tiles and more tiles than SMs on the 32-point tensor-core kernel; 1e-6
