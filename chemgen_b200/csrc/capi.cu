@@ -593,16 +593,16 @@ int chemgen_create(const void* blob, size_t nbytes, int device, chemgen_handle**
         delete h;
         return st;
     }
-    cudaDeviceProp prop;
-    cudaError_t e = cudaGetDeviceProperties(&prop, device);
+    cg::DeviceLimits dev;
+    cudaError_t e = cg::device_limits(device, &dev);
     if (e != cudaSuccess) {
         cudaFree(h->dbuf);
         delete h;
         return status_of(e);
     }
-    h->sm_count = prop.multiProcessorCount;
+    h->sm_count = dev.sms;
     long smem_pts = 0;
-    h->fp64_block = cg::fp64_smem_block(h->ns, prop.sharedMemPerMultiprocessor, prop.sharedMemPerBlockOptin,
+    h->fp64_block = cg::fp64_smem_block(h->ns, dev.smem_sm, dev.smem_block,
                                         &smem_pts);
     h->fp64_slices = (int64_t)h->sm_count * cg::fp64_global_blocks_per_sm();
     // The quad kernel whenever its tile fits: it is the FP64 kernel when the

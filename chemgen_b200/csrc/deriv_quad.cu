@@ -697,10 +697,10 @@ cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     const int32_t* ep = (const int32_t*)v.a[CG_EFF_PTR];
     const int32_t* es = (const int32_t*)v.a[CG_EFF_SP];
     const double* ev = (const double*)v.a[CG_EFF_VAL];
-    cudaDeviceProp prop;
-    cudaError_t e = cudaGetDeviceProperties(&prop, device);
+    DeviceLimits dev;
+    cudaError_t e = device_limits(device, &dev);
     if (e != cudaSuccess) return e;
-    const size_t limit = prop.sharedMemPerBlockOptin, per_sm = prop.sharedMemPerMultiprocessor;
+    const size_t limit = dev.smem_block, per_sm = dev.smem_sm;
     HostQuads h;
     build_quads(v, h, adjoint != 0);
     auto uses_m = [&](int r) {
@@ -767,7 +767,7 @@ cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     }
     pl.smem = bytes(pl.rows, pl.nchunk, pl.warps);
     const int resident = std::max(1, std::min((int)(per_sm / (pl.smem + 1024)), f32 ? 1 : 24 / pl.warps));
-    pl.grid = prop.multiProcessorCount * resident;
+    pl.grid = dev.sms * resident;
     std::vector<int4> run;
     std::vector<int> rbeg;
     build_runs(h, qbeg, pl.warps, run, rbeg);

@@ -350,13 +350,13 @@ struct JacPlan {
 cudaError_t jac_prepare(const DevMech& m, const cg_mech_view& v, int device, JacPlan** out) {
     *out = nullptr;
     const int ns = m.ns, nr = m.nr;
-    cudaDeviceProp prop;
-    cudaError_t e = cudaGetDeviceProperties(&prop, device);
+    DeviceLimits dev;
+    cudaError_t e = device_limits(device, &dev);
     if (e != cudaSuccess) return e;
     const size_t fixed = (size_t)3 * ns * kJTile * 8 + (size_t)kJMaxWarps * kJTile * 8;
     const size_t per_warp = (size_t)(ns + 1) * kJTile * 8;
-    if (fixed + 2 * per_warp > prop.sharedMemPerBlockOptin) return cudaErrorNotSupported;
-    const int warps = (int)std::min<size_t>(kJMaxWarps, (prop.sharedMemPerBlockOptin - fixed) / per_warp);
+    if (fixed + 2 * per_warp > dev.smem_block) return cudaErrorNotSupported;
+    const int warps = (int)std::min<size_t>(kJMaxWarps, (dev.smem_block - fixed) / per_warp);
     const int32_t* rp = (const int32_t*)v.a[CG_RPTR];
     const int32_t* pp = (const int32_t*)v.a[CG_PPTR];
     const int32_t* rsp = (const int32_t*)v.a[CG_RSP];
@@ -415,7 +415,7 @@ cudaError_t jac_prepare(const DevMech& m, const cg_mech_view& v, int device, Jac
     JacPlan* p = new JacPlan();
     p->warps = warps;
     p->smem = fixed + (size_t)warps * per_warp;
-    p->grid = prop.multiProcessorCount;
+    p->grid = dev.sms;
     e = cudaMalloc(&p->dbuf, b_ptr + b_rx + b_nu + b_row);
     char* d = (char*)p->dbuf;
     if (e == cudaSuccess) e = cudaMemcpy(d, lptr.data(), lptr.size() * sizeof(int), cudaMemcpyHostToDevice);

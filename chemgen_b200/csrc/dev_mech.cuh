@@ -8,11 +8,27 @@
 // the same time, so each load is one broadcast transaction served from L1).
 #pragma once
 
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
 #include "../../include/chemgen_mech.h"
 
 namespace cg {
+
+// What the plans need to know of a device.  Attribute by attribute:
+// cudaGetDeviceProperties takes 2 ms a call, and a handle makes nine plans.
+struct DeviceLimits {
+    int sms = 0, smem_block = 0, smem_sm = 0, regs_sm = 0, threads_sm = 0;
+};
+inline cudaError_t device_limits(int device, DeviceLimits* d) {
+    cudaError_t e = cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&d->smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&d->smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&d->regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&d->threads_sm, cudaDevAttrMaxThreadsPerMultiProcessor, device);
+    return e;
+}
 
 // chemgen/chemistry.py:204-206
 constexpr double kRc = 1.9872155832;

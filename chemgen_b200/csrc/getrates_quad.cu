@@ -453,10 +453,10 @@ cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     HostQuads h;
     build_quads(v, h);
     if (mixed && (!h.mixed_ok || 4 * h.nquad >= 0x1fff)) return cudaErrorNotSupported;
-    cudaDeviceProp prop;
-    cudaError_t e = cudaGetDeviceProperties(&prop, device);
+    DeviceLimits dev;
+    cudaError_t e = device_limits(device, &dev);
     if (e != cudaSuccess) return e;
-    const size_t limit = prop.sharedMemPerBlockOptin, per_sm = prop.sharedMemPerMultiprocessor;
+    const size_t limit = dev.smem_block, per_sm = dev.smem_sm;
     QuadPlan pl;
     pl.mixed = mixed;
     pl.nquad = h.nquad;
@@ -481,7 +481,7 @@ cudaError_t quad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     pl.warps = latency || fit < 2 ? 32 : fit <= 3 ? 16 : 8;
     pl.smem = bytes(pl.rows, pl.nchunk, pl.warps);
     const int resident = std::max(1, std::min((int)(per_sm / (pl.smem + 1024)), 32 / pl.warps));
-    pl.grid = prop.multiProcessorCount * resident;
+    pl.grid = dev.sms * resident;
     // per-species lists of (row, net coefficient), in sorted-reaction order
     std::vector<int> qbeg(pl.nchunk + 1);
     for (int c = 0; c <= pl.nchunk; ++c) qbeg[c] = std::min(h.nquad, c * qpc);

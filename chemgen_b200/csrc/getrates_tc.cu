@@ -1222,10 +1222,10 @@ cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, M
     const size_t rows = (size_t)ns + 1;                       // + the dummy row of TcFast
     const size_t base = 6 * (size_t)kABytes + 2 * (size_t)npad * 32 + rows * kTile * 4 + 4 * kTile * 8 + 32;
     const size_t with_g = base + rows * kTile * 8;
-    cudaDeviceProp prop;
-    cudaError_t e = cudaGetDeviceProperties(&prop, device);
+    DeviceLimits dev;
+    cudaError_t e = device_limits(device, &dev);
     if (e != cudaSuccess) return e;
-    const size_t limit = prop.sharedMemPerBlockOptin;
+    const size_t limit = dev.smem_block;
     if (base > limit) return cudaErrorNotSupported;
     MixedPlan* p = new MixedPlan();
     p->ns = ns;
@@ -1243,7 +1243,7 @@ cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, M
     p->group = npad <= 128 ? 4 : nchunk;
     p->smem = p->g_smem ? with_g : base;
     // resident CTAs per SM, limited by shared memory and by 512 TMEM columns
-    int per_sm = (int)(prop.sharedMemPerMultiprocessor / (p->smem + 1024));
+    int per_sm = (int)(dev.smem_sm / (p->smem + 1024));
     per_sm = std::min(per_sm, (int)(512 / tcols));
     per_sm = std::max(per_sm, 1);
     // threads per point: the most (4, 2, 1) whose registers still let per_sm
@@ -1252,19 +1252,19 @@ cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, M
     for (int nt : {4, 2}) {
         cudaFuncAttributes fa;
         if (cudaFuncGetAttributes(&fa, kernel_for(p->g_smem, nt)) != cudaSuccess) continue;
-        if ((long)per_sm * kTile * nt * fa.numRegs <= prop.regsPerMultiprocessor &&
-            per_sm * kTile * nt <= prop.maxThreadsPerMultiProcessor) {
+        if ((long)per_sm * kTile * nt * fa.numRegs <= dev.regs_sm &&
+            per_sm * kTile * nt <= dev.threads_sm) {
             p->nt = nt;
             break;
         }
     }
-    p->grid = prop.multiProcessorCount * per_sm;
+    p->grid = dev.sms * per_sm;
     // the 32-point kernel whenever its tile's state fits
     const size_t t32 = 12 * (size_t)kA32 + 4 * (size_t)npad * 32 + rows * kTP * 12 + kTWarps * kTP * 8 + sizeof(Tile32) + 64;
     if (t32 <= limit) {
         p->t32 = 1;
         p->smem32 = t32;
-        p->grid32 = prop.multiProcessorCount;
+        p->grid32 = dev.sms;
     }
     // nu chunks in the canonical K-major layout: B[n][k] = nu of species n in reaction 16*chunk + k
     std::vector<float> nuf((size_t)ns * nr, 0.0f);

@@ -211,3 +211,18 @@ def test_transposed_copies(rows, cols):
     out = torch.empty(cols, rows, dtype=torch.float64, device="cuda")
     assert transposed(x, out) is out and torch.equal(out, x.t())
     assert torch.equal(transposed(x[:, ::2]), x[:, ::2].t())
+
+
+def test_a_handle_is_made_in_a_few_milliseconds():
+    # plans and tables of 348/2158; querying every property of the device for each
+    # plan took 23 ms in all, the plans themselves take 7
+    import time
+    from conftest import load_golden
+    blob = pack.pack(load_golden("jetsurf2")[0]).to_blob()
+    t = []
+    for _ in range(6):
+        t0 = time.perf_counter()
+        gm = GpuMechanism(blob)
+        t.append(time.perf_counter() - t0)
+        gm.close()
+    assert min(t[1:]) < 12e-3, t
