@@ -437,9 +437,10 @@ static QuadKernel quad_kernel(int warps, int mixed) {
     }
 }
 
-// Species beyond which the FP64 call keeps its caller-visible workspace and
-// runs the global-scratch kernel.
-constexpr int kQuadMaxSpecies = 434;
+// Species up to which the FP64 call has needed no workspace from its caller
+// (what 32-point tiles of C and EGp left of shared memory); beyond, the
+// global-scratch kernel asks for one, although the tiles would fit to 511.
+constexpr int kQuadMaxSpecies = 437;
 
 int quad_tile_points() { return kQP; }
 int quad_general(const QuadPlan* p) { return p->general; }

@@ -36,6 +36,27 @@ def test_several_chunks_of_reactions():
     _check(synthetic.synthetic_mechanism(120, 4200, 40, 60, seed=9), 41)
 
 
+@pytest.mark.parametrize("ns", [434, 435, 437, 438])
+def test_the_largest_mechanisms_without_a_workspace(ns):
+    # up to 437 species the FP64 call needs no workspace and the counted call works
+    import torch
+    from chemgen_b200.runtime import lib
+    mech = synthetic.synthetic_mechanism(ns, 500, 20, 20, seed=1)
+    blob = pack.pack(mech).to_blob()
+    gm = GpuMechanism(blob)
+    ng = 21
+    P, T, Y = synthetic.states(mech.ns, ng, seed=2)
+    Pt, Tt, Yt = _cuda(P, T, Y)
+    W, count = torch.zeros_like(Yt), torch.tensor([ng], device="cuda")
+    st = lib().chemgen_getrates_counted(gm._h, Pt.data_ptr(), Tt.data_ptr(), ng, Yt.data_ptr(), W.data_ptr(),
+                                        count.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert (gm.workspace_bytes(ng) == 0, st) == ((True, 0) if ns <= 437 else (False, 6))
+    r = oracle.rates(blob, P, T, Y, mech.nr)
+    for w in [gm.getrates(Pt, Tt, Yt)] + ([W] if st == 0 else []):
+        e = oracle.errors(w.cpu().numpy(), r["wdot"], r["S"])
+        assert e["norm_max"] <= TOL_FP64, e
+
+
 def test_every_kind_and_general_stoichiometry():
     # PLOG, SRI, Lindemann; a negative and a zero pre-exponential factor,
     # fractional coefficients and four molecules on a side take the generic path
