@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
     // those below min(*count, n1)
     const int64_t npts = count ? min(n1, (int64_t)*count) : n1;
     if (threadIdx.x < 16) sTab[threadIdx.x] = kQExpTab[threadIdx.x];
-    if (warp == W - 1 && g == 0) quad_head(sH, i0 + (int64_t)blockIdx.x * kQP + p, npts, P, Tg);
+    if (warp == W - 1 && g == 0) quad_head<MIXED>(sH, i0 + (int64_t)blockIdx.x * kQP + p, npts, P, Tg);
     if (threadIdx.x < kQP) {
         sQ[v.rows * kQP + p] = 0.0;                        // the zero row of the lists
         if (MIXED) sCE[ns * kQP + p] = make_double2(0.0, __hiloint2double(0, __float_as_int(1.0f)));
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
                 }
             }
             if (c == 0 && warp == W - 1 && g == 0 && t0 + step < npts)
-                quad_head(sH + (buf ^ 1) * 4 * kQP, t0 + step + p, npts, P, Tg);
+                quad_head<MIXED>(sH + (buf ^ 1) * 4 * kQP, t0 + step + p, npts, P, Tg);
             __syncthreads();
             const bool last = c == v.nchunk - 1;
             if (warp < v.nsq) {

@@ -1087,7 +1087,7 @@ __global__ void __launch_bounds__(32 * (kTWarps + 1), 1)
             const int64_t i = tile * kTP + lane;
             const bool act = i < ng;
             const double T = act ? __ldcs(Tg + i) : 1000.0, Pv = act ? __ldcs(P + i) : kPatm;
-            const double lnT = cgm::cg_log(T), invT = fmin(1.0 / T, kQMaxInvT), lnT2 = lnT * kLog2eD;
+            const double lnT = cgm::cg_log(T), invT = 1.0 / T, lnT2 = lnT * kLog2eD;
             um::bar_sync(1, 32 * kTWarps);                      // the last tile's rates are done
             double part = 0.0;
 #pragma unroll 8

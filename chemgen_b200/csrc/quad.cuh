@@ -46,10 +46,13 @@ constexpr int kQKindGeneric = 6;       // reactions evaluated from their DRxn re
 // exact, and its low word is zero, as are those of the coefficients 1/5! ..
 // 1/7!, rounded to 21 bits where their rounding stays below 2^-57 of the
 // result: such constants are immediates of the FP64 instruction) and a tail.
-// Largest error 1.7 ulp over [-700, 700].  |x| < 9e7 (16 x / ln 2 in 32 bits): the
-// exponent saturates to 0 or +inf as cg_exp's does, so x needs no clamp; the
-// quad kernels keep 1/T <= 5 and evaluate reactions with Ea/Rc > 1.5e7 K
-// elsewhere for that.
+// Largest error 1.7 ulp over [-700, 700].  The exponent is taken from bits
+// 4..35 of the rounded 16 x / ln 2 and saturates to 0 or +inf as cg_exp's does,
+// so no x with |x| < 1.4e9 needs a clamp.  For that the FP64 kernels keep 1/T <=
+// 700 and evaluate reactions with Ea/Rc > 1e6 K elsewhere: a difference of two
+// exponents (falloff's ln k0 - ln kinf) then reaches it too.  Down to T = 1/700
+// K nothing is clamped; below, the clamp changes only rates with Ea/Rc < 1 K,
+// all others being 0 or +inf already.
 struct QExp {
     double l16, lo, c4, c3;
 };
@@ -59,14 +62,14 @@ static __constant__ double kQExpTab[16] = {
     1.0, 1.0442737824274138, 1.0905077326652577, 1.1387886347566916, 1.189207115002721, 1.241857812073484,
     1.2968395546510096, 1.3542555469368927, 1.4142135623730951, 1.4768261459394993, 1.5422108254079407,
     1.6104903319492543, 1.681792830507429, 1.7562521603732995, 1.8340080864093424, 1.9152065613971474};
-constexpr double kQMaxInvT = 5.0, kQMaxTheta = 1.5e7, kQMinArg = -9e7;
+constexpr double kQMaxInvT = 700.0, kQMaxTheta = 1e6, kQMinArg = -9e7;
 
 __device__ __forceinline__ double q_exp(double x, const double* tab) {
     const double t = fma(x, kQExp.l16, cgm::kRound);
     const double k = t - cgm::kRound;
     double r = fma(k, -0.04332166910171509, x);
     r = fma(k, kQExp.lo, r);
-    const int n = __double2loint(t);
+    const int n = __double2loint(t), k2 = (int)__funnelshift_r(n, __double2hiint(t), 4);   // floor(16 x / ln 2 / 16)
     double p = fma(0.00019841268658638, r, 0.00138888880610466);
     p = fma(p, r, 0.00833333283662796);
     p = fma(p, r, kQExp.c4);
@@ -74,7 +77,7 @@ __device__ __forceinline__ double q_exp(double x, const double* tab) {
     p = fma(p, r, 0.5);
     p = fma(p, r, 1.0);
     const double b = tab[n & 15];
-    const int e = max(0, min((n >> 4) + 1023, 2047));
+    const int e = max(0, min(k2 + 1023, 2047));
     return fma(b, p * r, b) * __hiloint2double(e << 20, 0);
 }
 
@@ -273,13 +276,15 @@ __device__ __forceinline__ double quad_falloff(int kind, const QRec& R, const QF
 
 // A tile's T, ln T, 1/T and P, [4][8] in shared memory.  One warp forms the
 // next tile's while the others evaluate reactions: ln T in every warp was a
-// tenth of a 53-species tile's instructions.
+// tenth of a 53-species tile's instructions.  The mixed form has no q_exp and
+// takes 1/T as it is, like the generated kernel.
+template <bool MIXED = false>
 __device__ __forceinline__ void quad_head(double* h, int64_t i, int64_t n, const double* P, const double* Tg) {
     const int p = threadIdx.x & (kQP - 1);
     const double T = i < n ? __ldcs(Tg + i) : 1000.0;
     h[p] = T;
     h[kQP + p] = cgm::cg_log(T);
-    h[2 * kQP + p] = fmin(cgm::cg_rcp(T), kQMaxInvT);
+    h[2 * kQP + p] = MIXED ? cgm::cg_rcp(T) : fmin(cgm::cg_rcp(T), kQMaxInvT);
     h[3 * kQP + p] = i < n ? __ldcs(P + i) : kPatm;
 }
 

@@ -72,6 +72,62 @@ def test_every_kind_and_general_stoichiometry():
     _check(mech, 83)
 
 
+def _cold(seed=7):
+    # irreversible reactions of small activation energy, which stay finite near
+    # 0 K, and states down to 2 mK
+    import dataclasses
+    mech = synthetic.synthetic_mechanism(6, 12, 0, 0, seed=seed, frac_reversible=0.0)
+    theta = [0.0, 0.01, 0.02, 0.1, 0.5, 2.0, -0.05, 8.0, 0.0, 30.0, 0.03, 1.0]
+    mech.reactions = [dataclasses.replace(r, arh=(1e3, 0.0 if i % 2 else 0.7, theta[i] * 1.9872155832))
+                      for i, r in enumerate(mech.reactions)]
+    P, T, Y = synthetic.states(6, 13, seed=seed)
+    T[:] = [0.002, 0.003, 0.01, 0.02, 0.05, 0.1, 0.19, 0.2, 0.21, 0.5, 3.0, 40.0, 300.0]
+    return mech, P, T, Y
+
+
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+def test_temperatures_near_zero(mode):
+    # 1/T up to 500 per K reaches the rates unchanged: FP64 tiles (through the
+    # counted call) and 32-point mixed tiles
+    import torch
+    from chemgen_b200.runtime import lib
+    mech, P, T, Y = _cold()
+    blob = pack.pack(mech).to_blob()
+    gm = GpuMechanism(blob)
+    Pt, Tt, Yt = _cuda(P, T, Y)
+    if mode == "fp64":
+        W, count = torch.zeros_like(Yt), torch.tensor([len(T)], device="cuda")
+        assert lib().chemgen_getrates_counted(gm._h, Pt.data_ptr(), Tt.data_ptr(), len(T), Yt.data_ptr(), W.data_ptr(),
+                                              count.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    else:
+        W = gm.getrates(Pt, Tt, Yt, mode=mode)
+    r = oracle.rates(blob, P, T, Y, mech.nr)
+    assert np.isfinite(r["wdot"]).all()
+    assert oracle.errors(W.cpu().numpy(), r["wdot"], r["S"])["norm_max"] <= (TOL_FP64 if mode == "fp64" else 1e-6)
+
+
+def test_derivatives_at_temperatures_near_zero():
+    # dq/dT = q (b + theta / T - n) / T for n reactant molecules, at constant Y and P
+    mech, P, T, Y = _cold()
+    gm = GpuMechanism(mech)
+    Pt, Tt, Yt = _cuda(P, T, Y)
+    J = gm.jacobian(Pt, Tt, Yt).cpu().numpy()
+    C = Y / np.array([s.mw for s in mech.species])[:, None]
+    C *= P / (8.314510e+07 * T * C.sum(0))
+    ref = np.zeros_like(Y)
+    for r in mech.reactions:
+        A, b, Ea = r.arh
+        th = Ea / 1.9872155832
+        q = A * T ** b * np.exp(-th / T)
+        for s, nu in r.reactants.items():
+            q = q * C[mech.species_names.index(s)] ** nu
+        d = q * (b + th / T - sum(r.reactants.values())) / T
+        for side, sign in ((r.reactants, -1.0), (r.products, 1.0)):
+            for s, nu in side.items():
+                ref[mech.species_names.index(s)] += sign * nu * d
+    assert (np.abs(J[:, 0] - ref).max(0) / np.abs(ref).max(0)).max() <= 1e-9
+
+
 def _derivatives(mech, ng, seed=0, states=None):
     """(Jacobian, adjoint) of the kernels and of autograd through the FP64 law."""
     import torch
