@@ -123,15 +123,16 @@ struct AdjSums {
     double t = 0.0, a = 0.0, rho = 0.0, p = 0.0;
 };
 
-// Falloff: forward rate constant kf, d ln kf/dT at fixed M, and gpr =
-// d ln kf / d ln M (falloff_d's formulas).
+// Falloff: forward rate constant kf = kfm M, d ln kf/dT at fixed M, and gpr =
+// d ln kf / d ln M (falloff_d's formulas).  kfm and not kf, so that nothing
+// divides by M, which is zero where no collider is present.
 __device__ __forceinline__ void quad_falloff_d(int kind, const QRec& R, const QFall* fall, double M, const PointT& pt,
-                                               const double* tab, double& kf, double& dlkf, double& gpr) {
+                                               const double* tab, double& kfm, double& dlkf, double& gpr) {
     const double2* q = reinterpret_cast<const double2*>(fall + R.aux);
     const double2 f0 = __ldg(q), f1 = __ldg(q + 1), f2 = __ldg(q + 2), f3 = __ldg(q + 3);
     const double lkinf = fma(R.b, pt.lnT, R.lnA) - R.th * pt.invT;
     const double lr = (fma(f0.y, pt.lnT, f0.x) - f1.x * pt.invT) - lkinf;
-    const double Pr = q_exp(lr, tab) * M;
+    const double k0r = q_exp(lr, tab), Pr = k0r * M;   // k0 / kinf
     const double dlkinf = fma(R.th, pt.invT, R.b) * pt.invT;
     const double dlPr = fma(f1.x, pt.invT, f0.y) * pt.invT - dlkinf;
     const double ipr = q_rcp(1.0 + Pr);
@@ -172,15 +173,15 @@ __device__ __forceinline__ void quad_falloff_d(int kind, const QRec& R, const QF
         gpr = ipr - 2.0 * lp * X * X * lb * kIln10;
         dlF_T = fma(X, dbase * q_rcp(base), f3.y * pt.invT);
     }
-    kf = cgm::cg_exp_clamped(lkinf + lnF) * (Pr * ipr);
+    kfm = cgm::cg_exp_clamped(lkinf + lnF) * (k0r * ipr);
     dlkf = fma(gpr, dlPr, dlkinf) + dlF_T;
 }
 
-// The rows of one reaction with q = mul (qf - qb): mul is M for a three-body
-// reaction, otherwise 1.  scale: dq/dM = scale (qf - qb) (M itself is no
-// divisor here: it is zero where a species without efficiency stands alone),
-// add: the reaction's share of s = add (qf - qb) beside the molecules' (ord
-// counts M of a three-body reaction).
+// The rows of one reaction with q = mul (qf - qb): mul is M for a three-body or
+// falloff reaction (kf then lacks that factor), otherwise 1.  scale: dq/dM =
+// scale (qf - qb) (M itself is no divisor: it is zero where a species without
+// efficiency stands alone), add: the reaction's share of s = add mul (qf - qb)
+// beside the molecules' (ord counts M of a three-body reaction).
 template <bool ADJ, bool WIDE, bool REV>
 __device__ __forceinline__ void grad_rows(const GradCtx& c, const QRec& R, double kf, double dlkf, bool usesM,
                                           double mul, double scale, double add, double* out, AdjSums& sum) {
@@ -352,20 +353,19 @@ __device__ __forceinline__ void grad_run(const DevMech& m, const GradView& v, co
         }
         const QRec R = load_qrec(rec);
         const double M = quad_m(v.eff, __ldg(v.efl + q), c.g, c.ctot, c.ce);
-        double kf, dlkf, mul = 1.0, scale = 1.0, add = 0.0;
+        double kf, dlkf, scale = 1.0, add = 0.0;
         if (kind == CG_THIRD_BODY) {
             kf = q_exp(fma(R.b, c.pt.lnT, R.lnA) - R.th * c.pt.invT, c.tab);
             dlkf = fma(R.th, c.pt.invT, R.b) * c.pt.invT;
-            mul = M;
         } else {
             quad_falloff_d(kind, R, v.fall, M, c.pt, c.tab, kf, dlkf, add);
-            scale = add * cgm::cg_rcp(M);
+            scale = add;
         }
         switch (cls & (kQWide | kQRev)) {
-            case 0: grad_rows<ADJ, false, false>(c, R, kf, dlkf, true, mul, scale, add, out, sum); break;
-            case kQRev: grad_rows<ADJ, false, true>(c, R, kf, dlkf, true, mul, scale, add, out, sum); break;
-            case kQWide: grad_rows<ADJ, true, false>(c, R, kf, dlkf, true, mul, scale, add, out, sum); break;
-            default: grad_rows<ADJ, true, true>(c, R, kf, dlkf, true, mul, scale, add, out, sum); break;
+            case 0: grad_rows<ADJ, false, false>(c, R, kf, dlkf, true, M, scale, add, out, sum); break;
+            case kQRev: grad_rows<ADJ, false, true>(c, R, kf, dlkf, true, M, scale, add, out, sum); break;
+            case kQWide: grad_rows<ADJ, true, false>(c, R, kf, dlkf, true, M, scale, add, out, sum); break;
+            default: grad_rows<ADJ, true, true>(c, R, kf, dlkf, true, M, scale, add, out, sum); break;
         }
     }
 }

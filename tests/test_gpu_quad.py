@@ -182,6 +182,23 @@ def test_derivatives_where_a_third_body_is_zero():
     assert _rel(v[1], r[1]) <= 1e-9
 
 
+def test_derivatives_where_a_falloff_has_no_collider():
+    # M = 0 of Lindemann reactions: the rate is zero, its derivative by M is
+    # k0 (prod C - prod C / Kc), and nothing divides by M.  Against autograd
+    mech = synthetic.synthetic_mechanism(10, 24, 0, 0, seed=5, n_lindemann=10)
+    for r in mech.reactions:
+        if r.kind == "lindemann":
+            r.efficiencies = {**r.efficiencies, "S3": -1.0}
+            r.reactants, r.products, r.reversible = {"S3": 2.0}, {"S1": 1.0, "S3": 1.0}, False
+    P, T, Y = synthetic.states(mech.ns, 9, seed=1)
+    Y[:] = 0.0
+    Y[3] = 1.0
+    (J64, J32, v), (J, r) = _derivatives(mech, 9, states=(P, T, Y))
+    assert bool((J[1].abs().amax(0) > 0).all())
+    assert _rel(J64, J) <= 1e-9 and _rel(J32, J) <= 1e-6
+    assert _rel(v[1], r[1]) <= 1e-9
+
+
 @pytest.mark.parametrize("mode", ["fp64", "mixed"])
 @pytest.mark.parametrize("name", ["gri30", "h2_burke", "synthetic_53_325", "all_kinds"])
 def test_small_batches_and_remainders_equal_the_generated_kernel(name, mode):
