@@ -59,7 +59,7 @@ struct __align__(16) JZero {
 static_assert(sizeof(JZero) == 16, "JZero must stay 16 bytes");
 
 struct GradPlan {
-    int adjoint = 0;
+    int adjoint = 0, other = 0;        // other: PLOG reactions, or some without a pre-decoded form
     int nchunk = 0, rows = 0, warps = 0, nown = 0, nrow = 0, nzero = 0;
     size_t smem = 0;
     int grid = 0;
@@ -181,10 +181,12 @@ __device__ __forceinline__ void quad_falloff_d(int kind, const QRec& R, const QF
 // falloff reaction (kf then lacks that factor), otherwise 1.  scale: dq/dM =
 // scale (qf - qb) (M itself is no divisor: it is zero where a species without
 // efficiency stands alone), add: the reaction's share of s = add mul (qf - qb)
-// beside the molecules' (ord counts M of a three-body reaction).
+// beside the molecules' (ord counts M of a three-body reaction).  plog: kf
+// depends on P, dlnp = d ln kf / d ln P.
 template <bool ADJ, bool WIDE, bool REV>
 __device__ __forceinline__ void grad_rows(const GradCtx& c, const QRec& R, double kf, double dlkf, bool usesM,
-                                          double mul, double scale, double add, double* out, AdjSums& sum) {
+                                          double mul, double scale, double add, double* out, AdjSums& sum,
+                                          bool plog = false, double dlnp = 0.0) {
     constexpr int N = WIDE ? 3 : 2;
     unsigned so[3] = {R.s[0], R.s[1], R.s2}, po[3] = {R.p[0], R.p[1], R.p2};
     double x[N], d[N];
@@ -246,6 +248,7 @@ __device__ __forceinline__ void grad_rows(const GradCtx& c, const QRec& R, doubl
     if (ADJ) {
         sum.t = fma(gq, dT, sum.t);
         sum.rho = fma(gq, s, sum.rho);
+        if (plog) sum.p = fma(gq, net * dlnp / c.P, sum.p);
         if (usesM) {
             const double gm = gq * m;
             sum.a += gm;
@@ -258,10 +261,41 @@ __device__ __forceinline__ void grad_rows(const GradCtx& c, const QRec& R, doubl
     }
 }
 
-// A reaction evaluated from its DRxn record: its rows in the same order.
+// grad_rows of the class cls.
 template <bool ADJ>
-__device__ __noinline__ AdjSums grad_rows_generic(const DevMech& m, GradCtx c, unsigned r, double* out) {
+__device__ __forceinline__ void grad_rows_of(int cls, const GradCtx& c, const QRec& R, double kf, double dlkf,
+                                             bool usesM, double mul, double scale, double add, double* out,
+                                             AdjSums& sum, bool plog = false, double dlnp = 0.0) {
+    switch (cls & (kQWide | kQRev)) {
+        case 0: grad_rows<ADJ, false, false>(c, R, kf, dlkf, usesM, mul, scale, add, out, sum, plog, dlnp); break;
+        case kQRev: grad_rows<ADJ, false, true>(c, R, kf, dlkf, usesM, mul, scale, add, out, sum, plog, dlnp); break;
+        case kQWide: grad_rows<ADJ, true, false>(c, R, kf, dlkf, usesM, mul, scale, add, out, sum, plog, dlnp); break;
+        default: grad_rows<ADJ, true, true>(c, R, kf, dlkf, usesM, mul, scale, add, out, sum, plog, dlnp); break;
+    }
+}
+
+// PLOG: {kf, d ln kf/dT, d ln kf/d ln P}.  Evaluated like the reactions below,
+// its arrays in local memory, 8 of 40 took a 15-species adjoint to 430 us for
+// 100003 points, now 219 (321 with the 32-point tiles before).
+__device__ __noinline__ double3 quad_plog_d(const DevMech& m, int row, double P, double lnP, PointT pt) {
+    double3 k;
+    plog_d(m, row, P, lnP, pt, k.x, k.y, k.z);
+    return k;
+}
+
+// A reaction evaluated from its DRxn record: its rows in the same order.  With
+// PLOG those too, from their pre-decoded records.
+template <bool ADJ, bool PLOG>
+__device__ __noinline__ AdjSums grad_rows_generic(const DevMech& m, GradCtx c, int cls, const QRec* rec, double* out) {
     AdjSums sum;
+    if (PLOG && (cls & 15) == CG_PLOG) {
+        const QRec R = load_qrec(rec);
+        double kf, dlkf, dlnp;
+        plog_d(m, (int)R.aux, c.P, c.lnP, c.pt, kf, dlkf, dlnp);
+        grad_rows_of<ADJ>(cls, c, R, kf, dlkf, false, 1.0, 0.0, 0.0, out, sum, true, dlnp);
+        return sum;
+    }
+    const unsigned r = __ldg(&rec->r);
     if (r == kQNone) return sum;
     const double* s0 = reinterpret_cast<const double*>(c.ce);
     const double* d0 = c.dg;
@@ -325,7 +359,12 @@ __device__ __forceinline__ void grad_standard(const GradCtx& c, const QRec* rec,
     }
 }
 
-template <int W, bool ADJ>
+// OTHER: the mechanism has PLOG reactions or some without a pre-decoded form.
+// Instances of their own for those, because what the call needs beside the loops
+// spills: without it 53/325 takes 325 instead of 351 us for the rates and adjoint
+// of 32768 points, 1118 instead of 1155 for the Jacobian of 65536.  (In 32 warps,
+// with 64 registers, PLOG goes out of line as a whole: in line it took 1.5 % more.)
+template <int W, bool ADJ, bool OTHER>
 __device__ __forceinline__ void grad_run(const DevMech& m, const GradView& v, const GradCtx& c, int cls, int q, int n,
                                          AdjSums& sum) {
     const int kind = cls & 15;
@@ -341,8 +380,8 @@ __device__ __forceinline__ void grad_run(const DevMech& m, const GradView& v, co
     }
     for (; n > 0; --n, q += W, rec += kQG * W) {
         double* out = c.out + __ldg(v.qrow + q) * kQP;
-        if (kind == kQKindGeneric) {
-            const AdjSums x = grad_rows_generic<ADJ>(m, c, __ldg(&rec->r), out);
+        if (OTHER && (W == 32 ? kind >= CG_PLOG : kind == kQKindGeneric)) {
+            const AdjSums x = grad_rows_generic<ADJ, W == 32>(m, c, cls, rec, out);
             if (ADJ) {
                 sum.t += x.t;
                 sum.a += x.a;
@@ -352,6 +391,11 @@ __device__ __forceinline__ void grad_run(const DevMech& m, const GradView& v, co
             continue;
         }
         const QRec R = load_qrec(rec);
+        if (OTHER && W < 32 && kind == CG_PLOG) {
+            const double3 k = quad_plog_d(m, (int)R.aux, c.P, c.lnP, c.pt);
+            grad_rows_of<ADJ>(cls, c, R, k.x, k.y, false, 1.0, 0.0, 0.0, out, sum, true, k.z);
+            continue;
+        }
         const double M = quad_m(v.eff, __ldg(v.efl + q), c.g, c.ctot, c.ce);
         double kf, dlkf, scale = 1.0, add = 0.0;
         if (kind == CG_THIRD_BODY) {
@@ -361,17 +405,12 @@ __device__ __forceinline__ void grad_run(const DevMech& m, const GradView& v, co
             quad_falloff_d(kind, R, v.fall, M, c.pt, c.tab, kf, dlkf, add);
             scale = add;
         }
-        switch (cls & (kQWide | kQRev)) {
-            case 0: grad_rows<ADJ, false, false>(c, R, kf, dlkf, true, M, scale, add, out, sum); break;
-            case kQRev: grad_rows<ADJ, false, true>(c, R, kf, dlkf, true, M, scale, add, out, sum); break;
-            case kQWide: grad_rows<ADJ, true, false>(c, R, kf, dlkf, true, M, scale, add, out, sum); break;
-            default: grad_rows<ADJ, true, true>(c, R, kf, dlkf, true, M, scale, add, out, sum); break;
-        }
+        grad_rows_of<ADJ>(cls, c, R, kf, dlkf, true, M, scale, add, out, sum);
     }
 }
 
 // The rows of a chunk's reactions.
-template <int W, bool ADJ>
+template <int W, bool ADJ, bool OTHER>
 __device__ __forceinline__ void grad_chunk(const DevMech& m, const GradView& v, const GradCtx& c, int chunk, int warp,
                                            AdjSums& sum) {
     const int* rb = v.rbeg + chunk * W + warp;
@@ -379,7 +418,7 @@ __device__ __forceinline__ void grad_chunk(const DevMech& m, const GradView& v, 
     for (int r = __ldg(rb); r < r1; ++r) {
         const int4 rn = __ldg(v.run + r);
         const int cls = __shfl_sync(0xffffffffu, rn.x, 0), n = __shfl_sync(0xffffffffu, rn.z, 0);
-        grad_run<W, ADJ>(m, v, c, cls, rn.y, n, sum);
+        grad_run<W, ADJ, OTHER>(m, v, c, cls, rn.y, n, sum);
     }
 }
 
@@ -488,7 +527,7 @@ __device__ __forceinline__ void jac_entries(const JEnt* e, int n, const double* 
 }
 
 // ---------------------------------------------------------------- Jacobian
-template <int W, int MINB, typename JT>
+template <int W, int MINB, bool OTHER, typename JT>
 __global__ void __launch_bounds__(32 * W, MINB)
     jacobian_quad(const __grid_constant__ DevMech m, const __grid_constant__ GradView v, const double* __restrict__ P,
                   const double* __restrict__ Tg, const double* __restrict__ Y, JT* __restrict__ J, int64_t ng) {
@@ -524,7 +563,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
         const bool act = i < ng;
         grad_state<W, false>(m, v, c, act, i, ng, sH + buf * 4 * kQP, Y, nullptr, warp, p, sCE, sDG, sRed);
         AdjSums none;
-        grad_chunk<W, false>(m, v, c, 0, warp, none);
+        grad_chunk<W, false, OTHER>(m, v, c, 0, warp, none);
         if (warp == W - 1 && g == 0 && t0 + stride < ng) quad_head(sH + (buf ^ 1) * 4 * kQP, i + stride, ng, P, Tg);
         __syncthreads();
         for_owners<W>(v.rlists, v.nrow, 0, warp, g, [&](const QOwn& o) {
@@ -580,7 +619,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
 }
 
 // ----------------------------------------------------------------- adjoint
-template <int W, int MINB>
+template <int W, int MINB, bool OTHER>
 __global__ void __launch_bounds__(32 * W, MINB)
     vjp_quad(const __grid_constant__ DevMech m, const __grid_constant__ GradView v, const double* __restrict__ P,
              const double* __restrict__ Tg, const double* __restrict__ Y, const double* __restrict__ G,
@@ -619,7 +658,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
             grad_state<W, true>(m, v, c, act, i, ng, sH + buf * 4 * kQP, Y, G, warp, p, sCE, sDG, sRed);
         AdjSums sum;
         for (int ch = 0; ch < v.nchunk; ++ch) {
-            grad_chunk<W, true>(m, v, c, ch, warp, sum);
+            grad_chunk<W, true, OTHER>(m, v, c, ch, warp, sum);
             if (ch == 0 && warp == W - 1 && g == 0 && t0 + stride < ng)
                 quad_head(sH + (buf ^ 1) * 4 * kQP, i + stride, ng, P, Tg);
             const bool last = ch == v.nchunk - 1;
@@ -660,18 +699,25 @@ __global__ void __launch_bounds__(32 * W, MINB)
     }
 }
 
+template <bool OTHER>
 const void* grad_kernel(const GradPlan* p, int precision) {
     if (p->adjoint)
-        return p->warps == 8 ? (const void*)vjp_quad<8, 3>
-                             : p->warps == 12 ? (const void*)vjp_quad<12, 2> : (const void*)vjp_quad<24, 1>;
-    if (p->warps == 32) return (const void*)jacobian_quad<32, 1, float>;
+        return p->warps == 8 ? (const void*)vjp_quad<8, 3, OTHER>
+                             : p->warps == 12 ? (const void*)vjp_quad<12, 2, OTHER> : (const void*)vjp_quad<24, 1, OTHER>;
+    // (64 registers: the instance without the call took 104.5 instead of 102.4 us for
+    // GRI30, 5003 points)
+    if (p->warps == 32) return (const void*)jacobian_quad<32, 1, true, float>;
     if (precision == 0)
-        return p->warps == 8 ? (const void*)jacobian_quad<8, 3, double>
-                             : p->warps == 12 ? (const void*)jacobian_quad<12, 2, double>
-                                              : (const void*)jacobian_quad<24, 1, double>;
-    return p->warps == 8 ? (const void*)jacobian_quad<8, 3, float>
-                         : p->warps == 12 ? (const void*)jacobian_quad<12, 2, float>
-                                          : (const void*)jacobian_quad<24, 1, float>;
+        return p->warps == 8 ? (const void*)jacobian_quad<8, 3, OTHER, double>
+                             : p->warps == 12 ? (const void*)jacobian_quad<12, 2, OTHER, double>
+                                              : (const void*)jacobian_quad<24, 1, OTHER, double>;
+    return p->warps == 8 ? (const void*)jacobian_quad<8, 3, OTHER, float>
+                         : p->warps == 12 ? (const void*)jacobian_quad<12, 2, OTHER, float>
+                                          : (const void*)jacobian_quad<24, 1, OTHER, float>;
+}
+
+const void* grad_kernel(const GradPlan* p, int precision) {
+    return p->other ? grad_kernel<true>(p, precision) : grad_kernel<false>(p, precision);
 }
 
 }  // namespace
@@ -702,7 +748,7 @@ cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     if (e != cudaSuccess) return e;
     const size_t limit = dev.smem_block, per_sm = dev.smem_sm;
     HostQuads h;
-    build_quads(v, h, adjoint != 0);
+    build_quads(v, h, adjoint != 0, true);
     auto uses_m = [&](int r) {
         return r >= m.seg[CG_THIRD_BODY] && r < m.seg[CG_PLOG];
     };
@@ -721,6 +767,7 @@ cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, in
     }
     GradPlan pl;
     pl.adjoint = adjoint;
+    pl.other = h.ngeneric + h.nplog > 0;
     auto bytes = [&](size_t rows, int chunks, int warps) {
         const size_t state = (size_t)8 + 4 * (ns + 1) + rows + 1 + (adjoint ? 4 : 1) * warps +
                              (adjoint ? (chunks > 1 ? ns : 0) : ns);

@@ -99,7 +99,7 @@ struct __align__(16) QRec {
     unsigned short s[2], p[2];         // the first two molecules of each side
     unsigned short s2, p2;             // the third ones
     unsigned int r;                    // reaction in kernel order
-    unsigned int aux;                  // falloff row; mixed: 2^f of a constant rate as FP32 bits, else 0
+    unsigned int aux;                  // falloff or PLOG row; mixed: 2^f of a constant rate as FP32 bits, else 0
     unsigned int ord;                  // molecules a side, << 0 / << 8 (M included)
 };
 static_assert(sizeof(QRec) == 48, "QRec must stay 48 bytes");
@@ -302,7 +302,7 @@ __device__ __forceinline__ double quad_total(const double* red, int g) {
 // ------------------------------------------------------------------ host
 // The reactions sorted into quads.
 struct HostQuads {
-    int ns = 0, nr = 0, nquad = 0, ngeneric = 0;
+    int ns = 0, nr = 0, nquad = 0, ngeneric = 0, nplog = 0;
     std::vector<QRec> rec, rec2;       // [4 nquad] FP64 and log2 (mixed) tables
     std::vector<int> key;              // [nquad] class
     std::vector<int2> efl;             // [nquad]
@@ -327,8 +327,9 @@ inline std::vector<double> quad_thermo_rows(const cg_mech_view& v) {
 }
 
 // `products`: a side of three products makes a reaction wide even when it is
-// irreversible (the adjoint reads every product).
-inline void build_quads(const cg_mech_view& v, HostQuads& h, bool products = false) {
+// irreversible (the adjoint reads every product).  `plog`: PLOG reactions have a
+// class of their own (else they are evaluated from their DRxn records).
+inline void build_quads(const cg_mech_view& v, HostQuads& h, bool products = false, bool plog = false) {
     const int ns = h.ns = (int)v.s[CG_S_NS], nr = h.nr = (int)v.s[CG_S_NR];
     const int32_t* flags = (const int32_t*)v.a[CG_FLAGS];
     const int32_t* rp = (const int32_t*)v.a[CG_RPTR];
@@ -363,8 +364,14 @@ inline void build_quads(const cg_mech_view& v, HostQuads& h, bool products = fal
         unsigned short mol[2][3];
         for (int j = 0; j < 6; ++j) mol[j / 3][j % 3] = (unsigned short)(ns * kQRow);
         int n[2] = {0, 0};
-        bool ok = kind != CG_PLOG && arh[3 * r] > 0.0 && (flags[r] & CG_F_INT_NU) && ns < 0x10000 / kQRow &&
-                  std::fabs(karh[4 * r + 2]) < kQMaxTheta;
+        bool ok = (flags[r] & CG_F_INT_NU) && ns < 0x10000 / kQRow;
+        if (kind == CG_PLOG) {
+            ok = ok && plog;
+            it.a.aux = (unsigned)(r - seg[CG_PLOG]);
+            ++h.nplog;
+        } else {
+            ok = ok && arh[3 * r] > 0.0 && std::fabs(karh[4 * r + 2]) < kQMaxTheta;
+        }
         if (falloff) {
             const int f = r - seg[CG_LINDEMANN];
             ok = ok && fall[8 * f] > 0.0 && std::fabs(kfall[4 * f + 2]) < kQMaxTheta;
