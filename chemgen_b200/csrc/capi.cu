@@ -35,10 +35,8 @@ struct MixedPlan;
 cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, MixedPlan** out);
 void mixed_release(MixedPlan* p);
 cudaError_t launch_getrates_mixed(const MixedPlan* p, const DevMech& m, const double* P, const double* T,
-                                  const double* Y, double* wdot, int64_t ng, void* scratch, size_t scratch_bytes,
-                                  cudaStream_t s);
-size_t mixed_workspace_bytes(const MixedPlan* p, int64_t ng);   // what a caller is asked for
-size_t mixed_scratch_bytes(const MixedPlan* p, int64_t ng);     // what the kernel needs
+                                  const double* Y, double* wdot, int64_t ng, cudaStream_t s);
+size_t mixed_workspace_bytes(const MixedPlan* p, int64_t ng);   // what a caller is asked for; no kernel uses it
 size_t deriv_workspace_bytes(int ns, int64_t ng);
 struct GradPlan;
 cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, int adjoint, int f32, GradPlan** out);
@@ -397,7 +395,7 @@ size_t ws_bytes_for(const chemgen_handle* h, int mode, int64_t ng, bool asked = 
     if (h->use_generated && h->gen_fn && (mode == 0 || mode == 1) && (h->gen_modes & (1u << mode))) return 0;
     if (mode == CHEMGEN_MODE_FP64) return fp64_ws_bytes(h, ng);
     if (mode == CHEMGEN_MODE_MIXED && h->mixed)
-        return asked ? cg::mixed_workspace_bytes(h->mixed, ng) : cg::mixed_scratch_bytes(h->mixed, ng);
+        return asked ? cg::mixed_workspace_bytes(h->mixed, ng) : 0;
     return 0;
 }
 
@@ -486,10 +484,7 @@ int launch(chemgen_handle* h, int mode, const double* P, const double* T, int64_
     }
     if (mode == CHEMGEN_MODE_MIXED) {
         if (!h->mixed) return h->mixed_err == cudaSuccess ? CHEMGEN_ERR_UNSUPPORTED : status_of(h->mixed_err);
-        size_t need = cg::mixed_scratch_bytes(h->mixed, ng);
-        if (need && (!ws || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 255u)))
-            return CHEMGEN_ERR_INVALID_ARGUMENT;
-        return status_of(cg::launch_getrates_mixed(h->mixed, h->m, P, T, Y, w, ng, ws, ws_bytes, s));
+        return status_of(cg::launch_getrates_mixed(h->mixed, h->m, P, T, Y, w, ng, s));
     }
     return CHEMGEN_ERR_INVALID_ARGUMENT;
 }

@@ -3,7 +3,9 @@
 // serves every mechanism loaded at run time, including 348-species /
 // 2163-reaction ones.
 //
-// Work split.  A CTA owns a tile of 128 grid points -- one point per thread,
+// Work split of the 128-point kernel (the 32-point one, for large mechanisms and
+// small batches, is described where it stands).  A CTA owns a tile of 128 grid
+// points -- one point per thread,
 // one point per TMEM lane.  For every chunk of 16 reactions each thread
 // computes its point's net rates of progress q (the reference's
 // rr = kf prod C^nu - kb prod C^nu, reactions/standard.j2:3-19, with the
@@ -23,8 +25,7 @@
 // q is FP32 and the accumulation FP32.  PLOG reactions and reactions with
 // fractional stoichiometry are evaluated in FP64 and rounded to FP32.
 //
-// Per-point state: C (FP32, shared memory) and G (FP64, shared memory, or a
-// per-CTA slice of global scratch when the mechanism is too large).
+// Per-point state: C (FP32) and G (FP64) in shared memory.
 // Every mbarrier wait is bounded; a time-out sets the error word.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -69,15 +70,14 @@ constexpr unsigned kFastFall = 16;   // falloff with positive A's, decoded for t
 struct MixedPlan {
     int ns = 0, nr = 0, npad = 0, nhalf = 0, nchunk = 0;
     uint32_t tcols = 0;
-    int g_smem = 0;
+    int t128 = 0;           // the 128-point tile fits (Gibbs terms in shared memory)
     size_t smem = 0;
     int grid = 0;
     int group = 4;          // chunks accumulated in FP32 before the FP64 flush
     int nt = 1;             // threads per point (blockDim = 128 nt)
     int hot = 0;            // species with FP64 accumulators in spare tensor-memory columns
     int hot_every = 8;      // chunks between the hot species' FP64 flushes
-    int t32 = 0;            // the 32-point kernel's tile fits
-    const TcFast* fast32 = nullptr;   // its records: species as byte offsets
+    const TcFast* fast32 = nullptr;   // the 32-point kernel's records: species as byte offsets
     size_t smem32 = 0;
     int grid32 = 0;
     const int* perm = nullptr;  // accumulator column -> species (-1: padding)
@@ -393,12 +393,12 @@ __global__ void build_fast_kernel(DevMech m, TcFast* out, int scale) {
 // memory), the 16 reactions of each chunk, and the accumulator columns of
 // each flush.  The FP32 sums live in tensor memory, so extra threads cost
 // no per-species registers.
-template <bool GS, int NT>
+template <int NT>
 __global__ void __launch_bounds__(kTile * NT, 1)
     getrates_tc_kernel(DevMech m, const __nv_bfloat16* __restrict__ nu, const TcFast* __restrict__ fast, int npad,
                        int nhalf, int nchunk, uint32_t tcols,
                        const double* __restrict__ P, const double* __restrict__ Tg, const double* __restrict__ Y,
-                       double* __restrict__ wdot, int64_t ng, double* __restrict__ gscratch, int* err, int group,
+                       double* __restrict__ wdot, int64_t ng, int* err, int group,
                        const int* __restrict__ perm, int hot, int hot_every) {
     extern __shared__ __align__(1024) unsigned char sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -408,9 +408,8 @@ __global__ void __launch_bounds__(kTile * NT, 1)
     unsigned char* sB = sm + 6 * kABytes;                      // [2 buffers][npad x 16] BF16
     const int rows = ns + 1;                                   // species + the dummy row of TcFast
     float* sC = reinterpret_cast<float*>(sB + 2 * npad * 32);  // [rows][128]
-    double* sG = GS ? reinterpret_cast<double*>(sC + rows * kTile) : gscratch + (int64_t)blockIdx.x * rows * kTile;
-    double* sRed = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(sC) + rows * kTile * 4 +
-                                             (GS ? rows * kTile * 8 : 0));   // [NT][128] partial sums
+    double* sG = reinterpret_cast<double*>(sC + rows * kTile);  // [rows][128]
+    double* sRed = sG + rows * kTile;                          // [NT][128] partial sums
     uint64_t* mbar = reinterpret_cast<uint64_t*>(sRed + NT * kTile);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 2);
     if (tid == 0) {
@@ -436,7 +435,7 @@ __global__ void __launch_bounds__(kTile * NT, 1)
         c.C = sC;
         c.G = sG;
         // inputs are read once: streaming loads, so that they do not push the
-        // Gibbs scratch and the stoichiometry image out of L2
+        // stoichiometry image out of L2
         c.T = act ? __ldcs(Tg + i) : 1000.0;
         c.Pv = act ? __ldcs(P + i) : kPatm;
         c.lnT = cgm::cg_log(c.T);
@@ -615,8 +614,7 @@ __global__ void __launch_bounds__(kTile * NT, 1)
                                     double x = (double)v[j];
                                     if (h64) x += __hiloint2double((int)d[2 * j + 1], (int)d[2 * j]);
                                     double* w = wdot + (int64_t)sp * ng + i;
-                                    // first (often only) group: a streaming store, so that
-                                    // wdot does not push the Gibbs scratch out of L2
+                                    // first (often only) group: a streaming store
                                     if (first_group) __stcs(w, x);
                                     else *w += x;
                                 }
@@ -640,14 +638,18 @@ __global__ void __launch_bounds__(kTile * NT, 1)
 //
 // One point per lane and one reaction per warp: every lane of a warp runs the
 // same reaction (no divergence, records read once per warp), and the tile's
-// C (FP32) and G (FP64) fit in shared memory up to ~410 species, where the
-// 128-point tile had to read G from L2 for every molecule.  The 16 warps take
+// C (FP32) and G (FP64) fit in shared memory for every mechanism that the mixed
+// mode takes (352 species), where a 128-point tile holds G up to 126 species
+// only and had to read it from L2 for every molecule beyond.  The 16 warps take
 // the 32 reactions of two chunks, two each; lane p's rates are row p of the A
 // operands.  The MMAs stay M = 128 (the tensor memory's lanes): rows 32..127
 // read whatever follows in shared memory, and nobody reads their sums.  A batch
 // of 20011 points is 5 rounds of 626 tiles instead of two waves of 157.  The
-// order of every sum -- reactions in K, chunks, splits, hot flushes -- is the
-// 128-point kernel's, and so is every bit of the result.
+// order of the contraction's sums -- reactions in K, chunks, splits, hot flushes --
+// is the 128-point kernel's.  The prologue's sums over species (16 parts), ctot, the
+// falloff (q_exp, q_rcp) and its Gibbs sum are not, in FP64: a rate whose FP32
+// rounding that tips differs by an ulp, so the two kernels agree to rounding
+// (far inside the mixed mode's 1e-6), not bit for bit.
 // Bound by latency (34 % of issue slots; FP64 chains, shared loads, records
 // from L1) with 17 warps of 96 registers.  Measured on B200: JetSurf 2.0, 20011
 // points 2.30 -> 1.12 ms, 256 points 1.11 -> 0.22 ms; 348/2163, 20011 points
@@ -1189,20 +1191,17 @@ __global__ void __launch_bounds__(32 * (kTWarps + 1), 1)
     if (warp == 0) um::tmem_dealloc(tbase, tcols);
 }
 
-const void* kernel_for(int g_smem, int nt) {
-    if (g_smem) return nt == 4 ? (const void*)getrates_tc_kernel<true, 4>
-                               : nt == 2 ? (const void*)getrates_tc_kernel<true, 2> : (const void*)getrates_tc_kernel<true, 1>;
-    return nt == 4 ? (const void*)getrates_tc_kernel<false, 4>
-                   : nt == 2 ? (const void*)getrates_tc_kernel<false, 2> : (const void*)getrates_tc_kernel<false, 1>;
+const void* kernel_for(int nt) {
+    return nt == 4 ? (const void*)getrates_tc_kernel<4>
+                   : nt == 2 ? (const void*)getrates_tc_kernel<2> : (const void*)getrates_tc_kernel<1>;
 }
 
-template <bool GS, int NT>
+template <int NT>
 cudaError_t launch_tc(const MixedPlan* p, const DevMech& m, const double* P, const double* T, const double* Y,
-                      double* wdot, int64_t ng, double* scratch, int64_t grid, cudaStream_t s) {
-    getrates_tc_kernel<GS, NT><<<(unsigned)grid, kTile * NT, p->smem, s>>>(m, p->nu, p->fast, p->npad, p->nhalf, p->nchunk,
-                                                                           p->tcols, P, T, Y, wdot, ng, scratch,
-                                                                           p->err, p->group, p->perm, p->hot,
-                                                                           p->hot_every);
+                      double* wdot, int64_t ng, int64_t grid, cudaStream_t s) {
+    getrates_tc_kernel<NT><<<(unsigned)grid, kTile * NT, p->smem, s>>>(m, p->nu, p->fast, p->npad, p->nhalf, p->nchunk,
+                                                                       p->tcols, P, T, Y, wdot, ng, p->err, p->group,
+                                                                       p->perm, p->hot, p->hot_every);
     return cudaGetLastError();
 }
 
@@ -1226,7 +1225,9 @@ cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, M
     cudaError_t e = device_limits(device, &dev);
     if (e != cudaSuccess) return e;
     const size_t limit = dev.smem_block;
-    if (base > limit) return cudaErrorNotSupported;
+    // up to 352 species; the 32-point tile then fits too (198 KB)
+    const size_t t32 = 12 * (size_t)kA32 + 4 * (size_t)npad * 32 + rows * kTP * 12 + kTWarps * kTP * 8 + sizeof(Tile32) + 64;
+    if (base > limit || t32 > limit) return cudaErrorNotSupported;
     MixedPlan* p = new MixedPlan();
     p->ns = ns;
     p->nr = nr;
@@ -1234,14 +1235,14 @@ cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, M
     p->nhalf = nhalf;
     p->nchunk = nchunk;
     p->tcols = tcols;
-    p->g_smem = with_g <= limit ? 1 : 0;
+    p->t128 = with_g <= limit ? 1 : 0;
     // FP32 accumulation runs over `group` chunks (16 reactions each) before
     // the partial sums are added into the FP64 output: 64 reactions for small
     // mechanisms (GRI30 needs it for 1e-6), the whole mechanism for large
     // ones, whose output does not fit in L2 and would otherwise be read back
     // from DRAM at every flush (348/2163: 3.5e-7 with one flush)
     p->group = npad <= 128 ? 4 : nchunk;
-    p->smem = p->g_smem ? with_g : base;
+    p->smem = p->t128 ? with_g : base;
     // resident CTAs per SM, limited by shared memory and by 512 TMEM columns
     int per_sm = (int)(dev.smem_sm / (p->smem + 1024));
     per_sm = std::min(per_sm, (int)(512 / tcols));
@@ -1251,7 +1252,7 @@ cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, M
     p->nt = 1;
     for (int nt : {4, 2}) {
         cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, kernel_for(p->g_smem, nt)) != cudaSuccess) continue;
+        if (!p->t128 || cudaFuncGetAttributes(&fa, kernel_for(nt)) != cudaSuccess) continue;
         if ((long)per_sm * kTile * nt * fa.numRegs <= dev.regs_sm &&
             per_sm * kTile * nt <= dev.threads_sm) {
             p->nt = nt;
@@ -1259,13 +1260,8 @@ cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, M
         }
     }
     p->grid = dev.sms * per_sm;
-    // the 32-point kernel whenever its tile's state fits
-    const size_t t32 = 12 * (size_t)kA32 + 4 * (size_t)npad * 32 + rows * kTP * 12 + kTWarps * kTP * 8 + sizeof(Tile32) + 64;
-    if (t32 <= limit) {
-        p->t32 = 1;
-        p->smem32 = t32;
-        p->grid32 = dev.sms;
-    }
+    p->smem32 = t32;
+    p->grid32 = dev.sms;
     // nu chunks in the canonical K-major layout: B[n][k] = nu of species n in reaction 16*chunk + k
     std::vector<float> nuf((size_t)ns * nr, 0.0f);
     const int32_t* rp = (const int32_t*)v.a[CG_RPTR];
@@ -1318,8 +1314,8 @@ cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, M
     if (e == cudaSuccess)
         e = cudaMemcpy((char*)p->dbuf + img_bytes + 2 * fast_bytes, perm.data(), perm.size() * sizeof(int),
                        cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel_for(p->g_smem, p->nt),
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
+    if (e == cudaSuccess && p->t128)
+        e = cudaFuncSetAttribute(kernel_for(p->nt), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
     if (e != cudaSuccess) {
         if (p->dbuf) cudaFree(p->dbuf);
         delete p;
@@ -1331,7 +1327,7 @@ cudaError_t mixed_prepare(const DevMech& m, const cg_mech_view& v, int device, M
     p->perm = (const int*)((char*)p->dbuf + img_bytes + 2 * fast_bytes);
     if (nr > 0) {
         build_fast_kernel<<<(nr + 127) / 128, 128>>>(m, (TcFast*)p->fast, 1);
-        if (p->t32) build_fast_kernel<<<(nr + 127) / 128, 128>>>(m, (TcFast*)p->fast32, kTP * 4);
+        build_fast_kernel<<<(nr + 127) / 128, 128>>>(m, (TcFast*)p->fast32, kTP * 4);
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
         if (e != cudaSuccess) {
@@ -1351,33 +1347,33 @@ void mixed_release(MixedPlan* p) {
     delete p;
 }
 
-// Scratch the kernel that runs needs (none with 32-point tiles), and the
-// scratch a caller is asked for: the latter stays what the 128-point kernel
-// needs, so that programs that size and pass it see no change.
-size_t mixed_workspace_bytes(const MixedPlan* p, int64_t ng);
-size_t mixed_scratch_bytes(const MixedPlan* p, int64_t ng) { return p && p->t32 ? 0 : mixed_workspace_bytes(p, ng); }
-
+// What a caller of chemgen_getrates_ws is asked for: what mechanisms beyond the
+// 128-point tile needed when it kept their Gibbs terms in global scratch.  No
+// kernel uses it any more; the size stays, so that programs that ask for it,
+// allocate it and pass it see no change.
 size_t mixed_workspace_bytes(const MixedPlan* p, int64_t ng) {
-    if (!p || p->g_smem) return 0;
+    if (!p || p->t128) return 0;
     int64_t tiles = (ng + kTile - 1) / kTile;
     int64_t grid = std::min<int64_t>(tiles, p->grid);
     return (size_t)grid * (p->ns + 1) * kTile * sizeof(double);
 }
 
 cudaError_t launch_getrates_mixed(const MixedPlan* p, const DevMech& m, const double* P, const double* T,
-                                  const double* Y, double* wdot, int64_t ng, void* scratch, size_t scratch_bytes,
-                                  cudaStream_t s) {
+                                  const double* Y, double* wdot, int64_t ng, cudaStream_t s) {
     if (ng <= 0) return cudaSuccess;
     // the kernel's shared-memory limit is this plan's, set under one lock with
     // the launch (a plan made later for a smaller mechanism sets it lower)
     static std::mutex mu;
     // Mechanisms whose Gibbs terms fit beside the 128-point tile run the faster
-    // of the two: on B200 at 53/325 a round of 32-point tiles takes 40 us and a
-    // wave of 128-point tiles 121 us (9/21: 12 and 29).  Larger ones always run
-    // 32-point tiles (348/2163: a round 0.17 ms, a wave 0.82 ms).
-    const int64_t rounds = (ng + (int64_t)kTP * p->grid32 - 1) / std::max<int64_t>(1, (int64_t)kTP * p->grid32);
+    // of the two.  On B200 at 53/325 a round of 32-point tiles takes 40 us and a
+    // wave of 128-point tiles, one to an SM, 121 us, with 60 PLOG reactions 57 and
+    // 171: there one or two rounds against a wave, or five against two, take the
+    // 32-point kernel.  Smaller mechanisms have several 128-point tiles to an SM and a
+    // wave for many more rounds: 9/21, 12 and 29 us, two rounds at most.  Larger
+    // ones always run 32-point tiles (348/2163: a round 0.17 ms, a wave 0.82 ms).
+    const int64_t rounds = (ng + (int64_t)kTP * p->grid32 - 1) / ((int64_t)kTP * p->grid32);
     const int64_t waves = (ng + (int64_t)kTile * p->grid - 1) / ((int64_t)kTile * p->grid);
-    if (p->t32 && (!p->g_smem || (double)rounds * 0.35 <= (double)waves)) {
+    if (!p->t128 || (double)rounds * 0.35 <= (double)waves) {
         const unsigned g32 = (unsigned)std::min<int64_t>((ng + kTP - 1) / kTP, p->grid32);
         std::lock_guard<std::mutex> lk(mu);
         const cudaError_t e = cudaFuncSetAttribute(getrates_tc32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1388,25 +1384,15 @@ cudaError_t launch_getrates_mixed(const MixedPlan* p, const DevMech& m, const do
                                                                   p->perm, p->hot, p->hot_every);
         return cudaGetLastError();
     }
-    int64_t tiles = (ng + kTile - 1) / kTile;
-    int64_t grid = std::min<int64_t>(tiles, p->grid);
-    if (!p->g_smem) {
-        const int64_t fit = (int64_t)(scratch_bytes / ((size_t)(p->ns + 1) * kTile * sizeof(double)));
-        grid = std::min<int64_t>(grid, fit);
-        if (grid < 1 || !scratch) return cudaErrorInvalidValue;
-    }
-    double* gs = p->g_smem ? nullptr : (double*)scratch;
+    const int64_t grid = std::min<int64_t>((ng + kTile - 1) / kTile, p->grid);
     std::lock_guard<std::mutex> lk(mu);
-    const cudaError_t e = cudaFuncSetAttribute(kernel_for(p->g_smem, p->nt),
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel_for(p->nt), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p->smem);
     if (e != cudaSuccess) return e;
-    switch ((p->g_smem ? 10 : 0) + p->nt) {
-        case 14: return launch_tc<true, 4>(p, m, P, T, Y, wdot, ng, gs, grid, s);
-        case 12: return launch_tc<true, 2>(p, m, P, T, Y, wdot, ng, gs, grid, s);
-        case 11: return launch_tc<true, 1>(p, m, P, T, Y, wdot, ng, gs, grid, s);
-        case 4: return launch_tc<false, 4>(p, m, P, T, Y, wdot, ng, gs, grid, s);
-        case 2: return launch_tc<false, 2>(p, m, P, T, Y, wdot, ng, gs, grid, s);
-        default: return launch_tc<false, 1>(p, m, P, T, Y, wdot, ng, gs, grid, s);
+    switch (p->nt) {
+        case 4: return launch_tc<4>(p, m, P, T, Y, wdot, ng, grid, s);
+        case 2: return launch_tc<2>(p, m, P, T, Y, wdot, ng, grid, s);
+        default: return launch_tc<1>(p, m, P, T, Y, wdot, ng, grid, s);
     }
 }
 

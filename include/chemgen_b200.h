@@ -82,7 +82,9 @@ int chemgen_getrates_counted(chemgen_handle* h, const double* P, const double* T
 
 /* Scratch a call needs for `ng` points in `mode` (0 when the per-point state
  * fits in shared memory), and the variant that uses caller-owned scratch of
- * at least that many bytes (256-byte aligned) instead of library-owned memory. */
+ * at least that many bytes (256-byte aligned) instead of library-owned memory.
+ * Mixed mode from 127 to 352 species: the kernel no longer uses the scratch that
+ * is asked for; the size is kept, and a call without it refused, as before. */
 int chemgen_workspace_bytes(const chemgen_handle* h, int mode, int64_t ng, size_t* bytes);
 int chemgen_getrates_ws(chemgen_handle* h, int mode, const double* P, const double* T, int64_t ng,
                         const double* Y, double* wdot, void* workspace, size_t workspace_bytes, void* stream);

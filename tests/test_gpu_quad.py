@@ -343,6 +343,26 @@ def test_mixed_32_point_tiles_falloff(kinds):
     assert oracle.errors(w, r["wdot"], r["S"])["norm_max"] <= 1e-6
 
 
+@pytest.mark.parametrize("ns,nr", [(53, 325), (10, 60), (126, 200)])
+def test_mixed_tiles_of_32_and_128_points_agree(ns, nr):
+    # the same points in a batch of one 32-point round and in one of a whole
+    # 128-point wave.  Their FP64 values differ in rounding, which can tip the FP32
+    # rounding of up to three concentrations, M, 2^f, the products and the sum: eight
+    # times 1.2e-7 of the gross rate S
+    import torch
+    mech = synthetic.synthetic_mechanism(ns, nr, 9, 9, seed=4, n_lindemann=3, n_sri=3, n_plog=3)
+    blob = pack.pack(mech).to_blob()
+    gm = GpuMechanism(blob)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    P, T, Y = _cuda(*synthetic.states(ns, 4 * 128 * sms, seed=3))
+    n = 32 * sms - 5
+    w = gm.getrates(P[:n].contiguous(), T[:n].contiguous(), Y[:, :n].contiguous(), mode="mixed")
+    ref = gm.getrates(P, T, Y, mode="mixed")[:, :n]
+    r = oracle.rates(blob, P[:n].cpu().numpy(), T[:n].cpu().numpy(), Y[:, :n].contiguous().cpu().numpy(), mech.nr)
+    S = torch.from_numpy(r["S"]).cuda()
+    assert float(((w - ref).abs() / S.clamp_min(1e-300)).max()) <= 1e-6
+
+
 @pytest.mark.parametrize("rows,cols", [(1 << 19, 1), (1, 1 << 19), (9893, 53), (53, 9893), (8129, 65), (348, 1507)])
 def test_transposed_copies(rows, cols):
     # tiles of 64 x 64: whole, part and single-row ones; the values are moved, not computed
