@@ -388,3 +388,36 @@ def test_a_handle_is_made_in_a_few_milliseconds():
         t.append(time.perf_counter() - t0)
         gm.close()
     assert min(t[1:]) < 12e-3, t
+
+
+def test_split_calls_from_two_threads_on_streams_of_their_own():
+    # a wave on the generated kernel and 5000 points on the tiles, from two threads
+    # of one handle; and with point-major tensors into a ragged out=
+    import threading
+    import torch
+    from chemgen_b200 import emit_cuda as E
+    from conftest import load_golden
+    mech = load_golden("gri30")[0]
+    gm = GpuMechanism(mech, generated=True)
+    n = 5000 + (E.choose_block(mech.ns, False, E.use_tmem(mech.ns, False)) *
+                torch.cuda.get_device_properties(0).multi_processor_count)
+    data = [_cuda(*synthetic.states(mech.ns, n, seed=s)) for s in (1, 2)]
+    ref = [gm.getrates(*d) for d in data]
+    out = torch.empty(n, mech.ns, dtype=torch.float64, device="cuda")
+    assert gm.getrates(data[0][0], data[0][1], data[0][2].t().contiguous(), layout="point_major", out=out) is out
+    assert torch.equal(out, ref[0].t())
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(k):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            for _ in range(10):
+                w = gm.getrates(*data[k])
+                s.synchronize()
+                if not torch.equal(w, ref[k]):
+                    bad.append(k)
+    th = [threading.Thread(target=work, args=(k,)) for k in (0, 1)]
+    [t.start() for t in th]
+    [t.join() for t in th]
+    assert not bad
