@@ -20,10 +20,11 @@
 // What bounds them: the load/store unit (60-70 % busy: state, records, rows)
 // and the issue rate (47 %), with one CTA per SM for the Jacobian (its 2000
 // rows take 130 KB; 24 warps, or 32 for FP32 storage), two of 12 for the
-// adjoint.  J itself is written once, in 64-byte pieces.  Measured on B200 at 53/325, 65536 points, against
-// the kernels they replaced (32-point tiles; the Jacobian's derivatives cached
-// in L2 and gathered row by row, the adjoint added into per-warp copies):
-// Jacobian FP64 3.17 -> 1.16 ms, FP32 3.10 -> 1.14 ms, adjoint 1.66 -> 0.42 ms.
+// adjoint.  J itself is written once, in 64-byte pieces.  Measured on B200 at
+// 53/325, 65536 points, against the kernels they replaced (32-point tiles; the
+// Jacobian's derivatives cached in L2 and gathered row by row, the adjoint added
+// into per-warp copies): Jacobian FP64 3.17 -> 1.12 ms, FP32 3.10 -> 1.14 ms,
+// adjoint 1.66 -> 0.39 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -725,10 +726,10 @@ const void* grad_kernel(const GradPlan* p, int precision) {
 void grad_release(GradPlan* p);
 
 // adjoint: any mechanism whose state fits (the reactions run in chunks).
-// Jacobian: the rows of every reaction at once (about 520 reactions), and at
-// most 32767 species-pair codes.  cudaErrorNotSupported otherwise.  f32: the
-// Jacobian's plan for FP32 storage where it has one of its own (the FP64 plan
-// serves both otherwise, and this returns cudaErrorNotSupported).
+// Jacobian: the rows of every reaction at once (about 520 reactions).  At most
+// 511 species.  cudaErrorNotSupported otherwise.  f32: the Jacobian's plan for FP32 storage
+// where it has one of its own (the FP64 plan serves both otherwise, and this
+// returns cudaErrorNotSupported).
 cudaError_t grad_prepare(const DevMech& m, const cg_mech_view& v, int device, int adjoint, int f32, GradPlan** out) {
     *out = nullptr;
     const int ns = m.ns, nr = m.nr;

@@ -650,7 +650,7 @@ __global__ void __launch_bounds__(kTile * NT, 1)
 // falloff (q_exp, q_rcp) and its Gibbs sum are not, in FP64: a rate whose FP32
 // rounding that tips differs by an ulp, so the two kernels agree to rounding
 // (far inside the mixed mode's 1e-6), not bit for bit.
-// Bound by latency (34 % of issue slots; FP64 chains, shared loads, records
+// Bound by latency (41 % of issue slots; FP64 chains, shared loads, records
 // from L1) with 17 warps of 96 registers.  Measured on B200: JetSurf 2.0, 20011
 // points 2.30 -> 1.12 ms, 256 points 1.11 -> 0.22 ms; 348/2163, 20011 points
 // 1.71 -> 0.89 ms, 65536 points 3.43 -> 2.47 ms.

@@ -61,7 +61,9 @@ int chemgen_num_reactions(const chemgen_handle* h);
 /* FP64 getrates on device pointers.
  * Replaces: getrates_hip_wrapper_v1..v4 (reactions_hip/hip_v1_cpp.j2:339-372,
  * hip_v2_cpp.j2:1078-1160) and the generated getrates (python_header.j2:25).
- * Any ng >= 0 (the reference requires ng to be a multiple of its block). */
+ * Any ng >= 0 (the reference requires ng to be a multiple of its block).
+ * Temperatures from 1.5 mK up are evaluated as given; below that the FP64 tile
+ * and derivative kernels use the rate constants of 1/700 K. */
 int chemgen_getrates(chemgen_handle* h, const double* P, const double* T, int64_t ng, const double* Y,
                      double* wdot, void* stream);
 
@@ -117,7 +119,11 @@ int chemgen_register_kernels(uint64_t fingerprint, int ns, int nr, unsigned mode
  * laid out for ng points, `block` points per SM and wave.  The library calls
  * it with i0 = 0 and i1 a multiple of `block`.  With it, a batch
  * that leaves most of its last wave empty runs that remainder (or all of a
- * small batch) on the table-driven tile kernel of the same arithmetic. */
+ * small batch) on the table-driven tile kernel.  In mixed mode the two give the
+ * same bits; in FP64 mode they sum in another order, so a point's result can
+ * differ in rounding (1e-12 of the largest rate) with the size of the batch, its
+ * place in it and the number of SMs, and between chemgen_getrates_host, which
+ * works in chunks, and a call on the whole batch. */
 typedef int (*chemgen_kernel_range_fn)(int mode, const double* P, const double* T, int64_t ng, const double* Y,
                                        double* wdot, int64_t i0, int64_t i1, void* stream);
 int chemgen_register_kernel_range(uint64_t fingerprint, int ns, int nr, int mode, int block,
